@@ -1,6 +1,7 @@
 // Power-of-two complex FFT plans and execution (the pass kernel is in
 // fft_pass.cuh).
 #include "fft_pass.cuh"
+#include "fix64.cuh"
 
 #include <algorithm>
 
@@ -30,8 +31,46 @@ int make_table(void **dst, long long count, long long mul, long long Np) {
   return GSFFT_OK;
 }
 
+// Fixed-point twiddles of an FP64 pass of radix 2^logr that reaches Np = 2^lg
+// points: the radix-16 stages' rows [e][k] = exp(-2 pi i e k / (16 Ns)) scaled by
+// 2^60, and exp(-2 pi i m / Np) as hi[m >> h] lo[m & (2^h - 1)] scaled by 2^62.
+// One launch: threads [0, ntw) the stage rows, then hi, then lo.
+__global__ void fx_tables_kernel(int logr, int lg, int h, int ntw, int nhi, int nlo, fx::Tw *tw,
+                                 longlong2 *hi, fx::Tw *lo) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < ntw) {
+    int logns = logr % 4 == 0 ? 4 : logr % 4;
+    const int at = i;
+    while (i >= (16 << logns)) {
+      i -= 16 << logns;
+      logns += 4;
+    }
+    const unsigned e = (unsigned)i >> logns, k = (unsigned)i & ((1u << logns) - 1u);
+    const fx::C64 w = fx::unit_root((unsigned long long)e * k, logns + 4);
+    tw[at] = fx::limbs(fx::C64{(w.x + 2) >> 2, (w.y + 2) >> 2});
+  } else if (i < ntw + nhi) {
+    const fx::C64 w = fx::unit_root((unsigned long long)(i - ntw) << h, lg);
+    hi[i - ntw] = make_longlong2(w.x, w.y);
+  } else if (i < ntw + nhi + nlo) {
+    lo[i - ntw - nhi] = fx::limbs(fx::unit_root((unsigned long long)(i - ntw - nhi), lg));
+  }
+}
+
+int make_fx_tables(FftPlan &p, int i, int lg) {
+  int ntw = 0;
+  for (int l = p.logR[i] % 4 == 0 ? 4 : p.logR[i] % 4; l < p.logR[i]; l += 4) ntw += 16 << l;
+  const int h = p.tw_h[i], nlo = 1 << h, nhi = 1 << (lg - h);
+  GS_CUDA(cudaMalloc(&p.fx_tw[i], sizeof(fx::Tw) * ntw));
+  GS_CUDA(cudaMalloc(&p.fx_hi[i], sizeof(longlong2) * nhi));
+  GS_CUDA(cudaMalloc(&p.fx_lo[i], sizeof(fx::Tw) * nlo));
+  fx_tables_kernel<<<(ntw + nhi + nlo + 127) / 128, 128>>>(p.logR[i], lg, h, ntw, nhi, nlo, (fx::Tw *)p.fx_tw[i],
+                                                          (longlong2 *)p.fx_hi[i], (fx::Tw *)p.fx_lo[i]);
+  GS_LAUNCHED();
+  return GSFFT_OK;
+}
+
 int dispatch_pass(bool dbl, int logr, const PassArgs &a, long long total_sub, cudaStream_t st) {
-  if (dbl) return logr <= 9 ? fft_pass_f64_lo(logr, a, total_sub, st) : fft_pass_f64_hi(logr, a, total_sub, st);
+  if (dbl) return logr <= 10 ? fft_pass_f64_lo(logr, a, total_sub, st) : fft_pass_f64_hi(logr, a, total_sub, st);
   return logr <= 10 ? fft_pass_f32_lo(logr, a, total_sub, st) : fft_pass_f32_hi(logr, a, total_sub, st);
 }
 
@@ -85,6 +124,7 @@ int fft_plan_init(FftPlan &p, long long n, int precision, int max_batch, int fir
       GS_CHECK(make_table<double>(&p.tw_lo[i], nlo, 1, Np));
       GS_CHECK(make_table<double>(&p.tw_hi[i], nhi, nlo, Np));
       GS_CHECK(make_table<double>(&p.tw_R[i], R, 1, R));
+      GS_CHECK(make_fx_tables(p, i, lg));
     } else {
       GS_CHECK(make_table<float>(&p.tw_lo[i], nlo, 1, Np));
       GS_CHECK(make_table<float>(&p.tw_hi[i], nhi, nlo, Np));
@@ -180,7 +220,11 @@ void fft_plan_free(FftPlan &p) {
     if (p.tw_hi[i]) cudaFree(p.tw_hi[i]);
     if (p.tw_lo[i]) cudaFree(p.tw_lo[i]);
     if (p.tw_R[i]) cudaFree(p.tw_R[i]);
+    if (p.fx_tw[i]) cudaFree(p.fx_tw[i]);
+    if (p.fx_hi[i]) cudaFree(p.fx_hi[i]);
+    if (p.fx_lo[i]) cudaFree(p.fx_lo[i]);
     p.tw_hi[i] = p.tw_lo[i] = p.tw_R[i] = nullptr;
+    p.fx_tw[i] = p.fx_hi[i] = p.fx_lo[i] = nullptr;
   }
   if (p.scratch) cudaFree(p.scratch);
   p.scratch = nullptr;
@@ -200,6 +244,7 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
   if (p.npass > 1 && (long long)batch * p.n * (p.npass == 3 ? 2 : 1) > p.scratch_elems)
     return GSFFT_ERR_PARAM;
   if (io.gather_x && batch > 8) return GSFFT_ERR_PARAM;
+  if (dbl && io.sum_rows > 1) return GSFFT_ERR_UNSUPPORTED;  // FP32 passes only
   const void *src = in;
   char *scr = (char *)p.scratch;
   long long Ns = 1;
@@ -226,6 +271,10 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
     a.tw_lo = p.tw_lo[i];
     a.tw_h = p.tw_h[i];
     a.twR = p.tw_R[i];
+    a.fx_tw = p.fx_tw[i];
+    a.fx_hi = p.fx_hi[i];
+    a.fx_lo = p.fx_lo[i];
+    a.one = 1;
     a.gx = (i == 0) ? io.gather_x : nullptr;
     for (int q = 0; q < 8; q++) a.goffs[q] = io.gather_offsets[q];
     a.gstride = io.gather_stride;

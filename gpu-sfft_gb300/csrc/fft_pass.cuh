@@ -12,12 +12,12 @@
 // Each CTA runs G sub-transforms of size R in shared memory as a Stockham
 // sequence of radix-16 register stages (one radix-2/4/8 stage for the
 // remainder).  G >= 2 (FP64) / 4 (FP32) so every strided global access moves
-// whole 32-byte sectors.  Twiddles come from exact-angle tables (sincospi in
-// FP64); FP64 looks every one up, FP32 builds some as products of a few
-// looked-up ones (at most about eight roundings, never a long recurrence).
-// Inverse = conj(DFT(conj(x))).
+// whole 32-byte sectors.  FP32 twiddles come from exact-angle tables (sincospi
+// in FP64), some as products of a few looked-up ones (at most about eight
+// roundings, never a long recurrence).  Inverse = conj(DFT(conj(x))).
 //
-// This header holds the pass kernel; its instantiations are spread over
+// This header holds the FP32 pass kernel and what the FP64 one
+// (fft_pass_fx.cuh) shares with it; the instantiations are spread over
 // fft_pass_*.cu so that they compile in parallel.
 #pragma once
 #include "gsfft_internal.cuh"
@@ -46,13 +46,17 @@ struct PassArgs {
   int nsum;           // first pass: add nsum partial inputs sstride apart
   long long sstride;
   int write_complex;
+  // FP64 passes: fixed-point twiddles -- the radix-16 stages' tables, and the
+  // two-level table of exp(-2 pi i m / Np)
+  const void *fx_tw, *fx_hi, *fx_lo;
+  int one;  // 1, as a value that the compiler does not see (fix64.cuh)
 };
 
 // Launch one pass of radix 2^logr (each covers the radices listed).
 int fft_pass_f32_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 5..10
 int fft_pass_f32_hi(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 11..14
-int fft_pass_f64_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 5..9
-int fft_pass_f64_hi(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 10..13
+int fft_pass_f64_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 7..10
+int fft_pass_f64_hi(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 11..13
 
 namespace {
 
@@ -114,17 +118,13 @@ template <> __host__ __device__ constexpr int g_of<double>(int logr) {
 template <> __host__ __device__ constexpr int g_of<float>(int logr) {
   return logr >= 14 ? 1 : (logr == 13 ? 2 : imax(4, 4096 >> logr));
 }
-template <typename T> __host__ __device__ constexpr int nt_of(int logr) {
-  return imin(((1 << logr) / 16) * g_of<T>(logr), 512);
-}
+__host__ __device__ constexpr int nt_of(int logr) { return imin(((1 << logr) / 16) * g_of<float>(logr), 512); }
 // Resident CTAs per SM the register budget is sized for, so that the loads,
 // shared-memory butterflies and stores of different CTAs overlap.  A thread
-// holds one radix-16 butterfly when (R/16)*G <= 512 (Q = 1); then FP32 fits
-// 64 registers (two 512-thread CTAs) and FP64 128 (two 256-thread CTAs).
-template <typename T> __host__ __device__ constexpr int minb_of(int logr) {
-  return ((1 << logr) / 16) * g_of<T>(logr) > 512
-             ? 1
-             : (sizeof(T) == 4 ? (nt_of<T>(logr) >= 512 ? 2 : 4) : (nt_of<T>(logr) >= 512 ? 1 : 2));
+// holds one radix-16 butterfly when (R/16)*G <= 512 (Q = 1) and fits 64
+// registers (two 512-thread CTAs).
+__host__ __device__ constexpr int minb_of(int logr) {
+  return ((1 << logr) / 16) * g_of<float>(logr) > 512 ? 1 : (nt_of(logr) >= 512 ? 2 : 4);
 }
 __host__ __device__ constexpr int padded(int i) { return i + (i >> 4); }
 // Row stride in elements.  Rows start in different banks; when a warp's load
@@ -136,23 +136,22 @@ __host__ __device__ constexpr int padded(int i) { return i + (i >> 4); }
 template <typename T> __host__ __device__ constexpr int rowpitch(int logr) {
   return padded(1 << logr) +
          ((sizeof(T) == 4 && g_of<T>(logr) >= 2 && g_of<T>(logr) <= 16 &&
-           nt_of<T>(logr) / g_of<T>(logr) >= 32)
+           nt_of(logr) / g_of<T>(logr) >= 32)
               ? 16 / g_of<T>(logr)
               : 1);
 }
-// twiddle table exp(-2 pi i m / R) copied into shared memory when it fits
 template <typename T> __host__ __device__ constexpr int data_smem_of(int logr) {
   return g_of<T>(logr) * rowpitch<T>(logr) * (int)sizeof(typename Cx<T>::V);
 }
-template <typename T> __host__ __device__ constexpr bool tw_in_smem(int logr) {
-  return data_smem_of<T>(logr) + (1 << logr) * (int)sizeof(typename Cx<T>::V) <= 220 * 1024;
+// FP32: the twiddle table exp(-2 pi i m / R) is copied into shared memory when it fits
+__host__ __device__ constexpr bool tw_in_smem(int logr) {
+  return data_smem_of<float>(logr) + (1 << logr) * (int)sizeof(float2) <= 220 * 1024;
 }
-template <typename T> __host__ __device__ constexpr int smem_of(int logr) {
-  return data_smem_of<T>(logr) +
-         (tw_in_smem<T>(logr) ? (1 << logr) * (int)sizeof(typename Cx<T>::V) : 0);
+__host__ __device__ constexpr int smem_of(int logr) {
+  return data_smem_of<float>(logr) + (tw_in_smem(logr) ? (1 << logr) * (int)sizeof(float2) : 0);
 }
 
-// Inter-pass twiddles folded into the first shared-memory stage (FP32 passes
+// Inter-pass twiddles folded into the first shared-memory stage (passes
 // after the first): the stage's inputs are conjugated (inverse) and
 // multiplied by W^(jm r) in registers instead of in a separate read-modify-
 // write of shared memory.  Element r = t + e NB of the row takes
@@ -171,31 +170,29 @@ __device__ __forceinline__ float2 tw_look(const PreTw &pt, long long mm) {
   return cmul(__ldg(&pt.thi[mm >> pt.h]), __ldg(&pt.tlo[mm & pt.hmask]));
 }
 
-template <typename V, int E, int Q, int NB, int TPF>
-__device__ __forceinline__ void apply_pretw(V (&v)[Q][E], const PreTw &pt, int g, int t0) {
-  if constexpr (sizeof(decltype(V().x)) == 4) {
-    if (!pt.on) return;
-    const long long jm = ((pt.u0 + g) & pt.Smask) & pt.Nsmask;
-    const float2 s1 = tw_look(pt, jm * NB);
-    float2 s4 = make_float2(1.f, 0.f);
-    if constexpr (E >= 8) s4 = tw_look(pt, jm * 4 * NB);
+template <int E, int Q, int NB, int TPF>
+__device__ __forceinline__ void apply_pretw(float2 (&v)[Q][E], const PreTw &pt, int g, int t0) {
+  if (!pt.on) return;
+  const long long jm = ((pt.u0 + g) & pt.Smask) & pt.Nsmask;
+  const float2 s1 = tw_look(pt, jm * NB);
+  float2 s4 = make_float2(1.f, 0.f);
+  if constexpr (E >= 8) s4 = tw_look(pt, jm * 4 * NB);
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      float2 wa = tw_look(pt, jm * (t0 + q * TPF)), w = wa;
+  for (int q = 0; q < Q; q++) {
+    float2 wa = tw_look(pt, jm * (t0 + q * TPF)), w = wa;
 #pragma unroll
-      for (int e = 0; e < E; e++) {
-        if (e > 0) {
-          if ((e & 3) == 0) {
-            wa = cmul(wa, s4);
-            w = wa;
-          } else {
-            w = cmul(w, s1);
-          }
+    for (int e = 0; e < E; e++) {
+      if (e > 0) {
+        if ((e & 3) == 0) {
+          wa = cmul(wa, s4);
+          w = wa;
+        } else {
+          w = cmul(w, s1);
         }
-        V x = v[q][e];
-        if (pt.inverse) x.y = -x.y;
-        v[q][e] = cmul(x, w);
       }
+      float2 x = v[q][e];
+      if (pt.inverse) x.y = -x.y;
+      v[q][e] = cmul(x, w);
     }
   }
 }
@@ -204,13 +201,12 @@ __device__ __forceinline__ void apply_pretw(V (&v)[Q][E], const PreTw &pt, int g
 // (twR[m] = exp(-2 pi i m / R)).
 template <typename V, int E>
 __device__ __forceinline__ void stage_twiddles(V (&v)[E], const V *__restrict__ twR, int k, int step) {
-  if constexpr (sizeof(v[0].x) == 8 || E < 4) {
-    // FP64: exact table entries (its FP64 pipe, not shared memory, is the limit)
+  if constexpr (E < 4) {
 #pragma unroll
     for (int e = 1; e < E; e++) v[e] = cmul(v[e], twR[k * e * step]);
   } else {
-    // FP32: two table reads (w, w^4), other powers by products at most four
-    // deep -- the strided table reads were the shared-memory bank hot spot
+    // two table reads (w, w^4), other powers by products at most four deep --
+    // the strided table reads were the shared-memory bank hot spot
     V w[E];
     w[1] = twR[k * step];
     w[2] = cmul(w[1], w[1]);
@@ -261,7 +257,7 @@ __device__ __forceinline__ void smem_stage(V *sm, const V *__restrict__ twR, con
 #pragma unroll
       for (int e = 0; e < E; e++) v[q][e] = rp[e * NB + ((e * NB) >> 4)];
     }
-    apply_pretw<V, E, Q, NB, TPF>(v, pt, g, t0);
+    apply_pretw<E, Q, NB, TPF>(v, pt, g, t0);
   }
 #pragma unroll
   for (int q = 0; q < Q; q++) {
@@ -289,11 +285,10 @@ __device__ __forceinline__ void smem_stage(V *sm, const V *__restrict__ twR, con
 // Radices up to 2^9 (G >= 8 rows per CTA): the same stages with Ns at run time
 // in one loop -- fully inlined compile-time stages spill there under the
 // 64-register budget of four resident CTAs.
-template <typename V, int LOGR, int G, int E>
+template <typename V, int LOGR, int G, int E, int NT>
 __device__ __forceinline__ void rt_smem_stage(V *sm, const V *__restrict__ twR, int Ns) {
   constexpr int R = 1 << LOGR;
   constexpr int RP = rowpitch<decltype(V().x)>(LOGR);
-  constexpr int NT = imin((R / 16) * G, 512);
   constexpr int TPF = NT / G;
   constexpr int NB = R / E;          // butterflies per row
   constexpr int Q = NB / TPF;        // butterflies per thread
@@ -309,7 +304,7 @@ __device__ __forceinline__ void rt_smem_stage(V *sm, const V *__restrict__ twR, 
       const int k = t % Ns;
       const int step = R / (Ns * E);
       if (sizeof(v[0][0].x) == 8 || E < 4) {
-        // FP64: exact table entries (its FP64 pipe, not shared memory, is the limit)
+        // FP64 (fx_fallback): exact table entries
 #pragma unroll
         for (int e = 1; e < E; e++) v[q][e] = cmul(v[q][e], twR[k * e * step]);
       } else {
@@ -347,15 +342,16 @@ __device__ __forceinline__ void rt_smem_stage(V *sm, const V *__restrict__ twR, 
   __syncthreads();
 }
 
-template <typename V, int LOGR, int G>
+// radix 16 where a thread holds 16 points, radix 8 where it holds 8
+template <typename V, int LOGR, int G, int NT>
 __device__ __forceinline__ void rt_cta_fft(V *sm, const V *__restrict__ twR) {
-  constexpr int LEFT = LOGR % 4;
+  constexpr int LOGE = (1 << LOGR) * G / NT >= 16 ? 4 : 3, LEFT = LOGR % LOGE;
   int Ns = 1;
-  if (LEFT == 1) { rt_smem_stage<V, LOGR, G, 2>(sm, twR, Ns); Ns <<= 1; }
-  if (LEFT == 2) { rt_smem_stage<V, LOGR, G, 4>(sm, twR, Ns); Ns <<= 2; }
-  if (LEFT == 3) { rt_smem_stage<V, LOGR, G, 8>(sm, twR, Ns); Ns <<= 3; }
+  if (LEFT == 1) { rt_smem_stage<V, LOGR, G, 2, NT>(sm, twR, Ns); Ns <<= 1; }
+  if (LEFT == 2) { rt_smem_stage<V, LOGR, G, 4, NT>(sm, twR, Ns); Ns <<= 2; }
+  if (LEFT == 3) { rt_smem_stage<V, LOGR, G, 8, NT>(sm, twR, Ns); Ns <<= 3; }
 #pragma unroll 1
-  for (int s = 0; s < LOGR / 4; s++) { rt_smem_stage<V, LOGR, G, 16>(sm, twR, Ns); Ns <<= 4; }
+  for (int s = 0; s < LOGR / LOGE; s++) { rt_smem_stage<V, LOGR, G, 1 << LOGE, NT>(sm, twR, Ns); Ns <<= LOGE; }
 }
 
 template <typename V, int LOGR, int G, int LOGNS>
@@ -381,8 +377,7 @@ __device__ __forceinline__ void cta_fft(V *sm, const V *__restrict__ twR, const 
 //   w_q = A_(q/4) B_(q mod 4),  A_0 = W^(jm r0), A_m = A_(m-1) W^(4 jm TPF),
 //   B_i = W^(i jm TPF),
 // so w_q is within about q/4 + 4 roundings of its exact value (q < 32).
-// Scattered table reads were the L1 limit of the pass; FP64 keeps exact
-// per-element look-ups.
+// Scattered table reads were the L1 limit of the pass.
 struct TwRun {
   float2 a, s4, b1, b2, b3;
   __device__ __forceinline__ static float2 look(const float2 *thi, const float2 *tlo, int h,
@@ -444,9 +439,7 @@ __device__ __forceinline__ void row_max_update(void *rm, long long b, float v) {
 // 32-byte sectors (G consecutive sub-transforms are adjacent on input, and
 // on output once Ns >= G; with Ns = 1 each sub-transform's outputs are
 // contiguous and 8 lanes write 64 bytes of it).
-template <typename T> __host__ __device__ constexpr bool fused_io(int logr) {
-  return sizeof(T) == 4 && (logr == 11 || logr == 12);
-}
+__host__ __device__ constexpr bool fused_io(int logr) { return logr == 11 || logr == 12; }
 
 // Radix of the first stage of a radix-2^LOGR transform (the remainder stage).
 template <int LOGR> __host__ __device__ constexpr int first_radix() {
@@ -467,7 +460,7 @@ __device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ s
                                                   int inverse) {
   constexpr int R = 1 << LOGR, E = first_radix<LOGR>();
   constexpr int LOGE = E == 2 ? 1 : (E == 4 ? 2 : (E == 8 ? 3 : 4));
-  constexpr int NT = nt_of<float>(LOGR), TPF = NT / G, RP = rowpitch<float>(LOGR);
+  constexpr int NT = nt_of(LOGR), TPF = NT / G, RP = rowpitch<float>(LOGR);
   constexpr int NB = R / E, Q = NB / TPF;
   static_assert(G == 4 && E >= 8 && Q * TPF == NB, "fused first stage: G = 4, radix 8 or 16");
   const int tid = threadIdx.x, g = tid % G;
@@ -486,7 +479,7 @@ __device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ s
 #pragma unroll
     for (int e = 0; e < E; e++) v[q][e] = __ldg(p + q * sq + e * se);
   if (pt.on) {
-    apply_pretw<V, E, Q, NB, TPF>(v, pt, g, t0);  // conjugates too when inverse
+    apply_pretw<E, Q, NB, TPF>(v, pt, g, t0);  // conjugates too when inverse
   } else if (inverse) {
 #pragma unroll
     for (int q = 0; q < Q; q++)
@@ -521,7 +514,7 @@ template <typename T, typename V, int LOGR, int G>
 __device__ __forceinline__ void fused_last_stage(const V *sm, const V *__restrict__ twR, const PassArgs &a,
                                                  long long b, long long d0, int logNs) {
   constexpr int R = 1 << LOGR, E = 16;
-  constexpr int NT = nt_of<T>(LOGR), TPF = NT / G, RP = rowpitch<T>(LOGR);
+  constexpr int NT = nt_of(LOGR), TPF = NT / G, RP = rowpitch<T>(LOGR);
   constexpr int NB = R / E, Q = NB / TPF;
   static_assert(Q * TPF == NB, "fused last stage: whole butterflies per thread");
   const int tid = threadIdx.x, g = tid % G, t0 = tid / G;
@@ -554,16 +547,17 @@ __device__ __forceinline__ void fused_last_stage(const V *sm, const V *__restric
   if (smp && a.row_max) row_max_update(a.row_max, b, tmax);
 }
 
-template <typename T, int LOGR>
-__global__ void __launch_bounds__(nt_of<T>(LOGR), minb_of<T>(LOGR)) fft_pass_kernel(PassArgs a) {
+template <int LOGR>
+__global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(PassArgs a) {
   pdl_enter();
-  typedef typename Cx<T>::V V;
-  constexpr int R = 1 << LOGR, G = g_of<T>(LOGR), NT = nt_of<T>(LOGR), RP = rowpitch<T>(LOGR);
+  typedef float T;
+  typedef float2 V;
+  constexpr int R = 1 << LOGR, G = g_of<T>(LOGR), NT = nt_of(LOGR), RP = rowpitch<T>(LOGR);
   constexpr int ITER = R * G / NT;  // elements per thread in the load / store phases
   extern __shared__ __align__(16) unsigned char smraw[];
   V *sm = reinterpret_cast<V *>(smraw);
   const V *twR = reinterpret_cast<const V *>(a.twR);
-  if (tw_in_smem<T>(LOGR)) {
+  if (tw_in_smem(LOGR)) {
     V *tws = reinterpret_cast<V *>(smraw + data_smem_of<T>(LOGR));
     for (int i = threadIdx.x; i < R; i += NT) tws[i] = twR[i];
     twR = tws;  // made visible by the barrier before the first butterfly stage
@@ -595,12 +589,12 @@ __global__ void __launch_bounds__(nt_of<T>(LOGR), minb_of<T>(LOGR)) fft_pass_ker
   pt.Smask = Smask;
   pt.Nsmask = Nsmask;
   pt.inverse = a.inverse;
-  // FP32 passes after the first fold the conjugation and the inter-pass
+  // passes after the first fold the conjugation and the inter-pass
   // twiddles into their first stage (fast load path; radix 2^11 to 2^13, where
   // the first stage keeps its inputs in registers without spilling)
-  pt.on = LOGR >= 11 && LOGR <= 13 && sizeof(T) == 4 && g_fast_in && !gx && a.nsum <= 1 &&
+  pt.on = LOGR >= 11 && LOGR <= 13 && g_fast_in && !gx && a.nsum <= 1 &&
           logNs > 0;
-  if constexpr (fused_io<T>(LOGR)) {
+  if constexpr (fused_io(LOGR)) {
     // S >= G with both powers of two: the grid covers the batch exactly and
     // all G sub-transforms of a CTA lie in one batch row
     if (g_fast_in && !gx && a.nsum <= 1) {
@@ -640,23 +634,15 @@ __global__ void __launch_bounds__(nt_of<T>(LOGR), minb_of<T>(LOGR)) fft_pass_ker
         if ((a.inverse || logNs > 0) && !pt.on) {
           // each thread rewrites only the elements it loaded: no barrier needed here
           TwRun tr;
-          if constexpr (sizeof(T) == 4)
-            if (logNs > 0)
-              tr.init(reinterpret_cast<const float2 *>(thi), reinterpret_cast<const float2 *>(tlo),
-                      a.tw_h, hmask, jm, r0, TPF);
+          if (logNs > 0)
+            tr.init(reinterpret_cast<const float2 *>(thi), reinterpret_cast<const float2 *>(tlo),
+                    a.tw_h, hmask, jm, r0, TPF);
 #pragma unroll
           for (int q = 0; q < ITER; q++) {
             V *p = dst + q * TPF + ((q * TPF) >> 4);
             V v = *p;
             if (a.inverse) v.y = -v.y;
-            if (logNs > 0) {
-              if constexpr (sizeof(T) == 4) {
-                v = cmul(v, tr.next(q));
-              } else {
-                const long long mm = mm0 + q * dmm;
-                v = cmul(v, cmul(thi[mm >> a.tw_h], tlo[mm & hmask]));
-              }
-            }
+            if (logNs > 0) v = cmul(v, tr.next(q));
             *p = v;
           }
         }
@@ -770,7 +756,7 @@ __global__ void __launch_bounds__(nt_of<T>(LOGR), minb_of<T>(LOGR)) fft_pass_ker
     }
   }
   __syncthreads();
-  if constexpr (LOGR <= 9) rt_cta_fft<V, LOGR, G>(sm, twR);
+  if constexpr (LOGR <= 9) rt_cta_fft<V, LOGR, G, NT>(sm, twR);
   else cta_fft<V, LOGR, G>(sm, twR, pt);
   V *__restrict__ out = reinterpret_cast<V *>(a.out);
   T *__restrict__ smp = reinterpret_cast<T *>(a.samples);
@@ -839,12 +825,12 @@ __global__ void __launch_bounds__(nt_of<T>(LOGR), minb_of<T>(LOGR)) fft_pass_ker
     if (smp && a.row_max && one_row && u0 < a.total) row_max_update(a.row_max, u0 >> logS, tmax);
   }
 }
-template <typename T, int LOGR>
+template <int LOGR>
 int launch_pass(const PassArgs &a, long long total_sub, cudaStream_t st) {
-  constexpr int G = g_of<T>(LOGR), NT = nt_of<T>(LOGR), SM = smem_of<T>(LOGR);
+  constexpr int G = g_of<float>(LOGR), NT = nt_of(LOGR), SM = smem_of(LOGR);
   static PerContext<int> attr;  // per instantiation and CUDA context
   GS_CHECK(attr.ensure_at_least(SM, [](int v) {
-    if (cudaFuncSetAttribute(fft_pass_kernel<T, LOGR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(fft_pass_kernel<LOGR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              v) == cudaSuccess)
       return (int)GSFFT_OK;
     set_last_error("fft_pass_kernel: %d bytes of shared memory refused: %s", v,
@@ -853,7 +839,7 @@ int launch_pass(const PassArgs &a, long long total_sub, cudaStream_t st) {
   }));
   long long grid = (total_sub + G - 1) / G;
   if (grid > 0x7fffffffLL) return GSFFT_ERR_UNSUPPORTED;
-  GS_CUDA(launch_pdl(fft_pass_kernel<T, LOGR>, dim3((unsigned)grid), dim3(NT), SM, st, a));
+  GS_CUDA(launch_pdl(fft_pass_kernel<LOGR>, dim3((unsigned)grid), dim3(NT), SM, st, a));
   GS_LAUNCHED();
   return GSFFT_OK;
 }

@@ -201,6 +201,10 @@ struct FftPlan {
   void *tw_lo[3] = {nullptr, nullptr, nullptr};
   int tw_h[3] = {0, 0, 0};
   void *tw_R[3] = {nullptr, nullptr, nullptr};  // exp(-2 pi i m / R) for the pass radix
+  // FP64: fixed-point twiddles of the pass (fft_pass_fx.cuh)
+  void *fx_tw[3] = {nullptr, nullptr, nullptr};
+  void *fx_hi[3] = {nullptr, nullptr, nullptr};
+  void *fx_lo[3] = {nullptr, nullptr, nullptr};
   bool tc[3] = {false, false, false};  // pass runs on the tensor cores (radix 4096 or 64, FP32)
   void *tc_F = nullptr;                // DFT_64 operand of the tensor-core pass (its layout
                                        // follows the pass: tc_build_F / tc_build_F_smem)
