@@ -113,7 +113,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
       tn.rlfc_first_radix < 0)
     return GSFFT_ERR_PARAM;
   if (tn.perm_filter_form == 1) flags = (flags | GSFFT_FLAG_FORCE_STREAM) & ~GSFFT_FLAG_FORCE_GATHER;
-  if (tn.perm_filter_form == 2) flags = (flags | GSFFT_FLAG_FORCE_GATHER) & ~GSFFT_FLAG_FORCE_STREAM;
+  if (tn.perm_filter_form == 2) flags &= ~GSFFT_FLAG_FORCE_STREAM;
   Plan *P = new Plan();
   P->p = pp;
   P->precision = precision;
@@ -155,11 +155,13 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   {
     const double stream_bytes = (double)p.n * V + 2.0 * p.RLFC_loops * p.W_RLFC * V;
     const double gather_bytes = 80.0 * ((double)p.loops * p.w + (double)p.RLFC_loops * p.W_RLFC);
-    const bool ok = stream_pf_supported(p.n, p.B, p.loops, p.W_RLFC, p.RLFC_loops) &&
-                    p.w / p.B < 32 && !(flags & GSFFT_FLAG_QUIRK_RESIDUE);
-    P->use_stream = ok && !(flags & GSFFT_FLAG_FORCE_GATHER) &&
+    const bool ok = stream_pf_supported(p.n, p.B, p.loops, p.W_RLFC, p.RLFC_loops) && p.w / p.B < 32;
+    P->use_stream = ok && !(flags & GSFFT_FLAG_QUIRK_RESIDUE) && !(flags & GSFFT_FLAG_FORCE_GATHER) && tn.perm_filter_form != 2 &&
                     ((flags & GSFFT_FLAG_FORCE_STREAM) ||
                      (precision == GSFFT_MIXED && stream_bytes < gather_bytes));
+    // FP64: gathers in column order, faster than in bucket order at every size
+    // (pf_cols_kernel).  FP32 lines hold twice the samples: the ordered pass wins there.
+    P->use_cols = ok && precision == GSFFT_FP64 && !P->use_stream && !(flags & GSFFT_FLAG_FORCE_GATHER);
   }
   if (tn.perm_filter_form == 1 && !P->use_stream) {
     plan_destroy(P);
@@ -174,8 +176,10 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
       }
       P->groups = tn.row_groups;
     }
-    A(ybuf, V * (size_t)p.RLFC_loops * p.W_RLFC);
     A(bpart, V * (size_t)P->groups * p.loops * p.B);
+  }
+  if (P->use_stream || P->use_cols) {
+    A(ybuf, V * (size_t)p.RLFC_loops * p.W_RLFC);
     A(filt_bm, V * (size_t)stream_taps_count(p.w, p.B));
   }
 #undef A
@@ -308,7 +312,8 @@ int plan_set_filter(Plan *P, const void *d_ft, const void *d_ff, cudaStream_t st
   const gsfft_params &p = P->p;
   if (!d_ft || !d_ff) return GSFFT_ERR_PARAM;
   GS_CHECK(launch_convert_taps((const double2 *)d_ft, P->filt, p.w, P->precision == GSFFT_MIXED, st));
-  if (P->use_stream) GS_CHECK(launch_stream_taps(P->precision, P->filt, p.w, p.B, P->filt_bm, st));
+  if (P->use_stream || P->use_cols)
+    GS_CHECK(launch_stream_taps(P->precision, P->filt, p.w, p.B, P->filt_bm, st));
   GS_CHECK(launch_hinv((const double2 *)d_ff, p.n, p.n / p.B, P->hinv, st));
   GS_CUDA(cudaStreamSynchronize(st));
   P->filter_set = true;
@@ -395,6 +400,9 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
     GS_CHECK(launch_perm_filter_stream(P->precision, d_x, p.n, P->filt_bm, p.w, p.B, p.loops, d,
                                        P->bpart, p.RLFC_loops, P->ybuf, p.W_RLFC, &P->ctl->err, st,
                                        P->groups));
+  else if (P->use_cols)
+    GS_CHECK(launch_perm_filter_cols(d_x, p.n, P->filt_bm, P->filt, p.w, p.B, p.loops, d, P->bins, p.RLFC_loops,
+                                     P->ybuf, p.W_RLFC, quirk, st));
   else
     GS_CHECK(launch_perm_filter(P->precision, d_x, p.n, P->filt, p.w, p.B, p.loops, d, quirk,
                                 P->bins, st));
@@ -443,7 +451,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   {
     FftIo io;
     const void *src = nullptr;
-    if (P->use_stream) {
+    if (P->use_stream || P->use_cols) {
       src = P->ybuf;
     } else {
       io.gather_x = d_x;  // strided gather fused into the first FFT pass

@@ -40,11 +40,12 @@ struct Plan {
   DevNode *topk = nullptr;
   RunCtl *ctl = nullptr;
   void *rmax = nullptr;  // per-row maxima: RLFC_loops rows then loops rows (u64 each)
-  void *ybuf = nullptr;  // RLFC sub-samples written by the streaming perm+filter
+  void *ybuf = nullptr;  // RLFC sub-samples written by the column-ordered perm+filter forms
   void *bpart = nullptr; // row-group partial bins of the streaming perm+filter
-  void *filt_bm = nullptr; // bucket-major taps of the streaming perm+filter
+  void *filt_bm = nullptr; // bucket-major taps of the column-ordered perm+filter forms
   int groups = 1;
   bool use_stream = false;
+  bool use_cols = false;   // FP64: column-ordered gathers (pf_cols_kernel)
   bool tc_bucket = false;  // bucket FFT with tensor-core passes
   bool tc_rlfc = false;    // RLFC FFT with a tensor-core first pass
   double floor_rel = 1e-10;

@@ -35,7 +35,6 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "stages.cuh"
 
@@ -412,6 +411,109 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
   }
 }
 
+// FP64 form: the same column-ordered walk, with each hit's sample gathered from
+// global memory instead of streamed.
+//
+// What bounds it: DRAM lines.  A 16-byte sample costs its 128-byte line.  In
+// bucket order (pf.cu) the loops * w gathers are random and nearly every one
+// fetches a line of its own: 2.45 GB at n = 2^27, k = 16000, 434 us, and the RLFC
+// rows, gathered by the W-point FFT's first pass, another 1.07 GB.  Here a CTA
+// owns 32 columns (four lines a row); its warps walk the loops of those columns in
+// ascending row order side by side (a barrier every PC_U hits keeps them together:
+// 482 -> 448 us), and its threads copy the RLFC columns at the same pace, so
+// samples that share a line are read close together.  At n = 2^27 the kernel takes
+// 440 us with the RLFC rows in it and the W-point FFT falls from 392 to 297 us; at
+// n = 2^14 .. 2^26 it is faster by itself (27 -> 11, 33 -> 17 at 2^20, 175 -> 107
+// at 2^25, 289 -> 224 us at 2^26), so every FP64 plan whose sizes allow it takes it.
+// Streaming the whole signal through shared memory (pf_tma_kernel) took 489 us at
+// n = 2^27: the divergent hit loop wastes FP64 issue slots (1.73 operations a clock
+// and SM); here every lane has a hit at every step.
+//
+// quirk: the partial tap as permFilterTillKernel indexes it (innerLoop.cu:745-754),
+// id = bucket * tiles + B, from the bucket-order taps qfilt.
+constexpr int PC_U = 3;  // hits in flight per thread
+__global__ void __launch_bounds__(512, 2)
+pf_cols_kernel(const double2 *__restrict__ x, const double2 *__restrict__ filt,
+               const double2 *__restrict__ qfilt, int logn, int logB, int w, int tiles, int L, Draws d,
+               HitTab ht, double2 *__restrict__ bins, int nrlfc, int logsig,
+               double2 *__restrict__ y, int W, int quirk) {
+  pdl_enter();
+  __shared__ unsigned S2[MAXL][2 * MAXT];
+  const int tid = threadIdx.x, lane = tid & 31, l = tid >> 5;
+  const int B = 1 << logB, lognb = logn - logB, nb = 1 << lognb;
+  const unsigned nbm = (unsigned)nb - 1u, nmask = (1u << logn) - 1u;
+  const int TT = taps_per_bucket(tiles);
+  for (int e = lane; e < 2 * MAXT; e += 32) S2[l][e] = e < tiles ? ht.s[l][e] : (e < 2 * tiles ? ht.s[l][e - tiles] : 0u);
+  __syncwarp();
+  const unsigned *S = S2[l];
+  const unsigned c = blockIdx.x * 32u + (unsigned)lane;
+  const unsigned a = (unsigned)d.a[l], beta = ht.beta[l];
+  const unsigned prod = c * a;
+  const int bl = (int)(prod & (unsigned)(B - 1));
+  const unsigned sl = (0u - ((prod & nmask) >> logB) * beta) & nbm;
+  const double2 *fcol = filt + (size_t)bl * TT;
+  const double2 *xcol = x + c;
+  const unsigned long long keep = policy_evict_last();
+  // first sorted entry whose row wraps past nb (pf_tma_kernel)
+  int lo = 0, hi = tiles;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((S[mid] >> 8) < (unsigned)nb - sl) lo = mid + 1;
+    else hi = mid;
+  }
+  // RLFC samples of this block: rows x (loops r) x (columns c = off_r mod n/W)
+  const int logcpr = logsig >= 5 ? 0 : 5 - logsig;  // log2 of a loop's columns in the block
+  const int steps = max((tiles + PC_U - 1) / PC_U, 1);
+  const int total = (nb * nrlfc) << logcpr;
+  const int per = (total + steps - 1) / steps;
+  const int nthr = 32 * L;
+  double re = 0.0, im = 0.0;
+  auto accumulate = [&](double2 xv, double2 f) {
+    re = fma(xv.x, f.x, re);
+    re = fma(-xv.y, f.y, re);
+    im = fma(xv.x, f.y, im);
+    im = fma(xv.y, f.x, im);
+  };
+  int k = 0;
+  for (int st = 0; st < steps; st++, k += PC_U) {
+    __syncthreads();  // keeps the warps on the same rows
+    double2 xv[PC_U], f[PC_U];
+#pragma unroll
+    for (int u = 0; u < PC_U; u++) {
+      if (k + u < tiles) {
+        const int m = lo + k + u;
+        const unsigned ent = S[m];
+        const unsigned row = (ent >> 8) + sl - (m < tiles ? (unsigned)nb : 0u);
+        xv[u] = __ldg(xcol + ((size_t)row << logB));
+        f[u] = ld_tap(fcol + (ent & 255u), keep);
+      }
+    }
+    const int e1 = min((st + 1) * per, total);
+    for (int e = st * per + tid; e < e1; e += nthr) {
+      const int ci = e & ((1 << logcpr) - 1), q = e >> logcpr;
+      const int rr = q % nrlfc, row = q / nrlfc;
+      const unsigned off = (unsigned)d.offs[rr];
+      const unsigned cc = ((off - blockIdx.x * 32u) & ((1u << logsig) - 1u)) + ((unsigned)ci << logsig);
+      if (cc < 32u) {
+        const unsigned t = ((unsigned)row << logB) + blockIdx.x * 32u + cc;
+        y[(size_t)rr * W + ((t - off) >> logsig)] = __ldg(x + t);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < PC_U; u++)
+      if (k + u < tiles) accumulate(xv[u], f[u]);
+  }
+  if (bl < (w & (B - 1))) {  // the partial tap
+    if (quirk && tiles > 0) {
+      const unsigned id = (unsigned)bl * (unsigned)tiles + (unsigned)B;
+      accumulate(__ldg(x + ((id * (unsigned)d.ai[l]) & nmask)), __ldg(qfilt + id));
+    } else {
+      accumulate(__ldg(xcol + ((size_t)((ht.xrow[l] + sl) & nbm) << logB)), ld_tap(fcol + tiles, keep));
+    }
+  }
+  bins[(size_t)l * B + bl] = make_double2(re, im);
+}
+
 // Bucket-major copy of the taps: tb[b * TT + j] = filt[j * B + b] (0 past w).
 template <typename V>
 __global__ void bucket_major_kernel(const V *__restrict__ filt, int w, int B, int TT, V *tb) {
@@ -604,6 +706,34 @@ bool stream_pf_groups_valid(int n, int B, int groups, int precision) {
   return nb / groups >= 4 * stream_rows_per_tile(n, B, precision) && nb % groups == 0;
 }
 
+// sorted hit rows of each loop: j * beta mod nb for j < tiles
+static void hit_table(int n, int B, int tiles, int loops, const Draws &d, HitTab &ht) {
+  const unsigned nbm = (unsigned)(n / B) - 1u;
+  memset(&ht, 0, sizeof(ht));
+  std::pair<unsigned, unsigned> v[MAXT];
+  for (int l = 0; l < loops; l++) {
+    const unsigned alpha = (unsigned)d.a[l] & nbm;
+    const unsigned beta = inv_odd(alpha) & nbm;
+    ht.beta[l] = beta;
+    ht.xrow[l] = ((unsigned)tiles * beta) & nbm;
+    for (int j = 0; j < tiles; j++) v[j] = {((unsigned)j * beta) & nbm, (unsigned)j};
+    std::sort(v, v + tiles);
+    for (int j = 0; j < tiles; j++) ht.s[l][j] = (v[j].first << 8) | v[j].second;
+  }
+}
+
+int launch_perm_filter_cols(const void *x, int n, const void *filt, const void *qfilt, int w, int B, int loops,
+                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st) {
+  if (!stream_pf_supported(n, B, loops, W, nrlfc) || w / B >= MAXT) return GSFFT_ERR_UNSUPPORTED;
+  HitTab ht;
+  hit_table(n, B, w / B, loops, d, ht);
+  GS_CUDA(launch_pdl(pf_cols_kernel, dim3(B / 32), dim3(32 * loops), 0, st, (const double2 *)x,
+                     (const double2 *)filt, (const double2 *)qfilt, ilog2(n), ilog2(B), w, w / B, loops, d, ht,
+                     (double2 *)bins, nrlfc, ilog2(n / W), (double2 *)y, W, quirk ? 1 : 0));
+  GS_LAUNCHED();
+  return GSFFT_OK;
+}
+
 int launch_perm_filter_stream(int precision, const void *x, int n, const void *filt, int w, int B,
                               int loops, const Draws &d, void *bins, int nrlfc, void *y, int W,
                               int *err, cudaStream_t st, int groups_req) {
@@ -612,20 +742,8 @@ int launch_perm_filter_stream(int precision, const void *x, int n, const void *f
   if (tiles >= MAXT || tiles > 255) return GSFFT_ERR_UNSUPPORTED;
   const int logn = ilog2(n), logB = ilog2(B), logsig = ilog2(n / W);
   const int nb = n / B;
-  const unsigned nbm = (unsigned)nb - 1u;
-  // sorted hit rows of each loop: j * beta mod nb for j < tiles
   HitTab ht;
-  memset(&ht, 0, sizeof(ht));
-  std::vector<std::pair<unsigned, unsigned>> v(tiles);
-  for (int l = 0; l < loops; l++) {
-    const unsigned alpha = (unsigned)d.a[l] & nbm;
-    const unsigned beta = inv_odd(alpha) & nbm;
-    ht.beta[l] = beta;
-    ht.xrow[l] = ((unsigned)tiles * beta) & nbm;
-    for (int j = 0; j < tiles; j++) v[j] = {((unsigned)j * beta) & nbm, (unsigned)j};
-    std::sort(v.begin(), v.end());
-    for (int j = 0; j < tiles; j++) ht.s[l][j] = (v[j].first << 8) | v[j].second;
-  }
+  hit_table(n, B, tiles, loops, d, ht);
   // x as a 2-D tensor of 8-byte words: nb rows of B (FP32) or 2B (FP64) words
   const bool dbl = precision == GSFFT_FP64;
   const int es = dbl ? 16 : 8;

@@ -55,6 +55,11 @@ int launch_stream_taps(int precision, const void *filt, int w, int B, void *taps
 int launch_perm_filter_stream(int precision, const void *x, int n, const void *filt, int w, int B,
                               int loops, const Draws &d, void *bins, int nrlfc, void *y, int W,
                               int *err, cudaStream_t st, int groups = 0);
+// The same walk over the columns with gathers instead of a streamed signal, FP64
+// (filt: the bucket-major table; qfilt: the taps in bucket order, for the residue
+// quirk; y as above).
+int launch_perm_filter_cols(const void *x, int n, const void *filt, const void *qfilt, int w, int B, int loops,
+                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st);
 // whether `groups` row groups suit the streaming pass at this shape (one, or
 // a power of two leaving at least four tiles of rows per group)
 bool stream_pf_groups_valid(int n, int B, int groups, int precision);

@@ -61,8 +61,8 @@ typedef enum { GSFFT_FP64 = 0, GSFFT_MIXED = 1 } gsfft_precision;
    (half the RLFC picks of a noiseless signal) tie and resolve by ascending
    index, the reference's tie rule, instead of by FFT rounding noise. */
 #define GSFFT_FLAG_FORCE_GATHER 4u   /* perm+filter by random gathers (one read per
-   tap, innerLoop.cu:725-773 order) even when one ordered pass over the signal
-   would move fewer DRAM bytes */
+   tap, innerLoop.cu:725-773 order) even when gathers in column order (FP64) or one
+   ordered pass over the signal would move fewer DRAM bytes */
 #define GSFFT_FLAG_FORCE_STREAM 8u   /* perm+filter (and the RLFC sub-sampling) by
    one ordered pass over the signal whenever the sizes allow it */
 #define GSFFT_FLAG_TC_BUCKET_FFT 16u /* MIXED: the B-point bucket FFT with a
