@@ -385,7 +385,7 @@ int gsfft_fft(const void *d_in, void *d_out, long long n_fft, int batch, int sig
   if (!d_in || !d_out || batch < 1 || (sign != 1 && sign != -1)) return GSFFT_ERR_PARAM;
   if (precision != GSFFT_FP64 && precision != GSFFT_MIXED) return GSFFT_ERR_PARAM;
   FftPlan fp;
-  int s = fft_plan_init(fp, n_fft, precision, batch);
+  int s = fft_plan_init(fp, n_fft, precision == GSFFT_FP64 ? FFT_FP64 : FFT_FP32, batch, S(stream));
   if (s == GSFFT_OK) {
     FftIo io;
     s = fft_exec(fp, d_in, d_out, batch, sign, io, S(stream));
@@ -421,11 +421,11 @@ int gsfft_check_bounded_wait(long long limit_cycles, void *stream) {
 }
 
 // an FP32 FFT with one of the tensor-core plans (its completion waits checked)
-static int fft_tc_run(int (*init)(FftPlan &, long long, int), const char *what, const void *d_in,
+static int fft_tc_run(FftKind kind, const char *what, const void *d_in,
                       void *d_out, long long n_fft, int batch, int sign, void *stream) {
   if (!d_in || !d_out || batch < 1 || (sign != 1 && sign != -1)) return GSFFT_ERR_PARAM;
   FftPlan fp;
-  int s = init(fp, n_fft, batch);
+  int s = fft_plan_init(fp, n_fft, kind, batch, S(stream));
   if (s == GSFFT_OK) {
     int *err = nullptr;
     if (cudaMalloc(&err, sizeof(int)) != cudaSuccess) {
@@ -455,12 +455,12 @@ static int fft_tc_run(int (*init)(FftPlan &, long long, int), const char *what, 
 
 int gsfft_fft_tc(const void *d_in, void *d_out, long long n_fft, int batch, int sign,
                  void *stream) {
-  return fft_tc_run(fft_plan_init_tc, "gsfft_fft_tc", d_in, d_out, n_fft, batch, sign, stream);
+  return fft_tc_run(FFT_FP32_TC, "gsfft_fft_tc", d_in, d_out, n_fft, batch, sign, stream);
 }
 
 int gsfft_fft_tc64(const void *d_in, void *d_out, long long n_fft, int batch, int sign,
                    void *stream) {
-  return fft_tc_run(fft_plan_init_tc64, "gsfft_fft_tc64", d_in, d_out, n_fft, batch, sign, stream);
+  return fft_tc_run(FFT_FP32_TC64, "gsfft_fft_tc64", d_in, d_out, n_fft, batch, sign, stream);
 }
 
 int gsfft_cutoff(const void *d_samples, int size, int num, int batch, int precision, int *d_out,
@@ -469,7 +469,10 @@ int gsfft_cutoff(const void *d_samples, int size, int num, int batch, int precis
       (precision != GSFFT_FP64 && precision != GSFFT_MIXED))
     return GSFFT_ERR_PARAM;
   SelectScratch ss;
-  int s = select_scratch_init(ss, batch, size);
+  Arena mem;
+  void *block = nullptr;
+  select_scratch_request(ss, batch, size, mem);
+  int s = mem.commit(&block, S(stream));
   if (s == GSFFT_OK)
     s = select_top(d_samples, precision == GSFFT_FP64 ? 8 : 4, size, nullptr, num, batch, size,
                    d_out, num, nullptr, ss, S(stream));
@@ -477,7 +480,7 @@ int gsfft_cutoff(const void *d_samples, int size, int num, int batch, int precis
     set_last_error("gsfft_cutoff: %s", cudaGetErrorString(cudaGetLastError()));
     s = GSFFT_ERR_CUDA;
   }
-  select_scratch_free(ss);
+  if (block) cudaFree(block);
   return s;
 }
 
@@ -490,24 +493,22 @@ int gsfft_cutoff_floor(const void *d_samples, int size, int num, int batch, int 
     return GSFFT_ERR_PARAM;
   const int kb = precision == GSFFT_FP64 ? 8 : 4;
   cudaStream_t st = S(stream);
-  void *rmax = nullptr;
+  void *rmax = nullptr, *block = nullptr;
   SelectScratch ss;
-  int s = select_scratch_init(ss, batch, size);
-  if (s == GSFFT_OK && !d_row_max && floor_rel > 0.0) {
-    if (cudaMalloc(&rmax, (size_t)kb * batch) != cudaSuccess) {
-      s = GSFFT_ERR_ALLOC;
-    } else if (cudaMemsetAsync(rmax, 0, (size_t)kb * batch, st) != cudaSuccess) {
-      s = GSFFT_ERR_CUDA;
-    } else {
-      const int chunks = (int)((size + 65535) / 65536);
-      if (kb == 8)
-        row_max_kernel<unsigned long long><<<batch * chunks, 256, 0, st>>>(
-            (const unsigned long long *)d_samples, size, chunks, (unsigned long long *)rmax);
-      else
-        row_max_kernel<unsigned><<<batch * chunks, 256, 0, st>>>((const unsigned *)d_samples, size,
-                                                                  chunks, (unsigned *)rmax);
-      if (cudaGetLastError() != cudaSuccess) s = GSFFT_ERR_CUDA;
-    }
+  Arena mem;
+  select_scratch_request(ss, batch, size, mem);
+  const bool find_max = !d_row_max && floor_rel > 0.0;
+  if (find_max) mem.add(&rmax, (size_t)kb * batch, true);
+  int s = mem.commit(&block, st);
+  if (s == GSFFT_OK && find_max) {
+    const int chunks = (int)((size + 65535) / 65536);
+    if (kb == 8)
+      row_max_kernel<unsigned long long><<<batch * chunks, 256, 0, st>>>(
+          (const unsigned long long *)d_samples, size, chunks, (unsigned long long *)rmax);
+    else
+      row_max_kernel<unsigned><<<batch * chunks, 256, 0, st>>>((const unsigned *)d_samples, size,
+                                                                chunks, (unsigned *)rmax);
+    if (cudaGetLastError() != cudaSuccess) s = GSFFT_ERR_CUDA;
   }
   if (s == GSFFT_OK)
     s = select_top(d_samples, kb, size, nullptr, num, batch, size, d_out, num, nullptr, ss, st,
@@ -516,8 +517,7 @@ int gsfft_cutoff_floor(const void *d_samples, int size, int num, int batch, int 
     set_last_error("gsfft_cutoff_floor: %s", cudaGetErrorString(cudaGetLastError()));
     s = GSFFT_ERR_CUDA;
   }
-  if (rmax) cudaFree(rmax);
-  select_scratch_free(ss);
+  if (block) cudaFree(block);
   return s;
 }
 
@@ -797,10 +797,13 @@ struct EvTimer {  // adds the elapsed seconds of a section to *acc
 
 int cutoff_device(const double *d_s, int size, int num, int *d_out) {
   SelectScratch ss;
-  int s = select_scratch_init(ss, 1, size);
+  Arena mem;
+  void *block = nullptr;
+  select_scratch_request(ss, 1, size, mem);
+  int s = mem.commit(&block, 0);
   if (s == GSFFT_OK) s = select_top(d_s, 8, size, nullptr, num, 1, size, d_out, num, nullptr, ss, 0);
   if (s == GSFFT_OK) s = sync_check(0, "cutoff");
-  select_scratch_free(ss);
+  if (block) cudaFree(block);
   return s;
 }
 }  // namespace
@@ -814,7 +817,7 @@ int restr_loc_freq_coeff(complex_t *d_x, int n, int B_thresh, int W_RLFC, int *d
   const int offset = (int)(unsigned)floor(drand48() * sigma);  /* innerLoop.cu:123 */
   FftPlan fp;
   double *s_d = nullptr;
-  int s = fft_plan_init(fp, W_RLFC, GSFFT_FP64, 1);
+  int s = fft_plan_init(fp, W_RLFC, FFT_FP64, 1, 0);
   if (s == GSFFT_OK && cudaMalloc(&s_d, sizeof(double) * W_RLFC) != cudaSuccess) s = GSFFT_ERR_ALLOC;
   if (s == GSFFT_OK) {
     FftIo io;
@@ -860,7 +863,7 @@ int perm_filter_cutoff(complex_t *d_x, int n, complex_t *d_filter_time, int d_fi
   EvTimer tm(BC_T);
   FftPlan fp;
   double *s_d = nullptr;
-  s = fft_plan_init(fp, B, GSFFT_FP64, 1);
+  s = fft_plan_init(fp, B, FFT_FP64, 1, 0);
   if (s == GSFFT_OK && cudaMalloc(&s_d, sizeof(double) * B) != cudaSuccess) s = GSFFT_ERR_ALLOC;
   if (s == GSFFT_OK) {
     FftIo io;

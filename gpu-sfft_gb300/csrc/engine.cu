@@ -74,15 +74,6 @@ __global__ void hinv_kernel(const double2 *__restrict__ ff, int n, int nb, doubl
   reinterpret_cast<float2 *>(hinv + nb + 1)[idx] = make_float2((float)v.x, (float)v.y);
 }
 
-template <typename P> int alloc(P **p, size_t bytes) {
-  cudaError_t e = cudaMalloc((void **)p, bytes ? bytes : 16);
-  if (e != cudaSuccess) {
-    set_last_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
-    return GSFFT_ERR_ALLOC;
-  }
-  return GSFFT_OK;
-}
-
 }  // namespace
 
 int validate_params(const gsfft_params &p) {
@@ -125,8 +116,9 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   int s = GSFFT_OK;
   const int nb = p.n / p.B;
   const size_t wW = (size_t)p.W_RLFC / 32;
-#define A(ptr, bytes) \
-  if (s == GSFFT_OK) s = alloc(&P->ptr, (bytes))
+  Arena mem;
+#define A(ptr, bytes) mem.add(&P->ptr, (bytes))
+#define A0(ptr, bytes) mem.add(&P->ptr, (bytes), true)
   A(filt, V * p.w);
   A(hinv, hinv_bytes(nb));
   A(rsamp, T * (size_t)p.RLFC_loops * p.W_RLFC);
@@ -138,7 +130,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   A(bm_j2, sizeof(unsigned) * wW);
   A(bm_sig, sizeof(unsigned) * wW * p.loops_loc);
   A(tile_tmp, sizeof(unsigned) * (wW / 2048 + 2));
-  A(vote, sizeof(unsigned) * (size_t)p.n);
+  A0(vote, sizeof(unsigned) * (size_t)p.n);
   A(cand, sizeof(int) * (size_t)P->cap);
   A(cnt, sizeof(int) * (size_t)p.B_thresh);
   A(blk, sizeof(int) * (size_t)vote_block_ints(p.B_thresh));
@@ -146,8 +138,8 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   A(mag2, sizeof(double) * (size_t)P->cap);
   A(topk_idx, sizeof(int) * (size_t)p.k + 16);
   A(topk, sizeof(DevNode) * (size_t)p.k + 16);
-  A(ctl, sizeof(RunCtl));
-  A(d_epoch, sizeof(unsigned) * 4);
+  A0(ctl, sizeof(RunCtl));
+  A0(d_epoch, sizeof(unsigned) * 4);
   A(d_draws, sizeof(Draws));
   A(rmax, sizeof(unsigned long long) * (size_t)(p.RLFC_loops + p.loops));
   // perm+filter form: one ordered pass over x when that moves fewer DRAM bytes
@@ -183,9 +175,11 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     A(filt_bm, V * (size_t)stream_taps_count(p.w, p.B));
   }
 #undef A
+#undef A0
   P->floor_rel = (flags & GSFFT_FLAG_RAW_SELECTION) ? 0.0 : 1e-10;
   // 2-bit vote counters (n/4 bytes, L2-resident) when no count can pass 3
   P->packed_vote = p.loops_loc <= 3;
+  const FftKind kind = precision == GSFFT_FP64 ? FFT_FP64 : FFT_FP32;
   if (s == GSFFT_OK) {
     int t = GSFFT_ERR_UNSUPPORTED;
     // tensor-core bucket FFT: the radix-64 last pass where B allows it
@@ -196,11 +190,11 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     const bool tc_asked = (flags & GSFFT_FLAG_TC_BUCKET_FFT) != 0;
     const bool tc_default = !(flags & GSFFT_FLAG_CC_BUCKET_FFT) && p.B >= (1 << 17) && p.B <= (1 << 20);
     if (precision == GSFFT_MIXED && (tc_asked || tc_default)) {
-      t = fft_plan_init_tc64(P->fftB, p.B, p.loops);
-      if (t == GSFFT_ERR_UNSUPPORTED && tc_asked) t = fft_plan_init_tc(P->fftB, p.B, p.loops);
+      t = fft_plan_shape(P->fftB, p.B, FFT_FP32_TC64);
+      if (t == GSFFT_ERR_UNSUPPORTED && tc_asked) t = fft_plan_shape(P->fftB, p.B, FFT_FP32_TC);
     }
     P->tc_bucket = t == GSFFT_OK;
-    if (!P->tc_bucket) s = fft_plan_init(P->fftB, p.B, precision, p.loops, tn.bucket_first_radix);
+    if (!P->tc_bucket) s = fft_plan_shape(P->fftB, p.B, kind, tn.bucket_first_radix);
   }
   if (s == GSFFT_OK) {
     // the RLFC transform reads the streaming pass's sub-samples; its first
@@ -208,14 +202,20 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     // gather into that pass instead)
     int t = GSFFT_ERR_UNSUPPORTED;
     if (precision == GSFFT_MIXED && (flags & GSFFT_FLAG_TC_RLFC_FFT) && P->use_stream)
-      t = fft_plan_init_tc(P->fftW, p.W_RLFC, p.RLFC_loops);
+      t = fft_plan_shape(P->fftW, p.W_RLFC, FFT_FP32_TC);
     P->tc_rlfc = t == GSFFT_OK;
-    if (!P->tc_rlfc)
-      s = fft_plan_init(P->fftW, p.W_RLFC, precision, p.RLFC_loops, tn.rlfc_first_radix);
+    if (!P->tc_rlfc) s = fft_plan_shape(P->fftW, p.W_RLFC, kind, tn.rlfc_first_radix);
   }
-  if (s == GSFFT_OK) s = select_scratch_init(P->selB, p.loops_loc, p.B);
-  if (s == GSFFT_OK) s = select_scratch_init(P->selW, p.RLFC_loops, p.W_RLFC);
-  if (s == GSFFT_OK) s = select_scratch_init(P->selK, 1, P->cap);
+  if (s == GSFFT_OK) {
+    fft_plan_request(P->fftB, p.loops, mem);
+    fft_plan_request(P->fftW, p.RLFC_loops, mem);
+    select_scratch_request(P->selB, p.loops_loc, p.B, mem);
+    select_scratch_request(P->selW, p.RLFC_loops, p.W_RLFC, mem);
+    select_scratch_request(P->selK, 1, P->cap, mem);
+    s = mem.commit(&P->mem, 0);
+  }
+  if (s == GSFFT_OK) s = fft_plan_fill(P->fftB, 0);
+  if (s == GSFFT_OK) s = fft_plan_fill(P->fftW, 0);
   P->selB.single_launch = P->selW.single_launch = P->selK.single_launch = tn.select_form != 2;
   // record the shapes in use
   P->tuning.perm_filter_form = P->use_stream ? 1 : 2;
@@ -236,10 +236,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     s = GSFFT_ERR_CUDA;
   }
   if (s == GSFFT_OK) {
-    cudaError_t e = cudaMemset(P->vote, 0, sizeof(unsigned) * (size_t)p.n);
-    if (e == cudaSuccess) e = cudaMemset(P->ctl, 0, sizeof(RunCtl));
-    if (e == cudaSuccess) e = cudaMemset(P->d_epoch, 0, sizeof(unsigned) * 4);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    const cudaError_t e = cudaDeviceSynchronize();  // tables and clears, before any stream uses them
     if (e != cudaSuccess) {
       set_last_error("plan init: %s", cudaGetErrorString(e));
       s = GSFFT_ERR_CUDA;
@@ -256,12 +253,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
 
 void plan_destroy(Plan *P) {
   if (!P) return;
-  void *ptrs[] = {P->filt, P->hinv, P->rsamp, P->J2b, P->J2, P->bins, P->bsamp, P->J,
-                  P->bm_j2, P->bm_sig, P->tile_tmp, P->vote, P->cand, P->cnt, P->blk,
-                  P->nodes, P->mag2, P->topk_idx, P->topk, P->ctl, P->rmax, P->ybuf, P->bpart,
-                  P->filt_bm, P->d_epoch, P->d_draws};
-  for (void *q : ptrs)
-    if (q) cudaFree(q);
+  if (P->mem) cudaFree(P->mem);
   for (cudaEvent_t e : P->events) cudaEventDestroy(e);
   if (P->ev_fork) cudaEventDestroy(P->ev_fork);
   if (P->ev_join) cudaEventDestroy(P->ev_join);
@@ -271,11 +263,6 @@ void plan_destroy(Plan *P) {
   if (P->ev_voted) cudaEventDestroy(P->ev_voted);
   if (P->aux) cudaStreamDestroy(P->aux);
   if (P->side) cudaStreamDestroy(P->side);
-  fft_plan_free(P->fftB);
-  fft_plan_free(P->fftW);
-  select_scratch_free(P->selB);
-  select_scratch_free(P->selW);
-  select_scratch_free(P->selK);
   delete P;
 }
 

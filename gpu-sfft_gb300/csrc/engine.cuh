@@ -22,6 +22,7 @@ struct Plan {
   unsigned epoch = 0;            // host mirror of *d_epoch after the last queued run
   unsigned *d_epoch = nullptr;   // device copy, advanced by each run's first kernel
   int launches_per_run = 0;
+  void *mem = nullptr;           // the one allocation that holds every buffer below
   FftPlan fftB, fftW;
   SelectScratch selB, selW, selK;
   void *filt = nullptr;

@@ -9,64 +9,57 @@ namespace gsfft {
 
 namespace {
 
-// exp(-2 pi i m / Np) for m in [0, count) at spacing `mul`
-template <typename V>
-__global__ void twiddle_table_kernel(V *t, long long count, long long mul, long long Np) {
-  long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= count) return;
-  double s, c;
-  // angle 2*pi*(m*mul)/Np, reduced exactly in integers
-  long long num = (m * mul) % Np;
-  sincospi(2.0 * (double)num / (double)Np, &s, &c);
-  t[m].x = (decltype(t[m].x))c;
-  t[m].y = (decltype(t[m].y))(-s);
-}
+// The tables of a plan, all built by one launch.
+enum TableKind { TAB_F32, TAB_F64, TAB_FX_STAGES, TAB_FX_HI, TAB_FX_LO };
+struct TableJob {
+  void *dst;
+  int kind, count, block;  // block: first block of the job
+  int lg;                  // angles in units of 2 pi / 2^lg
+  int shift;               // entry m has angle m << shift (F32, F64, FX_HI, FX_LO)
+  int logr;                // FX_STAGES: log2 of the pass's radix
+};
+constexpr int MAX_JOBS = 3 * 6;
+struct TableJobs {
+  TableJob j[MAX_JOBS];
+  int n, blocks;
+};
 
-template <typename T>
-int make_table(void **dst, long long count, long long mul, long long Np) {
-  typedef typename Cx<T>::V V;
-  GS_CUDA(cudaMalloc(dst, sizeof(V) * count));
-  twiddle_table_kernel<V><<<(unsigned)((count + 255) / 256), 256>>>((V *)*dst, count, mul, Np);
-  GS_LAUNCHED();
-  return GSFFT_OK;
-}
-
-// Fixed-point twiddles of an FP64 pass of radix 2^logr that reaches Np = 2^lg
-// points: the radix-16 stages' rows [e][k] = exp(-2 pi i e k / (16 Ns)) scaled by
-// 2^60, and exp(-2 pi i m / Np) as hi[m >> h] lo[m & (2^h - 1)] scaled by 2^62.
-// One launch: threads [0, ntw) the stage rows, then hi, then lo.
-__global__ void fx_tables_kernel(int logr, int lg, int h, int ntw, int nhi, int nlo, fx::Tw *tw,
-                                 longlong2 *hi, fx::Tw *lo) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ntw) {
-    int logns = logr % 4 == 0 ? 4 : logr % 4;
-    const int at = i;
-    while (i >= (16 << logns)) {
-      i -= 16 << logns;
+// F32, F64: exp(-2 pi i (m << shift) / 2^lg), the angle reduced exactly in
+// integers.  FP64 passes' fixed-point twiddles: FX_STAGES the radix-16 stages' rows
+// [e][k] = exp(-2 pi i e k / (16 Ns)) scaled by 2^60; FX_HI, FX_LO two-level
+// tables scaled by 2^62.
+__global__ void tables_kernel(TableJobs jobs) {
+  int q = jobs.n - 1;
+  while (q > 0 && (int)blockIdx.x < jobs.j[q].block) q--;
+  const TableJob &t = jobs.j[q];
+  const int i = ((int)blockIdx.x - t.block) * 256 + (int)threadIdx.x;
+  if (i >= t.count) return;
+  if (t.kind == TAB_F32 || t.kind == TAB_F64) {
+    const long long N = 1LL << t.lg, num = ((long long)i << t.shift) & (N - 1);
+    double s, c;
+    sincospi(2.0 * (double)num / (double)N, &s, &c);
+    if (t.kind == TAB_F32) reinterpret_cast<float2 *>(t.dst)[i] = make_float2((float)c, (float)(-s));
+    else reinterpret_cast<double2 *>(t.dst)[i] = make_double2(c, -s);
+  } else if (t.kind == TAB_FX_STAGES) {
+    int logns = t.logr % 4 == 0 ? 4 : t.logr % 4, at = i;
+    while (at >= (16 << logns)) {
+      at -= 16 << logns;
       logns += 4;
     }
-    const unsigned e = (unsigned)i >> logns, k = (unsigned)i & ((1u << logns) - 1u);
+    const unsigned e = (unsigned)at >> logns, k = (unsigned)at & ((1u << logns) - 1u);
     const fx::C64 w = fx::unit_root((unsigned long long)e * k, logns + 4);
-    tw[at] = fx::limbs(fx::C64{(w.x + 2) >> 2, (w.y + 2) >> 2});
-  } else if (i < ntw + nhi) {
-    const fx::C64 w = fx::unit_root((unsigned long long)(i - ntw) << h, lg);
-    hi[i - ntw] = make_longlong2(w.x, w.y);
-  } else if (i < ntw + nhi + nlo) {
-    lo[i - ntw - nhi] = fx::limbs(fx::unit_root((unsigned long long)(i - ntw - nhi), lg));
+    reinterpret_cast<fx::Tw *>(t.dst)[i] = fx::limbs(fx::C64{(w.x + 2) >> 2, (w.y + 2) >> 2});
+  } else {
+    const fx::C64 w = fx::unit_root((unsigned long long)i << t.shift, t.lg);
+    if (t.kind == TAB_FX_HI) reinterpret_cast<longlong2 *>(t.dst)[i] = make_longlong2(w.x, w.y);
+    else reinterpret_cast<fx::Tw *>(t.dst)[i] = fx::limbs(w);
   }
 }
 
-int make_fx_tables(FftPlan &p, int i, int lg) {
-  int ntw = 0;
-  for (int l = p.logR[i] % 4 == 0 ? 4 : p.logR[i] % 4; l < p.logR[i]; l += 4) ntw += 16 << l;
-  const int h = p.tw_h[i], nlo = 1 << h, nhi = 1 << (lg - h);
-  GS_CUDA(cudaMalloc(&p.fx_tw[i], sizeof(fx::Tw) * ntw));
-  GS_CUDA(cudaMalloc(&p.fx_hi[i], sizeof(longlong2) * nhi));
-  GS_CUDA(cudaMalloc(&p.fx_lo[i], sizeof(fx::Tw) * nlo));
-  fx_tables_kernel<<<(ntw + nhi + nlo + 127) / 128, 128>>>(p.logR[i], lg, h, ntw, nhi, nlo, (fx::Tw *)p.fx_tw[i],
-                                                          (longlong2 *)p.fx_hi[i], (fx::Tw *)p.fx_lo[i]);
-  GS_LAUNCHED();
-  return GSFFT_OK;
+int fx_stage_entries(int logr) {
+  int n = 0;
+  for (int l = logr % 4 == 0 ? 4 : logr % 4; l < logr; l += 4) n += 16 << l;
+  return n;
 }
 
 int dispatch_pass(bool dbl, int logr, const PassArgs &a, long long total_sub, cudaStream_t st) {
@@ -76,165 +69,134 @@ int dispatch_pass(bool dbl, int logr, const PassArgs &a, long long total_sub, cu
 
 }  // namespace
 
-int fft_plan_init(FftPlan &p, long long n, int precision, int max_batch, int first_logr) {
-  fft_plan_free(p);
+int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr) {
+  p = FftPlan();
   if (n < 256 || (n & (n - 1)) != 0) return GSFFT_ERR_UNSUPPORTED;
   int L = 0;
   while ((1LL << L) < n) L++;
-  const int one_pass_max = precision == GSFFT_FP64 ? 13 : 14;
-  p.n = n;
-  p.L = L;
-  p.precision = precision;
-  if (L <= one_pass_max) {
+  const int one_pass_max = kind == FFT_FP64 ? 13 : 14;
+  int r[3] = {0, 0, 0}, npass = 0;
+  if (kind == FFT_FP32_TC) {
+    // the second pass is a CUDA-core pass of radix 2^(L-12)
+    if (L - 12 < 5 || L - 12 > 14) return GSFFT_ERR_UNSUPPORTED;
+    npass = 2;
+    r[0] = 12;
+    r[1] = L - 12;
+    p.tc[0] = true;
+  } else if (kind == FFT_FP32_TC64) {
+    if (L < 13 || L > 20) return GSFFT_ERR_UNSUPPORTED;
+    npass = 2;
+    r[0] = L - 6;
+    r[1] = 6;
+    p.tc[1] = true;
+  } else if (L <= one_pass_max) {
     if (first_logr > 0) return GSFFT_ERR_PARAM;  // one pass: no first radix to choose
-    p.npass = 1;
-    p.logR[0] = L;
+    npass = 1;
+    r[0] = L;
   } else if (L <= 24) {
-    p.npass = 2;
-    p.logR[0] = (L + 1) / 2;
+    npass = 2;
+    r[0] = (L + 1) / 2;
     if (first_logr > 0) {
       if (first_logr < 7 || first_logr > one_pass_max || L - first_logr < 7 ||
           L - first_logr > one_pass_max)
         return GSFFT_ERR_PARAM;
-      p.logR[0] = first_logr;
+      r[0] = first_logr;
     }
-    p.logR[1] = L - p.logR[0];
+    r[1] = L - r[0];
   } else if (L <= 36) {
     if (first_logr > 0) return GSFFT_ERR_PARAM;
-    p.npass = 3;
-    p.logR[0] = (L + 2) / 3;
-    p.logR[1] = (L - p.logR[0] + 1) / 2;
-    p.logR[2] = L - p.logR[0] - p.logR[1];
+    npass = 3;
+    r[0] = (L + 2) / 3;
+    r[1] = (L - r[0] + 1) / 2;
+    r[2] = L - r[0] - r[1];
   } else {
     return GSFFT_ERR_UNSUPPORTED;
   }
-  for (int i = 0; i < p.npass; i++)
-    if (p.logR[i] < 7 || p.logR[i] > one_pass_max) return GSFFT_ERR_UNSUPPORTED;
-  const bool dbl = precision == GSFFT_FP64;
-  long long Np = 1;
+  if (kind == FFT_FP64 || kind == FFT_FP32)
+    for (int i = 0; i < npass; i++)
+      if (r[i] < 7 || r[i] > one_pass_max) return GSFFT_ERR_UNSUPPORTED;
+  p.n = n;
+  p.L = L;
+  p.precision = kind == FFT_FP64 ? GSFFT_FP64 : GSFFT_MIXED;
+  p.npass = npass;
+  int lg = 0;
+  for (int i = 0; i < npass; i++) {
+    p.logR[i] = r[i];
+    lg += r[i];
+    p.tw_h[i] = (lg + 1) / 2;
+  }
+  return GSFFT_OK;
+}
+
+void fft_plan_request(FftPlan &p, int max_batch, Arena &mem) {
+  const bool dbl = p.precision == GSFFT_FP64;
+  const size_t es = dbl ? sizeof(double2) : sizeof(float2);
+  int lg = 0;
   for (int i = 0; i < p.npass; i++) {
-    const long long R = 1LL << p.logR[i];
-    Np *= R;
-    int lg = 0;
-    while ((1LL << lg) < Np) lg++;
-    const int h = (lg + 1) / 2;
-    p.tw_h[i] = h;
-    const long long nlo = 1LL << h, nhi = (Np + nlo - 1) / nlo;
+    lg += p.logR[i];
+    const size_t nlo = (size_t)1 << p.tw_h[i], nhi = (size_t)1 << (lg - p.tw_h[i]);
+    mem.add(&p.tw_lo[i], es * nlo);
+    mem.add(&p.tw_hi[i], es * nhi);
+    mem.add(&p.tw_R[i], es << p.logR[i]);
     if (dbl) {
-      GS_CHECK(make_table<double>(&p.tw_lo[i], nlo, 1, Np));
-      GS_CHECK(make_table<double>(&p.tw_hi[i], nhi, nlo, Np));
-      GS_CHECK(make_table<double>(&p.tw_R[i], R, 1, R));
-      GS_CHECK(make_fx_tables(p, i, lg));
-    } else {
-      GS_CHECK(make_table<float>(&p.tw_lo[i], nlo, 1, Np));
-      GS_CHECK(make_table<float>(&p.tw_hi[i], nhi, nlo, Np));
-      GS_CHECK(make_table<float>(&p.tw_R[i], R, 1, R));
+      mem.add(&p.fx_tw[i], sizeof(fx::Tw) * fx_stage_entries(p.logR[i]));
+      mem.add(&p.fx_hi[i], sizeof(longlong2) * nhi);
+      mem.add(&p.fx_lo[i], sizeof(fx::Tw) * nlo);
     }
   }
+  if (p.tc[0]) mem.add(&p.tc_F, tc_F_bytes());
+  if (p.tc[1]) mem.add(&p.tc_F, tc_F_smem_bytes());
   if (p.npass > 1) {
-    const size_t es = dbl ? 16 : 8;
-    p.scratch_elems = (long long)n * max_batch * (p.npass == 3 ? 2 : 1);
-    GS_CUDA(cudaMalloc(&p.scratch, es * p.scratch_elems));
+    p.scratch_elems = p.n * max_batch * (p.npass == 3 ? 2 : 1);
+    mem.add(&p.scratch, es * p.scratch_elems);
   }
-  GS_CUDA(cudaDeviceSynchronize());
+}
+
+int fft_plan_fill(const FftPlan &p, cudaStream_t st) {
+  const bool dbl = p.precision == GSFFT_FP64;
+  TableJobs jobs;
+  jobs.n = jobs.blocks = 0;
+  auto add = [&](void *dst, int kind, int count, int lg, int shift, int logr) {
+    jobs.j[jobs.n++] = TableJob{dst, kind, count, jobs.blocks, lg, shift, logr};
+    jobs.blocks += (count + 255) / 256;
+  };
+  int lg = 0;
+  for (int i = 0; i < p.npass; i++) {
+    lg += p.logR[i];
+    const int h = p.tw_h[i], nlo = 1 << h, nhi = 1 << (lg - h), kind = dbl ? TAB_F64 : TAB_F32;
+    add(p.tw_lo[i], kind, nlo, lg, 0, 0);
+    add(p.tw_hi[i], kind, nhi, lg, h, 0);
+    add(p.tw_R[i], kind, 1 << p.logR[i], p.logR[i], 0, 0);
+    if (dbl) {
+      add(p.fx_tw[i], TAB_FX_STAGES, fx_stage_entries(p.logR[i]), 0, 0, p.logR[i]);
+      add(p.fx_hi[i], TAB_FX_HI, nhi, lg, h, 0);
+      add(p.fx_lo[i], TAB_FX_LO, nlo, lg, 0, 0);
+    }
+  }
+  tables_kernel<<<jobs.blocks, 256, 0, st>>>(jobs);
+  GS_LAUNCHED();
+  if (p.tc[0]) GS_CHECK(tc_build_F(p.tc_F, st));
+  if (p.tc[1]) GS_CHECK(tc_build_F_smem(p.tc_F, st));
   return GSFFT_OK;
 }
 
-// FP32 plan whose first pass is a radix-4096 tensor-core pass (two DFT_64
-// stages; its outputs are then contiguous) and whose second is a CUDA-core
-// pass of radix 2^(L-12): n = 2^L, 5 <= L-12 <= 14.
-int fft_plan_init_tc(FftPlan &p, long long n, int max_batch) {
+int fft_plan_init(FftPlan &p, long long n, FftKind kind, int max_batch, cudaStream_t st) {
   fft_plan_free(p);
-  if (n < 256 || (n & (n - 1)) != 0) return GSFFT_ERR_UNSUPPORTED;
-  int L = 0;
-  while ((1LL << L) < n) L++;
-  if (L - 12 < 5 || L - 12 > 14) return GSFFT_ERR_UNSUPPORTED;
-  p.n = n;
-  p.L = L;
-  p.precision = GSFFT_MIXED;
-  p.npass = 2;
-  p.logR[0] = 12;
-  p.logR[1] = L - 12;
-  p.tc[0] = true;
-  p.tc[1] = false;
-  long long Np = 1;
-  for (int i = 0; i < p.npass; i++) {
-    const long long R = 1LL << p.logR[i];
-    Np *= R;
-    int lg = 0;
-    while ((1LL << lg) < Np) lg++;
-    const int h = (lg + 1) / 2;
-    p.tw_h[i] = h;
-    const long long nlo = 1LL << h, nhi = (Np + nlo - 1) / nlo;
-    GS_CHECK(make_table<float>(&p.tw_lo[i], nlo, 1, Np));
-    GS_CHECK(make_table<float>(&p.tw_hi[i], nhi, nlo, Np));
-    GS_CHECK(make_table<float>(&p.tw_R[i], R, 1, R));
-  }
-  GS_CHECK(tc_build_F(&p.tc_F));
-  p.scratch_elems = (long long)n * max_batch;
-  GS_CUDA(cudaMalloc(&p.scratch, sizeof(float2) * p.scratch_elems));
-  GS_CUDA(cudaDeviceSynchronize());
-  return GSFFT_OK;
-}
-
-// FP32 plan whose first pass is a CUDA-core pass of radix 2^(L-6) and whose
-// last pass is a tensor-core radix-64 pass (one DFT_64 product per 128
-// sub-transforms, both sides read and written in 1 KiB runs): n = 2^L,
-// 13 <= L <= 20.
-int fft_plan_init_tc64(FftPlan &p, long long n, int max_batch) {
-  fft_plan_free(p);
-  if (n < 256 || (n & (n - 1)) != 0) return GSFFT_ERR_UNSUPPORTED;
-  int L = 0;
-  while ((1LL << L) < n) L++;
-  if (L < 13 || L > 20) return GSFFT_ERR_UNSUPPORTED;
-  p.n = n;
-  p.L = L;
-  p.precision = GSFFT_MIXED;
-  p.npass = 2;
-  p.logR[0] = L - 6;
-  p.logR[1] = 6;
-  p.tc[0] = false;
-  p.tc[1] = true;
-  long long Np = 1;
-  for (int i = 0; i < p.npass; i++) {
-    const long long R = 1LL << p.logR[i];
-    Np *= R;
-    int lg = 0;
-    while ((1LL << lg) < Np) lg++;
-    const int h = (lg + 1) / 2;
-    p.tw_h[i] = h;
-    const long long nlo = 1LL << h, nhi = (Np + nlo - 1) / nlo;
-    GS_CHECK(make_table<float>(&p.tw_lo[i], nlo, 1, Np));
-    GS_CHECK(make_table<float>(&p.tw_hi[i], nhi, nlo, Np));
-    GS_CHECK(make_table<float>(&p.tw_R[i], R, 1, R));
-  }
-  GS_CHECK(tc_build_F_smem(&p.tc_F));
-  p.scratch_elems = (long long)n * max_batch;
-  GS_CUDA(cudaMalloc(&p.scratch, sizeof(float2) * p.scratch_elems));
-  GS_CUDA(cudaDeviceSynchronize());
-  return GSFFT_OK;
+  GS_CHECK(fft_plan_shape(p, n, kind));
+  Arena mem;
+  fft_plan_request(p, max_batch, mem);
+  void *block = nullptr;
+  int s = mem.commit(&block, st);
+  p.mem = block;
+  if (s == GSFFT_OK) s = fft_plan_fill(p, st);
+  if (s != GSFFT_OK) fft_plan_free(p);
+  return s;
 }
 
 void fft_plan_free(FftPlan &p) {
-  for (int i = 0; i < 3; i++) {
-    if (p.tw_hi[i]) cudaFree(p.tw_hi[i]);
-    if (p.tw_lo[i]) cudaFree(p.tw_lo[i]);
-    if (p.tw_R[i]) cudaFree(p.tw_R[i]);
-    if (p.fx_tw[i]) cudaFree(p.fx_tw[i]);
-    if (p.fx_hi[i]) cudaFree(p.fx_hi[i]);
-    if (p.fx_lo[i]) cudaFree(p.fx_lo[i]);
-    p.tw_hi[i] = p.tw_lo[i] = p.tw_R[i] = nullptr;
-    p.fx_tw[i] = p.fx_hi[i] = p.fx_lo[i] = nullptr;
-  }
-  if (p.scratch) cudaFree(p.scratch);
-  p.scratch = nullptr;
-  if (p.tc_F) cudaFree(p.tc_F);
-  p.tc_F = nullptr;
-  for (int i = 0; i < 3; i++) p.tc[i] = false;
-  p.npass = 0;
+  if (p.mem) cudaFree(p.mem);
+  p = FftPlan();
 }
-
-int fft_launches(const FftPlan &p) { return p.npass; }
 
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
              const FftIo &io, cudaStream_t st) {

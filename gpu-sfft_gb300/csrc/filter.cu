@@ -193,15 +193,24 @@ int design_filter(const gsfft_params &p, double2 *d_ft, double2 *d_ff, cudaStrea
       s = GSFFT_ERR_CUDA;
     }
   };
-  ck(cudaMalloc(&win, sizeof(double2) * w));
-  ck(cudaMalloc(&a, sizeof(double2) * M));
-  ck(cudaMalloc(&b, sizeof(double2) * M));
-  ck(cudaMalloc(&g, sizeof(double2) * (size_t)n));
-  ck(cudaMalloc(&mx, sizeof(unsigned long long)));
-  if (!d_ff) ck(cudaMalloc(&ffb, sizeof(double2) * (size_t)n));
+  Arena mem;
+  void *block = nullptr;
+  mem.add(&win, sizeof(double2) * w);
+  mem.add(&a, sizeof(double2) * M);
+  mem.add(&b, sizeof(double2) * M);
+  mem.add(&g, sizeof(double2) * (size_t)n);
+  mem.add(&mx, sizeof(unsigned long long), true);
+  if (!d_ff) mem.add(&ffb, sizeof(double2) * (size_t)n);
+  s = fft_plan_shape(fm, M, FFT_FP64);
+  if (s == GSFFT_OK) s = fft_plan_shape(fn, n, FFT_FP64);
+  if (s == GSFFT_OK) {
+    fft_plan_request(fm, 1, mem);
+    fft_plan_request(fn, 1, mem);
+    s = mem.commit(&block, st);
+  }
   double2 *ff = d_ff ? d_ff : ffb;
-  if (s == GSFFT_OK) s = fft_plan_init(fm, M, GSFFT_FP64, 1);
-  if (s == GSFFT_OK) s = fft_plan_init(fn, n, GSFFT_FP64, 1);
+  if (s == GSFFT_OK) s = fft_plan_fill(fm, st);
+  if (s == GSFFT_OK) s = fft_plan_fill(fn, st);
   FftIo io;
   if (s == GSFFT_OK) {
     cheb_window_kernel<<<grid_of(w), FT, 0, st>>>(win, w, p.t0, p.tolerance);
@@ -224,7 +233,6 @@ int design_filter(const gsfft_params &p, double2 *d_ft, double2 *d_ff, cudaStrea
   }
   if (s == GSFFT_OK) s = fft_exec(fn, g, g, 1, -1, io, st);
   if (s == GSFFT_OK) {
-    ck(cudaMemsetAsync(mx, 0, sizeof(unsigned long long), st));
     boxcar_kernel<<<(unsigned)((n + BOX_TILE - 1) / BOX_TILE), FT, 0, st>>>(g, n, p.b_f, ff, mx);
     ck(cudaGetLastError());
     normalize_ramp_kernel<<<grid_of(n), FT, 0, st>>>(ff, n, w / 2, mx);
@@ -236,14 +244,7 @@ int design_filter(const gsfft_params &p, double2 *d_ft, double2 *d_ff, cudaStrea
     ck(cudaGetLastError());
     ck(cudaStreamSynchronize(st));
   }
-  fft_plan_free(fm);
-  fft_plan_free(fn);
-  cudaFree(win);
-  cudaFree(a);
-  cudaFree(b);
-  cudaFree(g);
-  cudaFree(mx);
-  if (ffb) cudaFree(ffb);
+  if (block) cudaFree(block);
   return s;
 }
 

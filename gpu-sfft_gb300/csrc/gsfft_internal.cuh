@@ -6,6 +6,8 @@
 #include <stdio.h>
 
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "gsfft.h"
 
@@ -109,6 +111,45 @@ extern thread_local int g_launch_counter;
     }                                                                         \
   } while (0)
 
+// ---------------------------------------------------------------- memory
+// Buffers of one object in one device allocation.  A cudaMalloc or cudaFree costs
+// about 10 us of host time, and a plan has some forty buffers: outer_loop, which
+// makes a plan per call, spent 0.8 of its 1.25 ms on them at n = 2^20.  add()
+// notes a buffer, commit() allocates the block and sets the pointers; the buffers
+// added with zero = true lie together and are cleared with one memset on st.
+class Arena {
+ public:
+  template <typename T>
+  void add(T **p, size_t bytes, bool zero = false) {
+    (zero ? zeroed_ : plain_).emplace_back(reinterpret_cast<void **>(p), bytes);
+  }
+  int commit(void **block, cudaStream_t st) {
+    size_t plain = 0, all = 0;
+    for (const auto &w : plain_) plain += round_up(w.second);
+    all = plain;
+    for (const auto &w : zeroed_) all += round_up(w.second);
+    *block = nullptr;
+    const cudaError_t e = cudaMalloc(block, all ? all : 16);
+    if (e != cudaSuccess) {
+      set_last_error("cudaMalloc(%zu): %s", all, cudaGetErrorString(e));
+      *block = nullptr;
+      return GSFFT_ERR_ALLOC;
+    }
+    char *b = static_cast<char *>(*block);
+    for (const auto &v : {plain_, zeroed_})
+      for (const auto &w : v) {
+        *w.first = b;
+        b += round_up(w.second);
+      }
+    if (all > plain) GS_CUDA(cudaMemsetAsync(static_cast<char *>(*block) + plain, 0, all - plain, st));
+    return GSFFT_OK;
+  }
+
+ private:
+  static size_t round_up(size_t v) { return (v + 511) / 512 * 512; }
+  std::vector<std::pair<void **, size_t>> plain_, zeroed_;
+};
+
 // ---------------------------------------------------------------- bounded waits
 // Every wait of a kernel on an mbarrier (a TMA copy's or a tensor-core
 // product's completion) gives up after `limit` SM clock cycles -- by default
@@ -210,6 +251,7 @@ struct FftPlan {
                                        // follows the pass: tc_build_F / tc_build_F_smem)
   void *scratch = nullptr; // one transform-sized buffer per batch entry (multi-pass)
   long long scratch_elems = 0;
+  void *mem = nullptr;     // the allocation of a plan of its own (fft_plan_init)
 };
 
 // One tensor-core pass of an FP32 FFT (tc_dft.cu): the radix-4096 first
@@ -231,9 +273,11 @@ struct TcPassArgs {
   int nsum = 1;         // radix-4096 form: add nsum partial inputs sstride apart
   long long sstride = 0;
 };
-int tc_build_F(void **F);
+size_t tc_F_bytes();
+int tc_build_F(void *F, cudaStream_t st);
 // radix 64 as the last pass (one DFT_64 product per 128 sub-transforms)
-int tc_build_F_smem(void **F);
+size_t tc_F_smem_bytes();
+int tc_build_F_smem(void *F, cudaStream_t st);
 int launch_tc64_last_pass(const TcPassArgs &a, cudaStream_t st);
 // radix 4096 = 64 x 64 in one pass (four-step, both DFT_64 stages on the tensor cores)
 int launch_tc4096_pass(const TcPassArgs &a, cudaStream_t st);
@@ -258,18 +302,24 @@ struct FftIo {
   int *err = nullptr;
 };
 
-// first_logr: log2 of the first pass's radix for two-pass sizes (0: ceil(L/2))
-int fft_plan_init(FftPlan &p, long long n, int precision, int max_batch, int first_logr = 0);
-// FP32 plan: radix-4096 tensor-core pass, then a CUDA-core pass of radix
-// n / 4096; GSFFT_ERR_UNSUPPORTED unless n = 2^(17..26)
-int fft_plan_init_tc(FftPlan &p, long long n, int max_batch);
-// FP32 plan: CUDA-core radix-2^(L-6) first pass, tensor-core radix-64 last pass (13 <= L <= 20)
-int fft_plan_init_tc64(FftPlan &p, long long n, int max_batch);
+// Kinds of plan: FP64 or FP32 on the integer / CUDA cores; FP32 with a radix-4096
+// tensor-core pass, then a CUDA-core pass of radix n / 4096 (n = 2^(17..26)); FP32
+// with a CUDA-core radix-2^(L-6) first pass, then a tensor-core radix-64 last pass
+// (13 <= L <= 20).  GSFFT_ERR_UNSUPPORTED for other sizes.
+enum FftKind { FFT_FP64, FFT_FP32, FFT_FP32_TC, FFT_FP32_TC64 };
+// A plan in three steps, so that its tables and scratch (max_batch transforms) can
+// share an allocation: its passes (first_logr: log2 of the first pass's radix for
+// two-pass sizes of the first two kinds, 0: ceil(L/2)), its buffers, the tables.
+int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr = 0);
+void fft_plan_request(FftPlan &p, int max_batch, Arena &mem);
+int fft_plan_fill(const FftPlan &p, cudaStream_t st);
+// The three steps with an allocation of its own; tables are built on st, the
+// stream that the plan is then used on (or synchronised with).
+int fft_plan_init(FftPlan &p, long long n, FftKind kind, int max_batch, cudaStream_t st);
 void fft_plan_free(FftPlan &p);
 // in: batch entries at in + b*n; out: out + b*n.  sign -1 forward, +1 inverse.
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
              const FftIo &io, cudaStream_t st);
-int fft_launches(const FftPlan &p);
 
 // ---------------------------------------------------------------- select
 // Top-`num` of each row by key (ties at the threshold: lowest index first),
@@ -286,15 +336,14 @@ struct SelectScratch {
   bool single_launch = true;   // cluster / cooperative form allowed (else multi-launch)
 };
 // Byte sizes of the SelectScratch regions for max_batch rows of at most
-// max_size samples (what select_scratch_init allocates); state and coop_hist
+// max_size samples (what select_scratch_request asks for); state and coop_hist
 // must hold zeros when a selection starts.
 struct SelectScratchBytes {
   size_t hist, state, tiles, coop_hist;
   int max_tiles;
 };
 SelectScratchBytes select_scratch_bytes(int max_batch, long long max_size);
-int select_scratch_init(SelectScratch &s, int max_batch, long long max_size);
-void select_scratch_free(SelectScratch &s);
+void select_scratch_request(SelectScratch &s, int max_batch, long long max_size, Arena &mem);
 // row_max (optional, per row, bit pattern of the largest sample) with
 // floor_rel > 0: samples below floor_rel * max are taken as exact zeros, so
 // rounding-level samples tie and resolve by ascending index.

@@ -919,29 +919,15 @@ SelectScratchBytes select_scratch_bytes(int max_batch, long long max_size) {
   return b;
 }
 
-int select_scratch_init(SelectScratch &s, int max_batch, long long max_size) {
-  select_scratch_free(s);
+void select_scratch_request(SelectScratch &s, int max_batch, long long max_size, Arena &mem) {
   const SelectScratchBytes b = select_scratch_bytes(max_batch, max_size);
   s.max_batch = max_batch;
   s.max_tiles = b.max_tiles;
-  GS_CUDA(cudaMalloc(&s.hist, b.hist));
-  GS_CUDA(cudaMalloc(&s.state, b.state));
-  GS_CUDA(cudaMalloc(&s.tiles, b.tiles));
-  GS_CUDA(cudaMemset(s.state, 0, b.state));
-  GS_CUDA(cudaMalloc(&s.coop_hist, b.coop_hist));
-  GS_CUDA(cudaMemset(s.coop_hist, 0, b.coop_hist));
-  return GSFFT_OK;
+  mem.add(&s.hist, b.hist);
+  mem.add(&s.state, b.state, true);
+  mem.add(&s.tiles, b.tiles);
+  mem.add(&s.coop_hist, b.coop_hist, true);
 }
-
-void select_scratch_free(SelectScratch &s) {
-  if (s.hist) cudaFree(s.hist);
-  if (s.state) cudaFree(s.state);
-  if (s.tiles) cudaFree(s.tiles);
-  if (s.coop_hist) cudaFree(s.coop_hist);
-  s.hist = s.state = s.tiles = s.coop_hist = nullptr;
-}
-
-size_t select_state_bytes() { return sizeof(SelState); }
 
 int select_top(const void *keys, int key_bytes, long long size, const int *size_dev, int num,
                int batch, long long row_stride, int *out, long long out_stride, int *count_out,

@@ -892,16 +892,16 @@ int launch_bounded_wait_probe(long long limit, int *gave_up, cudaStream_t st) {
   return GSFFT_OK;
 }
 
-int tc_build_F(void **F) {
-  GS_CUDA(cudaMalloc(F, 3 * FT_PART_BYTES));
-  tc_build_F_kernel<<<(TC_M * (TC_K / 2) + 255) / 256, 256>>>(static_cast<unsigned char *>(*F));
+size_t tc_F_bytes() { return 3 * FT_PART_BYTES; }
+int tc_build_F(void *F, cudaStream_t st) {
+  tc_build_F_kernel<<<(TC_M * (TC_K / 2) + 255) / 256, 256, 0, st>>>(static_cast<unsigned char *>(F));
   GS_LAUNCHED();
   return GSFFT_OK;
 }
 
-int tc_build_F_smem(void **F) {
-  GS_CUDA(cudaMalloc(F, 3 * A_BYTES));
-  tc_build_F_smem_kernel<<<(TC_M * TC_K + 255) / 256, 256>>>(static_cast<unsigned char *>(*F));
+size_t tc_F_smem_bytes() { return 3 * A_BYTES; }
+int tc_build_F_smem(void *F, cudaStream_t st) {
+  tc_build_F_smem_kernel<<<(TC_M * TC_K + 255) / 256, 256, 0, st>>>(static_cast<unsigned char *>(F));
   GS_LAUNCHED();
   return GSFFT_OK;
 }
