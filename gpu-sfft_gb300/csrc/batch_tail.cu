@@ -47,13 +47,13 @@ struct TailPlan {
   int Bt, n, nb, W, loops_loc, loops_thresh;
   const unsigned *epoch;
   unsigned *vote;
-  int *cnt, *blk, *cand;
+  int *cnt, *csum, *stash, *cand;
   int cap;
   RunCtl *ctl;
   const Draws *draws;
-  int vote_blocks;         // blocks of each stage (B_thresh / 8 buckets, one a warp)
+  int walk_blocks;         // blocks of a mark or count stage
+  int write_lanes, write_blocks;  // lanes per bucket and blocks of a write stage
   int packed;              // vote table of 2-bit counters
-  int per_item;            // consecutive blocks of a stage per work item
 };
 
 struct TailRange {  // items [first, first + count) cover the blocks of stage `stage` of `plan`
@@ -67,8 +67,8 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
 }
 
 // stage s of a plan -> (kind, location loop)
-__device__ __forceinline__ void stage_of(const TailPlan &tp, int s, int *kind, int *loop) {
-  const int marks = min(max(tp.loops_thresh - 1, 0), tp.loops_loc);
+__host__ __device__ __forceinline__ void stage_of(const TailPlan &tp, int s, int *kind, int *loop) {
+  const int want = tp.loops_thresh > 1 ? tp.loops_thresh - 1 : 0, marks = want < tp.loops_loc ? want : tp.loops_loc;
   if (s < marks) {
     *kind = ST_MARK;
     *loop = s;
@@ -77,6 +77,11 @@ __device__ __forceinline__ void stage_of(const TailPlan &tp, int s, int *kind, i
   const int r = s - marks;
   *kind = (r & 1) ? ST_WRITE : ST_COUNT;
   *loop = marks + r / 2;
+}
+__host__ __device__ __forceinline__ int blocks_of(const TailPlan &tp, int s) {
+  int kind, loop;
+  stage_of(tp, s, &kind, &loop);
+  return kind == ST_WRITE ? tp.write_blocks : tp.walk_blocks;
 }
 
 // Eight CTAs per SM (32 registers): the walks are chains of dependent L2 and
@@ -99,7 +104,7 @@ batch_tail_kernel(const TailPlan *__restrict__ plans, const TailRange *__restric
       if (r.stage > 0) {
         // every block of the plan's previous stage
         const int *dp = done + r.plan * MAX_STAGES + r.stage - 1;
-        const int want = plans[r.plan].vote_blocks;
+        const int want = blocks_of(plans[r.plan], r.stage - 1);
         const long long t0 = clock64();
         while (ld_acquire(dp) < want) {
           if (clock64() - t0 > kTailWaitLimit) {
@@ -127,20 +132,18 @@ batch_tail_kernel(const TailPlan *__restrict__ plans, const TailRange *__restric
     w.a = (unsigned)tp.draws->a[l];
     w.packed = tp.packed;
     const unsigned epoch = *tp.epoch;
-    const int nblk = tp.vote_blocks;
-    int *blk_pre = tp.blk + nblk + 1;
-    int *stash = tp.blk + 2 * (nblk + 1);
-    const int b0 = (item - r.first) * tp.per_item;
-    const int b1 = min(b0 + tp.per_item, nblk);
+    const int nblk = blocks_of(tp, r.stage);
+    const int b0 = (item - r.first) * kBlocksPerItem;
+    const int b1 = min(b0 + kBlocksPerItem, nblk);
     for (int b = b0; b < b1; b++) {
       if (kind == ST_MARK)
         vote_mark_block(w, epoch, tp.vote, b);
       else if (kind == ST_COUNT)
-        vote_count_block(w, epoch, (unsigned)tp.loops_thresh, tp.vote, tp.cnt, tp.blk, blk_pre,
-                         stash, tp.ctl, b, nblk);
+        vote_count_block(w, epoch, (unsigned)tp.loops_thresh, tp.vote, tp.cnt, tp.csum,
+                         tp.stash, b);
       else
-        vote_write_block(w, epoch, (unsigned)tp.loops_thresh, tp.vote, tp.cnt, blk_pre, stash,
-                         tp.cand, tp.cap, tp.ctl, b, nblk);
+        vote_write_block(w, l, tp.write_lanes, epoch, (unsigned)tp.loops_thresh, tp.vote, tp.cnt, tp.csum,
+                         tp.stash, tp.cand, tp.cap, tp.ctl, b, nblk);
       __syncthreads();  // the block bodies reuse their shared memory
     }
     // every thread's writes of this item reach gpu scope before it is counted
@@ -196,14 +199,16 @@ int batch_tail_create(Plan *const *plans, int count, BatchTail **out) {
     t.epoch = P->d_epoch;
     t.vote = P->vote;
     t.cnt = P->cnt;
-    t.blk = P->blk;
+    t.csum = P->csum;
+    t.stash = P->stash;
     t.cand = P->cand;
     t.cap = P->cap;
     t.ctl = P->ctl;
     t.draws = P->d_draws;
-    t.vote_blocks = (p.B_thresh + WPB - 1) / WPB;
+    t.walk_blocks = walk_blocks(p.B_thresh, t.nb);
+    t.write_lanes = write_lanes(p.B_thresh, t.nb, p.RLFC_loops * p.B_thresh, p.W_RLFC);
+    t.write_blocks = write_blocks(p.B_thresh, t.write_lanes);
     t.packed = P->packed_vote ? 1 : 0;
-    t.per_item = kBlocksPerItem;
     max_stages = std::max(max_stages, stages_of(p));
   }
   // items, stage-major over the plans
@@ -214,7 +219,7 @@ int batch_tail_create(Plan *const *plans, int count, BatchTail **out) {
       if (s >= stages_of(plans[i]->p)) continue;
       TailRange r;
       r.first = (int)total;
-      r.count = (tps[i].vote_blocks + tps[i].per_item - 1) / tps[i].per_item;
+      r.count = (blocks_of(tps[i], s) + kBlocksPerItem - 1) / kBlocksPerItem;
       r.plan = i;
       r.stage = s;
       ranges.push_back(r);

@@ -614,12 +614,13 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
   cudaStream_t st = S(stream);
   const int words = W_RLFC / 32;
   unsigned *bm = nullptr, *d_ep = nullptr;
-  int *cnt = nullptr, *blk = nullptr;
+  int *cnt = nullptr, *csum = nullptr, *stash = nullptr;
   RunCtl *ctl = nullptr;
   int s = GSFFT_OK;
   if (cudaMalloc(&bm, sizeof(unsigned) * words) != cudaSuccess ||
       cudaMalloc(&cnt, sizeof(int) * B_thresh) != cudaSuccess ||
-      cudaMalloc(&blk, sizeof(int) * vote_block_ints(B_thresh)) != cudaSuccess ||
+      cudaMalloc(&csum, sizeof(int) * vote_csum_ints(B_thresh, n / B)) != cudaSuccess ||
+      cudaMalloc(&stash, sizeof(int) * vote_stash_ints(B_thresh)) != cudaSuccess ||
       cudaMalloc(&ctl, sizeof(RunCtl)) != cudaSuccess ||
       cudaMalloc(&d_ep, sizeof(unsigned)) != cudaSuccess)
     s = GSFFT_ERR_ALLOC;
@@ -629,7 +630,7 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
   d.ai[0] = ai;
   RunCtl c;
   memset(&c, 0, sizeof(c));
-  c.cand_count = *h_count;
+  c.cand_count = c.base[0] = *h_count;
   c.num_rlfc = num_RLFC;
   if (s == GSFFT_OK && (cudaMemcpyAsync(ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st) != cudaSuccess ||
                         cudaMemcpyAsync(d_ep, &epoch, sizeof(unsigned), cudaMemcpyHostToDevice, st) !=
@@ -637,8 +638,8 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
     s = GSFFT_ERR_CUDA;
   if (s == GSFFT_OK) s = launch_sigma_bitmaps(d_J2, ctl, num_RLFC, W_RLFC, 1, d, bm, ctl, st);
   if (s == GSFFT_OK)
-    s = launch_vote_loop(0, d_J, B_thresh, n, B, W_RLFC, bm, d, loops_thresh, d_ep, d_vote, d_cand,
-                         cap, cnt, blk, ctl, true, st);
+    s = launch_vote_loop(0, d_J, B_thresh, n, B, W_RLFC, num_RLFC, bm, d, loops_thresh, d_ep, d_vote, d_cand,
+                         cap, cnt, csum, stash, ctl, true, st);
   if (s == GSFFT_OK && cudaMemcpyAsync(&c, ctl, sizeof(c), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     s = GSFFT_ERR_CUDA;
   if (s == GSFFT_OK) s = sync_check(st, "gsfft_stage_reverse_hash");
@@ -648,7 +649,8 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
   }
   cudaFree(bm);
   cudaFree(cnt);
-  cudaFree(blk);
+  cudaFree(csum);
+  cudaFree(stash);
   cudaFree(ctl);
   cudaFree(d_ep);
   return s;

@@ -133,7 +133,8 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   A0(vote, sizeof(unsigned) * (size_t)p.n);
   A(cand, sizeof(int) * (size_t)P->cap);
   A(cnt, sizeof(int) * (size_t)p.B_thresh);
-  A(blk, sizeof(int) * (size_t)vote_block_ints(p.B_thresh));
+  A(csum, sizeof(int) * (size_t)vote_csum_ints(p.B_thresh, nb));
+  A(stash, sizeof(int) * (size_t)vote_stash_ints(p.B_thresh));
   A(nodes, sizeof(DevNode) * (size_t)P->cap);
   A(mag2, sizeof(double) * (size_t)P->cap);
   A(topk_idx, sizeof(int) * (size_t)p.k + 16);
@@ -491,9 +492,9 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   BEGIN(ST_VOTE);
   const size_t wW = (size_t)p.W_RLFC / 32;
   for (int l = 0; l < p.loops_loc; l++)
-    GS_CHECK(launch_vote_loop(l, P->J + (size_t)l * p.B_thresh, p.B_thresh, p.n, p.B, p.W_RLFC,
+    GS_CHECK(launch_vote_loop(l, P->J + (size_t)l * p.B_thresh, p.B_thresh, p.n, p.B, p.W_RLFC, p.RLFC_loops * p.B_thresh,
                               P->bm_sig + wW * l, d, p.loops_thresh, P->d_epoch, P->vote, P->cand,
-                              P->cap, P->cnt, P->blk, P->ctl, l + 1 >= p.loops_thresh, st,
+                              P->cap, P->cnt, P->csum, P->stash, P->ctl, l + 1 >= p.loops_thresh, st,
                               P->packed_vote));
   END(ST_VOTE);
   }  // voting

@@ -34,7 +34,7 @@ struct Plan {
   unsigned *bm_j2 = nullptr, *bm_sig = nullptr, *tile_tmp = nullptr;
   unsigned *vote = nullptr;  // n epoch-tagged entries, or n/16 words of 2-bit counters
   bool packed_vote = false;  // 2-bit counters (at most 3 location loops)
-  int *cand = nullptr, *cnt = nullptr, *blk = nullptr;
+  int *cand = nullptr, *cnt = nullptr, *csum = nullptr, *stash = nullptr;
   DevNode *nodes = nullptr;
   double *mag2 = nullptr;
   int *topk_idx = nullptr;

@@ -21,10 +21,9 @@ struct RunCtl {
   int num_rlfc;        // |J2|
   int n_topk;
   int fmax[MAX_LOOPS]; // largest permuted residue per location loop
-  unsigned ticket;
+  int base[MAX_LOOPS + 1];  // first candidate of each location loop
   int err;  // a bounded device-side wait gave up (streaming perm+filter,
             // tensor-core FFT passes, persistent batch voting)
-  int pad[2];
 };
 
 struct DevNode {  // == Node (utils.h:42-45)
@@ -82,12 +81,15 @@ int launch_sigma_from_blocks(const int *J2b, int total, int W, int loops_loc, co
 // epoch: device word with the run's epoch (vote entries are epoch << 8 | count).
 // may_complete = false (location loop l < loops_thresh - 1 of a run, where no
 // count can reach the threshold) only records the votes.
-int launch_vote_loop(int l, const int *J, int B_thresh, int n, int B, int W,
+// nres: residues in bitmap_l, at most.
+int launch_vote_loop(int l, const int *J, int B_thresh, int n, int B, int W, int nres,
                      const unsigned *bitmap_l, const Draws &d, int loops_thresh, const unsigned *epoch,
-                     unsigned *vote, int *cand, int cap, int *cnt, int *blk, RunCtl *ctl,
+                     unsigned *vote, int *cand, int cap, int *cnt, int *csum, int *stash, RunCtl *ctl,
                      bool may_complete, cudaStream_t st, bool packed = false);
-// ints needed by the blk scratch of launch_vote_loop
-int vote_block_ints(int B_thresh);
+// ints of the candidate slots and of the count sums (both 16-byte aligned) of
+// launch_vote_loop; nb = n / B
+int vote_stash_ints(int B_thresh);
+int vote_csum_ints(int B_thresh, int nb);
 
 // A8: estimates + |value|^2 keys for the candidates.
 // cap: candidate capacity; the grid is sized for `expect` candidates (a

@@ -25,10 +25,19 @@
 //    bijection), so the update is a plain read-modify-write without races.
 //  * Candidates (count reaching loops_thresh) are appended in canonical order
 //    (location loop, bucket index, window position) by a count pass and a
-//    write pass with per-block prefix sums.  The count pass records each
-//    bucket's first STASH candidates in window order, so the write pass
-//    copies them instead of walking the window and the vote table again
-//    (buckets with more candidates are walked again).
+//    write pass.  The count pass records each bucket's first STASH candidates in
+//    window order, so the write pass copies them instead of walking the window and
+//    the vote table again (buckets with more candidates are walked again).  A block
+//    of the write pass adds up the count pass's block sums before it: no scan pass, no
+//    atomics (adding the counts of 256 buckets into one word with atomics took the
+//    count pass from 17 to 41 us).
+//
+// What bounds it: the latency of the table's atomics, whose results the count pass
+// waits for.  A lane takes 32 offsets of the window at any alignment, so a window
+// of 1024 positions costs one such latency (a lane per offset paid one for each of
+// its 32 steps).  n = 2^27, k = 16000: count 31 -> 18 us, write (a thread per
+// bucket instead of a warp) 15 -> 7; k = 43000 (windows of 512, two buckets a warp):
+// count 71 -> 23, write 30 -> 8.
 #include "vote_dev.cuh"
 
 namespace gsfft {
@@ -126,11 +135,10 @@ __global__ void sigma_from_blocks_kernel(const int *__restrict__ J2b, int total,
 }
 
 __global__ void __launch_bounds__(VT)
-vote_count_kernel(WalkArgs w, const unsigned *epoch_p, unsigned thresh, unsigned *vote, int *cnt,
-                  int *blk, int *blk_pre, int *stash, RunCtl *ctl) {
+vote_count_kernel(WalkArgs w, const unsigned *epoch_p, unsigned thresh, unsigned *vote, int *cnt, int *csum,
+                  int *stash) {
   pdl_enter();
-  vote_count_block(w, *epoch_p, thresh, vote, cnt, blk, blk_pre, stash, ctl, (int)blockIdx.x,
-                   (int)gridDim.x);
+  vote_count_block(w, *epoch_p, thresh, vote, cnt, csum, stash, (int)blockIdx.x);
 }
 
 __global__ void __launch_bounds__(VT)
@@ -140,12 +148,11 @@ vote_mark_kernel(WalkArgs w, const unsigned *epoch_p, unsigned *vote) {
 }
 
 __global__ void __launch_bounds__(VT)
-vote_write_kernel(WalkArgs w, const unsigned *epoch_p, unsigned thresh, const unsigned *__restrict__ vote,
-                  const int *__restrict__ cnt, const int *__restrict__ blk_pre, int nblk,
-                  const int *__restrict__ stash, int *cand, int cap, RunCtl *ctl) {
+vote_write_kernel(WalkArgs w, int l, int lw, const unsigned *epoch_p, unsigned thresh, const unsigned *__restrict__ vote,
+                  const int *__restrict__ cnt, const int *__restrict__ csum, const int *__restrict__ stash, int *cand,
+                  int cap, RunCtl *ctl) {
   pdl_enter();
-  vote_write_block(w, *epoch_p, thresh, vote, cnt, blk_pre, stash, cand, cap, ctl, (int)blockIdx.x,
-                   nblk);
+  vote_write_block(w, l, lw, *epoch_p, thresh, vote, cnt, csum, stash, cand, cap, ctl, (int)blockIdx.x, (int)gridDim.x);
 }
 
 }  // namespace
@@ -186,9 +193,9 @@ int launch_sigma_from_blocks(const int *J2b, int total, int W, int loops_loc, co
   return GSFFT_OK;
 }
 
-int launch_vote_loop(int l, const int *J, int B_thresh, int n, int B, int W,
+int launch_vote_loop(int l, const int *J, int B_thresh, int n, int B, int W, int nres,
                      const unsigned *bitmap_l, const Draws &d, int loops_thresh, const unsigned *epoch,
-                     unsigned *vote, int *cand, int cap, int *cnt, int *blk, RunCtl *ctl,
+                     unsigned *vote, int *cand, int cap, int *cnt, int *csum, int *stash, RunCtl *ctl,
                      bool may_complete, cudaStream_t st, bool packed) {
   WalkArgs w;
   w.J = J;
@@ -200,28 +207,24 @@ int launch_vote_loop(int l, const int *J, int B_thresh, int n, int B, int W,
   w.fmax = &ctl->fmax[l];
   w.a = (unsigned)d.a[l];
   w.packed = packed ? 1 : 0;
-  const int grid = (B_thresh + WPB - 1) / WPB;
+  const int grid = walk_blocks(B_thresh, w.nb);
   if (!may_complete) {
     GS_CUDA(launch_pdl(vote_mark_kernel, dim3(grid), dim3(VT), 0, st, w, epoch, vote));
     GS_LAUNCHED();
     return GSFFT_OK;
   }
-  // blk: 2 * (grid + 1) ints of block counts and prefixes, then STASH
-  // candidate slots per heavy bucket
-  int *blk_pre = blk + grid + 1;
-  int *stash = blk + 2 * (grid + 1);
   GS_CUDA(launch_pdl(vote_count_kernel, dim3(grid), dim3(VT), 0, st, w, epoch, (unsigned)loops_thresh,
-                     vote, cnt, blk, blk_pre, stash, ctl));
+                     vote, cnt, csum, stash));
   GS_LAUNCHED();
-  GS_CUDA(launch_pdl(vote_write_kernel, dim3(grid), dim3(VT), 0, st, w, epoch, (unsigned)loops_thresh,
-                     (const unsigned *)vote, (const int *)cnt, (const int *)blk_pre, grid,
+  const int lw = write_lanes(B_thresh, w.nb, nres, W);
+  GS_CUDA(launch_pdl(vote_write_kernel, dim3(write_blocks(B_thresh, lw)), dim3(VT), 0, st, w, l, lw, epoch,
+                     (unsigned)loops_thresh, (const unsigned *)vote, (const int *)cnt, (const int *)csum,
                      (const int *)stash, cand, cap, ctl));
   GS_LAUNCHED();
   return GSFFT_OK;
 }
 
-int vote_block_ints(int B_thresh) {
-  return 2 * ((B_thresh + WPB - 1) / WPB + 1) + B_thresh * STASH;
-}
+int vote_stash_ints(int B_thresh) { return B_thresh * STASH; }
+int vote_csum_ints(int B_thresh, int nb) { return walk_blocks(B_thresh, nb); }
 
 }  // namespace gsfft

@@ -3,9 +3,8 @@
 // that the per-plan kernels (vote.cu) and the persistent kernel that runs the
 // tails of a whole batch (batch_tail.cu) run the same code.  Loads of data
 // that another block of the same launch may have written (the vote table, the
-// block counts and scans, the stashed candidates, the candidate count) bypass
-// L1 (ld.global.cg), so the persistent kernel sees what its earlier work items
-// wrote.
+// bucket counts, the stashed candidates, the loop's first candidate) bypass L1
+// (ld.global.cg), so the persistent kernel sees what its earlier work items wrote.
 #pragma once
 #include "stages.cuh"
 
@@ -114,285 +113,242 @@ __device__ __forceinline__ int window_low(int J, int n, int nb) {
   return (int)((c + n) & (long long)(n - 1));
 }
 
-// One warp per heavy bucket.  The window [low, low + n/B) is cut into chunks;
-// in chunk c lane L holds a 32-bit mask of visited positions (window offsets
-// 1024c + 32L .. +31 when the window is 32-aligned, else the single offset
-// 32c + L).  Chunks, lanes and bits in ascending order give the window in
-// ascending order.  chunk_fn(mask, pos_of_bit) is called once per chunk by
-// every lane (warp-uniform trip count).
-struct ChunkPos {
-  int r0, base, key, W, n, aligned;
-  // position of bit t of this lane's mask
-  __device__ __forceinline__ int operator()(int t) const {
-    const int rr = aligned ? r0 + t : r0;
-    const int blk = (rr >= key) ? base : ((base + W) & (n - 1));
-    return blk + rr;
-  }
-};
+// A group of lpb lanes walks a heavy bucket: lane s of the group holds the 32
+// offsets c0 + 32 s .. + 31 of its window [low, low + n/B) as one mask (two bitmap
+// words and a funnel shift, whatever the alignment), so a window of 1024 offsets is
+// one step and all its table accesses overlap; 32 / lpb buckets share a warp.
+// Lanes, then bits, in ascending order give the window in ascending order.
+__host__ __device__ __forceinline__ int lanes_per_bucket(int nb) {
+  int l = 1;
+  while (l < 32 && 32 * l < nb) l <<= 1;
+  return l;
+}
 
+// chunk_fn(mask, off) for every step, by every lane (the trip count is the same for
+// all groups); bit b of mask is the visited position low + off + b.
 template <class F>
-__device__ __forceinline__ void for_each_chunk(const WalkArgs &w, int J, F &&chunk_fn) {
-  const int lane = threadIdx.x & 31;
-  const int low = window_low(J, w.n, w.nb);
+__device__ __forceinline__ void for_each_chunk(const WalkArgs &w, int low, bool live, int sub, int lpb,
+                                               F &&chunk_fn) {
   const int key = low & (w.W - 1);
-  if (key > *w.fmax) return;  // reference clamp: nothing visited
-  const int base = low - key;
-  const int aligned = ((key & 31) == 0 && (w.nb & 31) == 0) ? 1 : 0;
-  const int span = aligned ? 1024 : 32;
-  for (int c0 = 0; c0 < w.nb; c0 += span) {
+  if (key > *w.fmax) live = false;  // reference clamp: nothing visited
+  for (int c0 = 0; c0 < w.nb; c0 += 32 * lpb) {
     unsigned mask = 0;
-    int r0 = 0;
-    if (aligned) {
-      const int off = c0 + lane * 32;
-      if (off < w.nb) {
-        r0 = key + off;
-        if (r0 >= w.W) r0 -= w.W;  // aligned words never straddle W
-        mask = __ldg(&w.bm[r0 >> 5]);
-      }
-    } else {
-      const int off = c0 + lane;
-      if (off < w.nb) {
-        int r = key + off;
-        if (r >= w.W) r -= w.W;
-        r0 = r;
-        mask = (__ldg(&w.bm[r >> 5]) >> (r & 31)) & 1u;
-      }
+    const int off = c0 + 32 * sub;
+    if (live && off < w.nb) {
+      int r = key + off;
+      if (r >= w.W) r -= w.W;
+      const int wi = r >> 5, wn = wi + 1 == (w.W >> 5) ? 0 : wi + 1;
+      mask = __funnelshift_r(__ldg(&w.bm[wi]), __ldg(&w.bm[wn]), r & 31);
+      if (w.nb - off < 32) mask &= (1u << (w.nb - off)) - 1u;
     }
-    ChunkPos pos{r0, base, key, w.W, w.n, aligned};
-    chunk_fn(mask, pos);
+    chunk_fn(mask, off);
   }
 }
 
-__device__ __forceinline__ unsigned warp_excl_scan(unsigned v, unsigned *total) {
-  const int lane = threadIdx.x & 31;
+// exclusive scan over groups of lpb lanes
+__device__ __forceinline__ unsigned group_excl_scan(unsigned v, int sub, int lpb, unsigned *total) {
   unsigned x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  for (int o = 1; o < lpb; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o, lpb);
+    if (sub >= o) x += y;
   }
-  *total = __shfl_sync(0xffffffffu, x, 31);
+  *total = __shfl_sync(0xffffffffu, x, lpb - 1, lpb);
   return x - v;
 }
 
-constexpr int WPB = VT / 32;  // buckets (warps) per block
 constexpr int STASH = 32;     // candidates recorded per heavy bucket by the count pass
 
-// Votes of heavy bucket t (one warp): returns this lane's number of visited
-// positions whose count reached the threshold, and records the bucket's
-// first STASH of them, in window order, at slot[] (global or shared memory).
-__device__ __forceinline__ unsigned count_walk(const WalkArgs &w, int t, unsigned epoch, unsigned thresh,
-                                               unsigned *vote, int *slot) {
+// buckets per block of the mark and count passes
+__host__ __device__ __forceinline__ int buckets_per_block(int nb) { return VT / lanes_per_bucket(nb); }
+__host__ __device__ __forceinline__ int walk_blocks(int Bt, int nb) {
+  return (Bt + buckets_per_block(nb) - 1) / buckets_per_block(nb);
+}
+// Lanes per bucket in the write pass.  One where buckets are many and have few
+// candidates (n = 2^27, k = 16000: 4000 blocks of warps 15 us, 125 of threads 7 us); a
+// warp where they are few, or where more than 24 visited positions a window (nres
+// residues of W) can bring more candidates than slots, which are walked again.
+__host__ __device__ __forceinline__ int write_lanes(int Bt, int nb, int nres, int W) {
+  return Bt <= 8192 || (long long)nb * nres > 24LL * W ? 32 : 1;
+}
+__host__ __device__ __forceinline__ int write_blocks(int Bt, int lw) { return (Bt + VT / lw - 1) / (VT / lw); }
+
+// Takes up to four visited positions of a lane's mask (low bits first).
+__device__ __forceinline__ int take_four(unsigned &mask, unsigned first, unsigned a, unsigned nmask,
+                                         unsigned (&loc)[4], unsigned (&bit)[4]) {
+  int nq = 0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (mask) {
+      bit[q] = (unsigned)__ffs(mask) - 1u;
+      mask &= mask - 1;
+      loc[q] = ((first + bit[q]) * a) & nmask;
+      nq = q + 1;
+    }
+  }
+  return nq;
+}
+
+// Votes of heavy bucket t (one group of lanes): returns the number of visited
+// positions whose count reached the threshold, and records the bucket's first STASH
+// of them, in window order, at slot[].
+__device__ __forceinline__ unsigned count_walk(const WalkArgs &w, int t, int sub, int lpb, unsigned epoch,
+                                               unsigned thresh, unsigned *vote, int *slot) {
   const unsigned nmask = (unsigned)w.n - 1u;
-  unsigned c = 0;
-  unsigned recorded = 0;  // this bucket's candidates so far (warp-uniform)
-  for_each_chunk(w, w.J[t], [&](unsigned mask, const ChunkPos &pos) {
-    // up to four visited positions at a time: their table reads are
-    // independent, so they overlap instead of paying one DRAM latency each
+  const bool live = t < w.Bt;
+  const int low = live ? window_low(w.J[t], w.n, w.nb) : 0;
+  unsigned recorded = 0;  // this bucket's candidates so far (the same in its group)
+  for_each_chunk(w, low, live, sub, lpb, [&](unsigned mask, int off) {
+    const unsigned first = (unsigned)low + (unsigned)off;
     unsigned app = 0;  // bits of this lane's mask whose count reached the threshold
     while (mask) {
-      unsigned loc[4];
-      int nq = 0;
-      const unsigned before = mask;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (mask) {
-          const int bq = __ffs(mask) - 1;
-          mask &= mask - 1;
-          loc[q] = ((unsigned)pos(bq) * w.a) & nmask;
-          nq = q + 1;
-        }
-      }
-      unsigned cv[4];
+      unsigned loc[4], bit[4], cv[4];
+      const int nq = take_four(mask, first, w.a, nmask, loc, bit);
       vote_update(w, epoch, vote, loc, nq, cv);
-      unsigned hitq = 0;  // bit q: position q of this round reached the threshold
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (q < nq) hitq |= (unsigned)(cv[q] == thresh) << q;
-      // the round's positions are the lowest set bits of `before`, in order
-      unsigned taken = before & ~mask;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const unsigned low = taken & (0u - taken);
-        taken ^= low;
-        if ((hitq >> q) & 1u) app |= low;
-      }
+        if (q < nq && cv[q] == thresh) app |= 1u << bit[q];
     }
-    c += (unsigned)__popc(app);
-    // window order: chunks, then lanes, then bits (as the write pass walks)
+    __syncwarp();
     if (__any_sync(0xffffffffu, app != 0u)) {
       unsigned ctot;
-      unsigned o = recorded + warp_excl_scan((unsigned)__popc(app), &ctot);
+      unsigned o = recorded + group_excl_scan((unsigned)__popc(app), sub, lpb, &ctot);
       while (app) {
         const int b = __ffs(app) - 1;
         app &= app - 1;
-        if (o < (unsigned)STASH) slot[o] = (int)(((unsigned)pos(b) * w.a) & nmask);
+        if (o < (unsigned)STASH) slot[o] = (int)(((first + (unsigned)b) * w.a) & nmask);
         o++;
       }
       recorded += ctot;
     }
   });
-  return c;
+  return recorded;
 }
 
-// Appends heavy bucket t's cw candidates (warp-uniform) at cand[next ..]:
-// copied from slot[] when the count walk recorded them all (GLOBAL_SLOT: the
-// slots were written by another launch or block, so the loads bypass L1),
-// else found again by walking the window and the vote table.
-template <bool GLOBAL_SLOT>
-__device__ __forceinline__ void write_bucket(const WalkArgs &w, int t, unsigned epoch, unsigned thresh,
-                                             const unsigned *vote, unsigned cw, const int *slot,
-                                             int *cand, int cap, long long next) {
-  const int lane = threadIdx.x & 31;
-  if (cw <= (unsigned)STASH) {
-    for (unsigned j = lane; j < cw; j += 32) {
-      const long long o = next + j;
-      if (o < cap) cand[o] = GLOBAL_SLOT ? __ldcg(&slot[j]) : slot[j];
-    }
-    return;
+// One block of the count pass: votes of the location loop, each bucket's candidate
+// count and first STASH candidates, and the sum of the block's counts (csum[bid]).
+__device__ __forceinline__ void vote_count_block(const WalkArgs &w, unsigned epoch, unsigned thresh,
+                                                 unsigned *vote, int *cnt, int *csum, int *stash, int bid) {
+  const int lpb = lanes_per_bucket(w.nb), sub = threadIdx.x & (lpb - 1);
+  const int t = bid * (VT / lpb) + (int)threadIdx.x / lpb;
+  const unsigned c = count_walk(w, t, sub, lpb, epoch, thresh, vote, stash + (size_t)t * STASH);
+  __shared__ int s_sum;
+  if (threadIdx.x == 0) s_sum = 0;
+  __syncthreads();
+  if (sub == 0 && t < w.Bt) {
+    cnt[t] = (int)c;
+    if (c) atomicAdd(&s_sum, (int)c);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) csum[bid] = s_sum;
+}
+
+// One block of a location loop before the (loops_thresh - 1)-th, which cannot bring
+// any count to the threshold: votes only.
+__device__ __forceinline__ void vote_mark_block(const WalkArgs &w, unsigned epoch, unsigned *vote,
+                                                int bid) {
+  const int lpb = lanes_per_bucket(w.nb), sub = threadIdx.x & (lpb - 1);
+  const int t = bid * (VT / lpb) + (int)threadIdx.x / lpb;
   const unsigned nmask = (unsigned)w.n - 1u;
-  for_each_chunk(w, w.J[t], [&](unsigned mask, const ChunkPos &pos) {
-    // appended positions of this lane, in bit order
+  const bool live = t < w.Bt;
+  const int low = live ? window_low(w.J[t], w.n, w.nb) : 0;
+  for_each_chunk(w, low, live, sub, lpb, [&](unsigned mask, int off) {
+    while (mask) {
+      unsigned loc[4], bit[4], cv[4];
+      const int nq = take_four(mask, (unsigned)low + (unsigned)off, w.a, nmask, loc, bit);
+      vote_update(w, epoch, vote, loc, nq, cv);
+    }
+  });
+}
+
+// Heavy bucket t with more candidates than slots (a whole warp): walks the window
+// and the vote table again and appends its candidates at cand[next ..].
+__device__ __forceinline__ void write_walk(const WalkArgs &w, int t, unsigned epoch, unsigned thresh,
+                                           const unsigned *vote, int *cand, int cap, long long next) {
+  const int lane = threadIdx.x & 31;
+  const unsigned nmask = (unsigned)w.n - 1u;
+  const int low = window_low(w.J[t], w.n, w.nb);
+  for_each_chunk(w, low, true, lane, 32, [&](unsigned mask, int off) {
+    const unsigned first = (unsigned)low + (unsigned)off;
     unsigned app = 0;
-    unsigned m = mask;
-    while (m) {
+    while (mask) {
       unsigned loc[4], bit[4];
-      int nq = 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (m) {
-          bit[q] = __ffs(m) - 1;
-          m &= m - 1;
-          loc[q] = ((unsigned)pos((int)bit[q]) * w.a) & nmask;
-          nq = q + 1;
-        }
-      }
+      const int nq = take_four(mask, first, w.a, nmask, loc, bit);
 #pragma unroll
       for (int q = 0; q < 4; q++)
         if (q < nq && vote_at_threshold(w, epoch, vote, loc[q], thresh)) app |= 1u << bit[q];
     }
+    __syncwarp();
     unsigned ctot;
-    long long o = next + warp_excl_scan((unsigned)__popc(app), &ctot);
+    long long o = next + group_excl_scan((unsigned)__popc(app), lane, 32, &ctot);
     while (app) {
       const int b = __ffs(app) - 1;
       app &= app - 1;
-      if (o < cap) cand[o] = (int)(((unsigned)pos(b) * w.a) & nmask);
+      if (o < cap) cand[o] = (int)(((first + (unsigned)b) * w.a) & nmask);
       o++;
     }
     next += ctot;
   });
 }
 
-// One block of the count pass (block bid of nblk): votes of the location
-// loop, each bucket's candidate count and first STASH candidates; the last
-// block to finish writes the exclusive scan of the block counts.
-__device__ __forceinline__ void vote_count_block(const WalkArgs &w, unsigned epoch, unsigned thresh,
-                                                 unsigned *vote, int *cnt, int *blk, int *blk_pre,
-                                                 int *stash, RunCtl *ctl, int bid, int nblk) {
+// One block of the write pass of location loop l, lw lanes per bucket (1 or 32):
+// appends the block's candidates at their canonical offsets, after those of the
+// earlier buckets (the count pass's block sums); the last block stores the next
+// loop's offset and the candidate count.
+__device__ __forceinline__ void vote_write_block(const WalkArgs &w, int l, int lw, unsigned epoch, unsigned thresh,
+                                                 const unsigned *vote, const int *cnt, const int *csum,
+                                                 const int *stash, int *cand, int cap, RunCtl *ctl, int bid,
+                                                 int nblk) {
   __shared__ unsigned ws[VT / 32];
-  __shared__ int is_last;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = bid * WPB + warp;
-  unsigned c = 0;
-  if (t < w.Bt) c = count_walk(w, t, epoch, thresh, vote, stash + (size_t)t * STASH);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if (lane == 0 && t < w.Bt) cnt[t] = (int)c;
-  const unsigned s = blk_sum(lane == 0 ? c : 0u, ws);
-  // last block: exclusive scan of the block counts.  Only the block count has
-  // to be visible to it, so only thread 0 fences (a fence in every thread
-  // would wait for that thread's vote-table writes to reach memory).
-  if (threadIdx.x == 0) {
-    blk[bid] = (int)s;
-    __threadfence();
-    const unsigned tk = atomicAdd(&ctl->ticket, 1u);
-    is_last = tk == (unsigned)nblk - 1u;
+  const int base = __ldcg(&ctl->base[l]);
+  const int t0 = bid * (VT / lw), t = t0 + (int)threadIdx.x / lw, lane = threadIdx.x & 31;
+  unsigned before = 0;
+  // whole blocks of the count pass, four sums a load, then the buckets left
+  const int bpb = buckets_per_block(w.nb), nsum = t0 / bpb, n4 = nsum / 4;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n4; i += VT) {
+    const int4 v = __ldcg(reinterpret_cast<const int4 *>(csum) + i);
+    before += (unsigned)(v.x + v.y + v.z + v.w);
   }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  // Each thread scans a contiguous run of block counts: all its L2 loads are
-  // independent, then one block scan (the serial tail used to pay an L2 round
-  // trip and three barriers per 256 counts).
-  const int per = (nblk + VT - 1) / VT;
-  const int i0 = min(nblk, (int)threadIdx.x * per), i1 = min(nblk, i0 + per);
-  unsigned sum = 0;
-  for (int i = i0; i < i1; i++) sum += (unsigned)__ldcg(&blk[i]);
+  for (int i = 4 * n4 + (int)threadIdx.x; i < nsum; i += VT) before += (unsigned)__ldcg(&csum[i]);
+  for (int i = nsum * bpb + (int)threadIdx.x; i < t0; i += VT) before += (unsigned)__ldcg(&cnt[i]);
+  unsigned c = t < w.Bt && (lw == 1 || lane == 0) ? (unsigned)__ldcg(&cnt[t]) : 0u;
+  before = blk_sum(before, ws);
   unsigned tot;
-  unsigned run = blk_excl_scan(sum, ws, &tot);
-  for (int i = i0; i < i1; i++) {
-    blk_pre[i] = (int)run;
-    run += (unsigned)__ldcg(&blk[i]);
-  }
-  if (threadIdx.x == 0) {
-    blk_pre[nblk] = (int)tot;
-    ctl->ticket = 0;
-  }
-}
-
-// Location loops before the (loops_thresh-1)-th cannot bring any count to
-// the threshold: they only record their votes.
-// One block of a location loop that cannot complete a count: votes only.
-__device__ __forceinline__ void vote_mark_block(const WalkArgs &w, unsigned epoch, unsigned *vote,
-                                                int bid) {
-  const int warp = threadIdx.x >> 5;
-  const int t = bid * WPB + warp;
-  if (t >= w.Bt) return;
-  const unsigned nmask = (unsigned)w.n - 1u;
-  for_each_chunk(w, w.J[t], [&](unsigned mask, const ChunkPos &pos) {
-    while (mask) {
-      unsigned loc[4], cv[4];
-      int nq = 0;
+  const unsigned pre = blk_excl_scan(c, ws, &tot);
+  long long next = (long long)base + before + pre;
+  if (lw == 1) {
+    if (c && c <= (unsigned)STASH) {
+      const int4 *slot = reinterpret_cast<const int4 *>(stash + (size_t)t * STASH);
+      for (unsigned j = 0; j < c; j += 4) {
+        const int4 v = __ldcg(slot + j / 4);
+        const int vs[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (mask) {
-          const int b = __ffs(mask) - 1;
-          mask &= mask - 1;
-          loc[q] = ((unsigned)pos(b) * w.a) & nmask;
-          nq = q + 1;
-        }
+        for (unsigned q = 0; q < 4; q++)
+          if (j + q < c && next + j + q < cap) cand[next + j + q] = vs[q];
       }
-      vote_update(w, epoch, vote, loc, nq, cv);
     }
-  });
-}
-
-// One block of the write pass: appends the block's candidates at their
-// canonical offsets; the last block to finish publishes the new count.
-__device__ __forceinline__ void vote_write_block(const WalkArgs &w, unsigned epoch, unsigned thresh,
-                                                 const unsigned *vote, const int *cnt,
-                                                 const int *blk_pre, const int *stash, int *cand,
-                                                 int cap, RunCtl *ctl, int bid, int nblk) {
-  __shared__ unsigned ws[VT / 32];
-  __shared__ int is_last;
-  const int base_prev = __ldcg(&ctl->cand_count);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = bid * WPB + warp;
-  const unsigned c = (t < w.Bt && lane == 0) ? (unsigned)__ldcg(&cnt[t]) : 0u;
-  unsigned tot;
-  const unsigned wpre = blk_excl_scan(c, ws, &tot);  // lane 0 of each warp carries its count
-  long long next = (long long)base_prev + __ldcg(&blk_pre[bid]) + __shfl_sync(0xffffffffu, wpre, 0);
-  const unsigned cw = __shfl_sync(0xffffffffu, c, 0);
-  if (cw) write_bucket<true>(w, t, epoch, thresh, vote, cw, stash + (size_t)t * STASH, cand, cap, next);
-  // the last block to finish publishes the new candidate count; every block
-  // read the old one before its thread 0 takes a ticket (barrier + fence)
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned tk = atomicAdd(&ctl->ticket, 1u);
-    is_last = tk == (unsigned)nblk - 1u;
+    unsigned big = __ballot_sync(0xffffffffu, c > (unsigned)STASH);
+    while (big) {
+      const int src = __ffs(big) - 1;
+      big &= big - 1;
+      write_walk(w, t - lane + src, epoch, thresh, vote, cand, cap, __shfl_sync(0xffffffffu, next, src));
+    }
+  } else {
+    c = __shfl_sync(0xffffffffu, c, 0);
+    next = __shfl_sync(0xffffffffu, next, 0);
+    if (c > (unsigned)STASH)
+      write_walk(w, t, epoch, thresh, vote, cand, cap, next);
+    else if ((unsigned)lane < c && next + lane < cap)
+      cand[next + lane] = __ldcg(&stash[(size_t)t * STASH + lane]);
   }
-  __syncthreads();
-  if (is_last && threadIdx.x == 0) {
-    __threadfence();
-    const long long nc = (long long)base_prev + __ldcg(&blk_pre[nblk]);
-    ctl->cand_count = (int)(nc > 0x7fffffffLL ? 0x7fffffffLL : nc);
+  if (bid == nblk - 1 && threadIdx.x == 0) {
+    const long long nc = (long long)base + before + tot;
+    const int count = (int)(nc > 0x7fffffffLL ? 0x7fffffffLL : nc);
+    ctl->base[l + 1] = count;
+    ctl->cand_count = count;
     if (nc > cap) ctl->overflow = 1;
-    ctl->ticket = 0;
   }
 }
-
 
 }  // namespace
 
