@@ -347,21 +347,42 @@ int select_impl(const void *keys, long long size, const int *size_dev, int num, 
 
 
 // ---------------------------------------------------------------------------
-// Single-launch form: the same selection in one cooperative kernel.  Row b
-// is split into `cpr` contiguous chunks, one per CTA.  Each radix pass builds
-// the CTA's chunk histogram in shared memory and adds it to the row's global
-// histogram once; after a grid-wide sync every CTA derives its row's digit
-// itself.  A pass ends the descent early when the threshold's bin is "pure":
-// it holds one sample, or it is the first pass's digit 0 while the rounding
-// floor maps every key of that digit to exact zero.  Keys are then compared
-// on the bits decided so far; in the second case the first pass has already
-// stored every chunk's (nonzero, zero) counts, which are the (#greater,
-// #equal) counts of threshold 0, so the counting pass is skipped too (a
-// noiseless spectrum: one histogram pass and the write pass).  Counting and
-// writing use per-thread runs of contiguous samples and one packed block scan
-// per sub-tile, so ids come out ascending.  Rows that start on 16-byte
-// boundaries (with a capacity of whole 16-byte words) are read with 16-byte
-// loads.  Histograms are left zeroed for the next call.
+// Single-launch form: the same selection in one kernel.  Row b is split into `cpr`
+// contiguous chunks, one per CTA.
+//
+// sel_lists, the usual way, reads the samples once:
+//   1. a sample of about 2^18 samples a row (whole groups of 128 or 64, spread over the
+//      chunk; short rows are taken whole) is counted by leading digits, and the
+//      lower edge L of the digit that holds about 1.1 num samples above it is
+//      chosen -- or the smallest non-zero sample when that few are non-zero;
+//   2. every warp lists its samples >= L, in order, in shared memory, and their
+//      next digits are counted;
+//   3. either every non-zero sample is listed and they are at most num: all are
+//      taken, and the first zeros fill the rest; or the digit with the num-th largest
+//      is known, its few samples are exchanged, and each CTA finds the num-th by
+//      rank (key, then index) and writes its own.
+// A guess that proves wrong (a list too small, fewer than num above L, many samples
+// in the last digit) costs time only: sel_passes then does the selection.
+//
+// sel_passes: each radix pass builds the CTA's chunk histogram in shared memory and
+// adds it to the row's global histogram once; after a grid-wide sync every CTA
+// derives its row's digit itself.  A pass ends the descent early when the
+// threshold's bin is "pure": it holds one sample, or it is the first pass's digit 0
+// while the rounding floor maps every key of that digit to exact zero.  Keys are
+// then compared on the bits decided so far; in the second case the first pass has
+// already stored every chunk's (nonzero, zero) counts, which are the (#greater,
+// #equal) counts of threshold 0, so the counting pass is skipped too.  Counting and
+// writing use per-thread runs of contiguous samples and one packed block scan per
+// sub-tile, so ids come out ascending.
+//
+// What bounds them: instructions and block barriers, not the reads.  sel_passes ran
+// 80 instructions a sample on a noiseless row (two reads, 38 us for two rows of 2^22
+// floats) and read a noisy row five times (72 us; two rows of 2^24: 194 us);
+// sel_lists takes 26, 33 and 54 us.  Short rows (a cluster, or one CTA) are a chain of
+// barriers in both: 23 -> 21 us for rows of 2^17, 12 -> 9 for one CTA.
+//
+// Rows that start on 16-byte boundaries (with a capacity of whole 16-byte words) are
+// read with 16-byte loads.  Histograms are left zeroed for the next call.
 //
 // Two launch forms of the same kernel, differing only in their barrier:
 //   - cooperative (CLU = false): one grid over all rows, `grid.sync()`; used
@@ -386,10 +407,7 @@ constexpr int CLUSTER_MAX = 16;  // CTAs per row in the cluster form (non-portab
 // Rows up to this many samples (and top-k rows with a device-side live size)
 // take the cluster form.
 constexpr long long CLUSTER_ROW_MAX = 1LL << 18;
-// CTAs per SM the register budget is set for: three for 32-bit keys (the
-// large scans need the memory parallelism; two measured slower), two for
-// 64-bit keys (no spills; the top-k rows are short).
-template <typename K> constexpr int coop_ctas_per_sm() { return sizeof(K) == 4 ? 3 : 2; }
+constexpr int COOP_CTAS_PER_SM = 2;  // that the register budget (64) is set for
 
 struct CoopArgs {
   const void *keys;
@@ -499,19 +517,440 @@ __device__ __forceinline__ void for_chunk_keys(const void *row, long long lo, lo
   }
 }
 
-template <typename K, bool CLU, bool VEC>
-__global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(CoopArgs a) {
-  // Launched without programmatic serialization (it follows its predecessor
-  // completely); the trigger lets the next kernel's launch overlap this one,
-  // whose blocks are all resident already.
-  pdl_enter();
-  // Every barrier below is reached by all threads of all CTAs that take part
-  // in it: the conditions around them are uniform over the grid (cooperative
-  // form) or over the row's cluster (cluster form).
-  auto sync_all = [&]() {
-    if constexpr (CLU) cg::this_cluster().sync();
-    else cg::this_grid().sync();
+// ---------------------------------------------------------------- lists
+// Every barrier below is reached by all threads of all CTAs that take part in it:
+// the conditions around them are uniform over the grid (cooperative form) or over
+// the row's cluster (cluster form).
+template <bool CLU> __device__ __forceinline__ void sync_all() {
+  if constexpr (CLU) cg::this_cluster().sync();
+  else cg::this_grid().sync();
+}
+
+// rounding floor of row r (0: none)
+template <typename K> __device__ __forceinline__ K row_floor(const CoopArgs &a, int r) {
+  if (!(a.row_max && a.floor_rel > 0.0)) return (K)0;
+  if (sizeof(K) == 8) {
+    const double m = __longlong_as_double((long long)reinterpret_cast<const unsigned long long *>(a.row_max)[r]);
+    return (K)(unsigned long long)__double_as_longlong(m * a.floor_rel);
+  }
+  const float m = __uint_as_float(reinterpret_cast<const unsigned *>(a.row_max)[r]);
+  return (K)__float_as_uint((float)((double)m * a.floor_rel));
+}
+
+constexpr int WARPS = CT / 32;
+constexpr int AMB_MAX = 768;   // samples of the deciding digit, at most
+constexpr int LIST_SLOTS = 5;  // row slots of HIST_BINS words that sel_lists uses and clears
+// dynamic shared memory: per-warp lists (16-bit offset in the warp's segment, key),
+// a histogram, the exchanged samples
+template <typename K> constexpr int list_cap() { return sizeof(K) == 4 ? 512 : 288; }
+template <typename K> struct ListSmem {
+  K key[WARPS][list_cap<K>()];
+  unsigned short off[WARPS][list_cap<K>()];
+  union {
+    unsigned hist[HIST_BINS];
+    struct {
+      K key[AMB_MAX];
+      int idx[AMB_MAX];
+    } amb;
   };
+};
+static_assert(sizeof(ListSmem<unsigned>) <= COOP_SMEM && sizeof(ListSmem<unsigned long long>) <= COOP_SMEM,
+              "lists fit beside each other in the radix passes' shared memory");
+
+// First digit: 2048 bins from the top.  Floats: 8 per octave.  Doubles: 4 per octave
+// below the row's maximum when it is known, else one.
+template <typename K> struct FirstDigit {
+  int shift;
+  unsigned base;
+  __device__ __forceinline__ FirstDigit(const CoopArgs &a, int row) {
+    if constexpr (sizeof(K) == 4) {
+      shift = 20;
+      base = 0;
+    } else {
+      shift = a.row_max ? 50 : 52;
+      base = 0;
+      if (a.row_max) {
+        const unsigned m = (unsigned)(reinterpret_cast<const unsigned long long *>(a.row_max)[row] >> 50);
+        base = m > (unsigned)HIST_BINS - 1u ? m - ((unsigned)HIST_BINS - 1u) : 0u;
+      }
+    }
+  }
+  __device__ __forceinline__ unsigned of(K k) const {
+    const unsigned t = (unsigned)(k >> shift);
+    return t <= base ? 0u : min(t - base, (unsigned)HIST_BINS - 1u);
+  }
+  __device__ __forceinline__ K edge(unsigned d) const { return d ? (K)(d + base) << shift : (K)0; }
+};
+// Next digit of a key >= L: 2048 bins in the octave above it (1024 in each of two
+// where the first digit is an octave wide), so few samples share the deciding one.
+template <typename K> __device__ __forceinline__ unsigned next_digit(K key, K L, int shift) {
+  const K t = (key - L) >> shift;
+  return t < (K)(HIST_BINS - 1) ? (unsigned)t : (unsigned)HIST_BINS - 1u;
+}
+
+// EPQ contiguous samples of this lane in a group of 32 EPQ, read as 0 past hi.
+template <typename K, bool VEC>
+__device__ __forceinline__ void load_group(const void *row, long long i, long long hi, K (&ks)[keys_per_quad<K>()]) {
+  constexpr int EPQ = keys_per_quad<K>();
+  if constexpr (VEC) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (i < hi) v = __ldg(reinterpret_cast<const uint4 *>(row) + i / EPQ);
+    unpack_quad<K>(v, ks);
+#pragma unroll
+    for (int e = 0; e < EPQ; e++)
+      if (i + e >= hi) ks[e] = (K)0;
+  } else {
+#pragma unroll
+    for (int e = 0; e < EPQ; e++) ks[e] = i + e < hi ? raw_key<K>(row, i + e) : (K)0;
+  }
+}
+
+// Returns false (uniformly) when sel_passes has to do the selection; sz > num.
+template <typename K, bool CLU, bool VEC>
+__device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long long sz, long long lo, long long hi) {
+  extern __shared__ unsigned wh[];
+  ListSmem<K> &sm = *reinterpret_cast<ListSmem<K> *>(wh);
+  __shared__ unsigned ws[WARPS], wcnt[WARPS];
+  __shared__ unsigned s_digit, s_need, s_amb;
+  __shared__ K s_key;
+  __shared__ int s_idx;
+  __shared__ int s_last;
+  constexpr int EPQ = keys_per_quad<K>(), GK = 32 * EPQ, CAP = list_cap<K>();
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const void *row = reinterpret_cast<const char *>(a.keys) + (size_t)b * a.row_stride * sizeof(K);
+  // a row in one CTA keeps all of it in shared memory
+  __shared__ unsigned s_ctl[3];
+  const bool solo = CLU && a.cpr == 1;
+  auto slot = [&](int p, int r) -> unsigned * { return a.hist + ((size_t)p * MAXB + r) * HIST_BINS; };
+  // slot 0: sampled first digits; 1: next digits; 2: [0] overflow, [1] listed, [2] all
+  // non-zero samples are listed, [3] exchanged, [4] ticket; 3, 4: exchanged keys, indices
+  const K floor = row_floor<K>(a, b), lowest = floor > (K)1 ? floor : (K)1;
+  const FirstDigit<K> dig(a, b);
+  const int shift2 = sizeof(K) == 4 ? 12 : (dig.shift == 50 ? 41 : 42);
+  const int ngroups = (int)((hi - lo + GK - 1) / GK), gpw = (ngroups + WARPS - 1) / WARPS;
+  const int g0 = min(wid * gpw, ngroups), g1 = min(g0 + gpw, ngroups);
+
+  // 1. the sample
+  const int step = sz >> 18 > 1 ? (int)(sz >> 18) : 1;
+  for (int i = tid; i < HIST_BINS; i += CT) sm.hist[i] = 0;
+  __syncthreads();
+  for (int j = wid; j * step < ngroups; j += WARPS) {
+    const int g = j * step + (step > 1 ? (int)((((unsigned)j * 0x9E3779B1u) >> 16) % (unsigned)step) : 0);
+    if (g < ngroups) {
+      K ks[EPQ];
+      load_group<K, VEC>(row, lo + (long long)g * GK + lane * EPQ, hi, ks);
+#pragma unroll
+      for (int e = 0; e < EPQ; e++)
+        if (ks[e] >= lowest) atomicAdd(&sm.hist[dig.of(ks[e])], 1u);
+    }
+  }
+  __syncthreads();
+  auto publish = [&](int p) {  // the histogram to its row's slot
+    if (solo) return;
+    unsigned *gh = slot(p, b);
+    for (int i = tid; i < HIST_BINS; i += CT)
+      if (sm.hist[i]) atomicAdd(&gh[i], sm.hist[i]);
+    sync_all<CLU>();
+  };
+  auto four_bins = [&](int p, int r) -> uint4 {  // this thread's bins of row r
+    if (solo) return reinterpret_cast<const uint4 *>(sm.hist)[tid];
+    return __ldcg(reinterpret_cast<const uint4 *>(slot(p, r)) + tid);
+  };
+  publish(0);
+  // the lower edge: the highest digit with at least `want` sampled samples from it up
+  K L = lowest;
+  {
+    const float mean = (float)a.num / (float)step;
+    const unsigned want = step > 1 ? (unsigned)(mean + 5.f * sqrtf(mean) + 8.f) : (unsigned)a.num;
+    const uint4 h = four_bins(0, b);
+    const unsigned hs[4] = {h.x, h.y, h.z, h.w};
+    unsigned tot;
+    unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);  // samples below the bin
+    if (tid == 0) s_digit = 0u;
+    __syncthreads();
+    if (tot >= want) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        // samples from this bin up: tot - from
+        if (tot - from >= want && tot - from - hs[q] < want) s_digit = (unsigned)(4 * tid + q);
+        from += hs[q];
+      }
+    }
+    __syncthreads();
+    const K e = dig.edge(s_digit);
+    if (e > L) L = e;
+  }
+  const bool all_listed = L == lowest;
+
+  // 2. the lists
+  for (int i = tid; i < HIST_BINS; i += CT) sm.hist[i] = 0;
+  unsigned wc = 0;  // of this warp
+  constexpr int GU = 4;  // groups in flight
+  const int gfull = (int)((hi - lo) / GK);  // groups without a bound check
+  const uint4 *vrow = reinterpret_cast<const uint4 *>(row) + lo / EPQ + lane;
+  for (int g = g0; g < g1; g += GU) {
+    K ks[GU][EPQ];
+    if (VEC && g + GU <= min(g1, gfull)) {
+      uint4 v[GU];
+#pragma unroll
+      for (int u = 0; u < GU; u++) v[u] = __ldg(vrow + (g + u) * 32);
+#pragma unroll
+      for (int u = 0; u < GU; u++) unpack_quad<K>(v[u], ks[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < GU; u++)
+        load_group<K, VEC>(row, g + u < g1 ? lo + (long long)(g + u) * GK + lane * EPQ : hi, hi, ks[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < GU; u++) {
+      K top = ks[u][0];
+#pragma unroll
+      for (int e = 1; e < EPQ; e++) top = ks[u][e] > top ? ks[u][e] : top;
+      const unsigned lanes = __ballot_sync(0xffffffffu, top >= L);
+      if (!lanes) continue;
+      unsigned m = 0;
+#pragma unroll
+      for (int e = 0; e < EPQ; e++) m |= (ks[u][e] >= L ? 1u : 0u) << e;
+      const int at = (g + u - g0) * GK + lane * EPQ;
+      if (!__any_sync(0xffffffffu, m & (m - 1u))) {  // at most one a lane
+        const unsigned pos = wc + __popc(lanes & ((1u << lane) - 1u));
+        if (m && pos < (unsigned)CAP) {
+          sm.key[wid][pos] = top;
+          sm.off[wid][pos] = (unsigned short)(at + __ffs(m) - 1);
+        }
+        wc += __popc(lanes);
+      } else {
+        unsigned pre = 0, tot = 0;
+#pragma unroll
+        for (int e = 0; e < EPQ; e++) {
+          const unsigned bl = __ballot_sync(0xffffffffu, (m >> e) & 1u);
+          pre += __popc(bl & ((1u << lane) - 1u));
+          tot += __popc(bl);
+        }
+        unsigned pos = wc + pre;
+#pragma unroll
+        for (int e = 0; e < EPQ; e++)
+          if ((m >> e) & 1u) {
+            if (pos < (unsigned)CAP) {
+              sm.key[wid][pos] = ks[u][e];
+              sm.off[wid][pos] = (unsigned short)(at + e);
+            }
+            pos++;
+          }
+        wc += tot;
+      }
+    }
+  }
+  if (lane == 0) wcnt[wid] = wc;
+  __syncthreads();  // lists and the cleared histogram
+  const int nl = (int)min(wc, (unsigned)CAP);
+  for (int j = lane; j < nl; j += 32) atomicAdd(&sm.hist[next_digit<K>(sm.key[wid][j], L, shift2)], 1u);
+  if (wid == 0) {
+    const unsigned v = lane < WARPS ? wcnt[lane] : 0u;
+    const unsigned c = __reduce_add_sync(0xffffffffu, v);
+    const bool over = __any_sync(0xffffffffu, v > (unsigned)CAP);
+    if (lane == 0) {
+      if (solo) {
+        s_ctl[0] = over;
+        s_ctl[1] = c;
+        s_ctl[2] = all_listed;
+      } else {
+        unsigned *ctl = slot(2, b);
+        if (over) atomicOr(&ctl[0], 1u);
+        if (c) atomicAdd(&ctl[1], c);
+        if (all_listed) atomicOr(&ctl[2], 1u);
+      }
+      a.tiles[((size_t)b * a.max_tiles + ci) * 2] = c;
+    }
+  }
+  __syncthreads();
+  publish(1);
+
+  // 3. what is known of every row behind the barrier (own row last, so its figures stay)
+  bool bad = false, any_rank = false, my_rank = false;
+  const int nrows = CLU ? 1 : a.batch;
+  unsigned digit = 0, need = 0, amb = 0;
+  for (int q = 1; q <= nrows; q++) {
+    const int r = CLU ? b : (b + q) % nrows;
+    const unsigned *ctl = slot(2, r);
+    const unsigned over = solo ? s_ctl[0] : __ldcg(&ctl[0]), listed = solo ? s_ctl[1] : __ldcg(&ctl[1]),
+                   all = solo ? s_ctl[2] : __ldcg(&ctl[2]);
+    my_rank = false;
+    if (over || (listed < (unsigned)a.num && !all)) {
+      bad = true;
+    } else if (listed > (unsigned)a.num || !all) {
+      my_rank = any_rank = true;
+      const uint4 h = four_bins(1, r);
+      const unsigned hs[4] = {h.x, h.y, h.z, h.w};
+      unsigned tot;
+      unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const unsigned up = tot - from;  // listed samples from this bin up
+        if (up >= (unsigned)a.num && up - hs[e] < (unsigned)a.num) {
+          s_digit = (unsigned)(4 * tid + e);
+          s_need = (unsigned)a.num - (up - hs[e]);
+          s_amb = hs[e];
+        }
+        from += hs[e];
+      }
+      __syncthreads();
+      digit = s_digit;
+      need = s_need;
+      amb = s_amb;
+      __syncthreads();
+      if (amb > (unsigned)AMB_MAX) bad = true;
+    }
+  }
+  auto clear_slots = [&](int r, int part, int parts) {
+    for (int i = part * CT + tid; i < LIST_SLOTS * HIST_BINS; i += parts * CT) slot(i / HIST_BINS, r)[i % HIST_BINS] = 0;
+  };
+  if (bad) {
+    if (solo) {
+      __syncthreads();
+      return false;
+    }
+    sync_all<CLU>();  // every CTA has read the row's figures
+    for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++) clear_slots(r, CLU ? ci : blockIdx.x, CLU ? a.cpr : gridDim.x);
+    sync_all<CLU>();
+    return false;
+  }
+
+  int *o = a.out + (size_t)b * a.out_stride;
+  const unsigned *tb = a.tiles + (size_t)b * a.max_tiles * 2;
+  const long long seg = lo + (long long)g0 * GK;  // this warp's first sample
+  if (my_rank) {
+    // exchange the deciding digit's samples
+    unsigned na = 0, nd = 0;
+    for (int j = lane; j < nl; j += 32) {
+      const unsigned d = next_digit<K>(sm.key[wid][j], L, shift2);
+      nd += d > digit;
+      na += d == digit;
+    }
+    const unsigned packed = na | (nd << 16);  // at most 16 x 512 listed samples a CTA
+    unsigned tot;
+    const unsigned pre = ct_excl_scan(packed, ws, &tot);
+    if (tid == 0) {
+      a.tiles[((size_t)b * a.max_tiles + ci) * 2 + 1] = tot >> 16;
+      s_need = !solo && (tot & 0xffffu) ? atomicAdd(&slot(2, b)[3], tot & 0xffffu) : 0u;
+    }
+    __syncthreads();
+    unsigned at = s_need + (pre & 0xffffu);
+    K *ek = solo ? sm.amb.key : reinterpret_cast<K *>(slot(3, b));
+    int *ei = solo ? sm.amb.idx : reinterpret_cast<int *>(slot(4, b));
+    for (int j = lane; j < nl; j += 32)
+      if (next_digit<K>(sm.key[wid][j], L, shift2) == digit) {
+        ek[at] = sm.key[wid][j];
+        ei[at] = (int)(seg + sm.off[wid][j]);
+        at++;
+      }
+  }
+  if (any_rank && !solo) sync_all<CLU>();
+  if (my_rank) {
+    // the num-th largest: rank `need` of the exchanged samples by key, then index
+    for (int e = tid; !solo && e < (int)amb; e += CT) {
+      sm.amb.key[e] = __ldcg(reinterpret_cast<const K *>(slot(3, b)) + e);
+      sm.amb.idx[e] = __ldcg(reinterpret_cast<const int *>(slot(4, b)) + e);
+    }
+    __syncthreads();
+    for (int e = tid; e < (int)amb; e += CT) {
+      const K k = sm.amb.key[e];
+      const int ix = sm.amb.idx[e];
+      unsigned rank = 0;
+      for (int f = 0; f < (int)amb; f++)
+        rank += sm.amb.key[f] > k || (sm.amb.key[f] == k && sm.amb.idx[f] < ix);
+      if (rank == need - 1u) {
+        s_key = k;
+        s_idx = ix;
+      }
+    }
+    __syncthreads();
+    const K kt = s_key;
+    const int it = s_idx;
+    // samples taken in earlier chunks: the surely larger ones, and exchanged ones
+    unsigned before = 0;
+    for (int c = tid; c < ci; c += CT) before += __ldcg(&tb[c * 2 + 1]);
+    for (int e = tid; e < (int)amb; e += CT)
+      before += sm.amb.idx[e] < lo && (sm.amb.key[e] > kt || (sm.amb.key[e] == kt && sm.amb.idx[e] <= it));
+    unsigned first;
+    ct_excl_scan(before, ws, &first);
+    unsigned mine = 0;
+    for (int j = lane; j < nl; j += 32) {
+      const K k = sm.key[wid][j];
+      mine += k > kt || (k == kt && (int)(seg + sm.off[wid][j]) <= it);
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) wcnt[wid] = mine;
+    __syncthreads();
+    unsigned pos = first;
+    for (int i = 0; i < wid; i++) pos += wcnt[i];
+    for (int j0 = 0; j0 < nl; j0 += 32) {
+      const int j = j0 + lane;
+      bool take = false;
+      int ix = 0;
+      if (j < nl) {
+        const K k = sm.key[wid][j];
+        ix = (int)(seg + sm.off[wid][j]);
+        take = k > kt || (k == kt && ix <= it);
+      }
+      const unsigned bl = __ballot_sync(0xffffffffu, take);
+      if (take) o[pos + __popc(bl & ((1u << lane) - 1u))] = ix;
+      pos += __popc(bl);
+    }
+  } else {
+    // every listed sample is taken, and the first z zeros
+    unsigned before = 0, all = 0;
+    for (int c = tid; c < a.cpr; c += CT) {
+      const unsigned v = __ldcg(&tb[c * 2]);
+      if (c < ci) before += v;
+      all += v;
+    }
+    unsigned R, T, cnt = 0;
+    ct_excl_scan(before, ws, &R);  // listed samples before the chunk
+    ct_excl_scan(all, ws, &T);
+    for (int i = 0; i < WARPS; i++) cnt += wcnt[i];
+    const long long z = (long long)a.num - T, zb = lo - (long long)R, zin = (hi - lo) - (long long)cnt;
+    if (zb + zin <= z) {  // every sample up to here is taken
+      for (long long i = lo + tid; i < hi; i += CT) o[i] = (int)i;
+    } else {
+      unsigned j0 = 0;  // list position of this warp
+      for (int i = 0; i < wid; i++) j0 += wcnt[i];
+      if (zb >= z) {
+        for (int j = lane; j < nl; j += 32) o[z + R + j0 + j] = (int)(seg + sm.off[wid][j]);
+      } else {
+        // the last zero taken is this chunk's (z - zb)-th: list entries with fewer
+        // zeros before them lie ahead of it
+        const long long zl = z - zb;
+        unsigned ahead = 0;
+        for (int j = lane; j < nl; j += 32)
+          ahead += seg + sm.off[wid][j] - lo - (long long)(j0 + j) < zl;
+        unsigned na;
+        ct_excl_scan(ahead, ws, &na);
+        const long long last = lo + zl - 1 + na;
+        for (long long i = lo + tid; i <= last; i += CT) o[i] = (int)i;
+        for (int j = lane; j < nl; j += 32)
+          if (j0 + j >= na) o[z + R + j0 + j] = (int)(seg + sm.off[wid][j]);
+      }
+    }
+  }
+  // the last CTA to get here leaves the slots zero for the next call
+  if (solo) return true;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&slot(2, CLU ? b : 0)[4], 1u) == (CLU ? (unsigned)a.cpr : gridDim.x) - 1u;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++) clear_slots(r, 0, 1);
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------- radix passes
+template <typename K, bool CLU, bool VEC>
+__device__ __noinline__ void sel_passes(const CoopArgs &a, int b, int ci, long long sz, long long lo, long long hi) {
   // one private histogram per warp, two 16-bit counters per word, so warps
   // never contend on a bin (a warp counts at most chunk / 16 < 65536 keys)
   extern __shared__ unsigned wh[];  // [CT / 32][HIST_BINS / 2]
@@ -526,43 +965,21 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
   const int w32[3] = {11, 11, 10};
   constexpr int npass = kb == 64 ? 6 : 3;
   constexpr int shift0 = kb - 11;  // shift of the first pass's digit
-  const int b = blockIdx.x / a.cpr, ci = blockIdx.x % a.cpr;
-  // row state (identical in every CTA of the row)
-  long long sz = a.size;
-  if (a.size_dev) {
-    const long long dv = *a.size_dev;
-    sz = dv < a.size ? dv : a.size;
-    if (sz < 0) sz = 0;
-  }
-  // rounding floor of row r (0: none)
-  auto row_floor = [&](int r) -> K {
-    if (!(a.row_max && a.floor_rel > 0.0)) return (K)0;
-    if (kb == 64) {
-      const double m = __longlong_as_double((long long)reinterpret_cast<const unsigned long long *>(a.row_max)[r]);
-      return (K)(unsigned long long)__double_as_longlong(m * a.floor_rel);
-    }
-    const float m = __uint_as_float(reinterpret_cast<const unsigned *>(a.row_max)[r]);
-    return (K)__float_as_uint((float)((double)m * a.floor_rel));
-  };
   // With a floor of at least 2^shift0, every key is either 0 or at least the
   // floor, so digit 0 of the first pass holds exactly the row's zeros.
-  auto zero_digit = [&](int r) -> bool { return (unsigned long long)row_floor(r) >= (1ull << shift0); };
-  const K floor = row_floor(b);
+  auto zero_digit = [&](int r) -> bool { return (unsigned long long)row_floor<K>(a, r) >= (1ull << shift0); };
+  const K floor = row_floor<K>(a, b);
   const bool zdig = zero_digit(b);
-  const bool take_all = sz <= a.num;
-  const long long chunk = ((sz + a.cpr - 1) / a.cpr + 31) & ~31LL;
-  const long long lo = (long long)ci * chunk < sz ? (long long)ci * chunk : sz;
-  const long long hi = lo + chunk < sz ? lo + chunk : sz;
   const void *row = reinterpret_cast<const char *>(a.keys) + (size_t)b * a.row_stride * sizeof(K);
   const long long rank0 = sz - a.num - 1;  // the same for every row (rows share one size)
   unsigned long long prefix = 0;
   long long rank = rank0;
   int cmp_shift = 0;  // low bits ignored by the final comparisons
-  bool done = take_all;
+  bool done = false;
   bool counted = false;  // the chunk counts for the final threshold are already stored
   // every row settled (the cluster form: this row settled): uniform over the
   // CTAs sharing the barrier, so every one of them skips the same barriers
-  bool all_done = take_all;
+  bool all_done = false;
   int shift = kb;
   for (int p = 0; p < npass && !all_done; p++) {
     const int width = kb == 64 ? w64[p] : w32[p];
@@ -610,7 +1027,7 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
       }
       __syncthreads();  // the per-warp histograms are rebuilt next pass
     }
-    sync_all();
+    sync_all<CLU>();
     if (!done) {
       // the digit holding ascending rank `rank` of this row
       const unsigned *gh = a.hist + ((size_t)p * MAXB + b) * HIST_BINS;
@@ -667,7 +1084,7 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
   const K thr = (K)prefix;
   const unsigned long long thr_c = (unsigned long long)thr >> cmp_shift;
   unsigned gt = 0, eq = 0;
-  if (!take_all && !counted)
+  if (!counted)
     for_chunk_keys<K, VEC>(row, lo, hi, floor, [&](long long, K key) {
       const unsigned long long kc = (unsigned long long)key >> cmp_shift;
       gt += kc > thr_c;
@@ -680,7 +1097,7 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
     a.tiles[((size_t)b * a.max_tiles + ci) * 2 + 0] = tgt;
     a.tiles[((size_t)b * a.max_tiles + ci) * 2 + 1] = teq;
   }
-  sync_all();
+  sync_all<CLU>();
   // the histograms were read by every CTA before the barrier above: zero
   // them for the next call (the cluster form: its own row's)
   if constexpr (CLU) {
@@ -693,9 +1110,7 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
   }
   // writing pass
   int *o = a.out + (size_t)b * a.out_stride;
-  if (take_all) {
-    for (long long i = lo + tid; i < hi; i += CT) o[i] = (int)i;
-  } else {
+  {
     // chunk prefix and row totals
     unsigned bg = 0, be = 0, tg = 0;
     const unsigned *tb = a.tiles + (size_t)b * a.max_tiles * 2;
@@ -774,7 +1189,34 @@ __global__ void __launch_bounds__(CT, coop_ctas_per_sm<K>()) sel_coop_kernel(Coo
       eq_run += tot >> 16;
     }
   }
-  if (a.count_out && ci == 0 && tid == 0) a.count_out[b] = take_all ? (int)sz : a.num;
+}
+
+template <typename K, bool CLU, bool VEC>
+__global__ void __launch_bounds__(CT, COOP_CTAS_PER_SM)
+sel_coop_kernel(const __grid_constant__ CoopArgs a) {
+  // Launched without programmatic serialization (it follows its predecessor
+  // completely); the trigger lets the next kernel's launch overlap this one,
+  // whose blocks are all resident already.
+  pdl_enter();
+  const int b = blockIdx.x / a.cpr, ci = blockIdx.x % a.cpr;
+  // live size (the same for every row: rows share one size)
+  long long sz = a.size;
+  if (a.size_dev) {
+    const long long dv = *a.size_dev;
+    sz = dv < a.size ? dv : a.size;
+    if (sz < 0) sz = 0;
+  }
+  const long long chunk = ((sz + a.cpr - 1) / a.cpr + 31) & ~31LL;
+  const long long lo = (long long)ci * chunk < sz ? (long long)ci * chunk : sz;
+  const long long hi = lo + chunk < sz ? lo + chunk : sz;
+  const bool take_all = sz <= a.num;
+  if (take_all) {
+    int *o = a.out + (size_t)b * a.out_stride;
+    for (long long i = lo + threadIdx.x; i < hi; i += CT) o[i] = (int)i;
+  } else if (!sel_lists<K, CLU, VEC>(a, b, ci, sz, lo, hi)) {
+    sel_passes<K, CLU, VEC>(a, b, ci, sz, lo, hi);
+  }
+  if (a.count_out && ci == 0 && threadIdx.x == 0) a.count_out[b] = take_all ? (int)sz : a.num;
 }
 
 // CTAs of the cooperative form on the current device (-1: not available).
@@ -794,7 +1236,7 @@ int coop_grid() {
     }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sel_coop_kernel<K, false, VEC>, CT, COOP_SMEM);
     cudaGetLastError();
-    if (per > coop_ctas_per_sm<K>()) per = coop_ctas_per_sm<K>();
+    if (per > COOP_CTAS_PER_SM) per = COOP_CTAS_PER_SM;
     return per > 0 ? per * sms : -1;
   });
 }
