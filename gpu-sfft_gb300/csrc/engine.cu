@@ -206,6 +206,11 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
       t = fft_plan_shape(P->fftW, p.W_RLFC, FFT_FP32_TC);
     P->tc_rlfc = t == GSFFT_OK;
     if (!P->tc_rlfc) s = fft_plan_shape(P->fftW, p.W_RLFC, kind, tn.rlfc_first_radix);
+    // the ordered pass writes whole sectors of the sub-samples where the FFT reads them so
+    const int nbW = nb < p.W_RLFC ? nb : p.W_RLFC;
+    int lognc = 0;
+    while (((long long)nbW << lognc) < p.W_RLFC) lognc++;
+    P->y_lognc = P->use_stream && fft_reads_row_blocks(P->fftW, lognc) ? lognc : -1;
   }
   if (s == GSFFT_OK) {
     fft_plan_request(P->fftB, p.loops, mem);
@@ -387,7 +392,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   if (P->use_stream)
     GS_CHECK(launch_perm_filter_stream(P->precision, d_x, p.n, P->filt_bm, p.w, p.B, p.loops, d,
                                        P->bpart, p.RLFC_loops, P->ybuf, p.W_RLFC, &P->ctl->err, st,
-                                       P->groups));
+                                       P->groups, P->y_lognc >= 0 ? 2 : 0));
   else if (P->use_cols)
     GS_CHECK(launch_perm_filter_cols(d_x, p.n, P->filt_bm, P->filt, p.w, p.B, p.loops, d, P->bins, p.RLFC_loops,
                                      P->ybuf, p.W_RLFC, quirk, st));
@@ -441,6 +446,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
     const void *src = nullptr;
     if (P->use_stream || P->use_cols) {
       src = P->ybuf;
+      io.in_lognc = P->y_lognc;
     } else {
       io.gather_x = d_x;  // strided gather fused into the first FFT pass
       for (int r = 0; r < p.RLFC_loops; r++) io.gather_offsets[r] = d.offs[r];

@@ -42,6 +42,7 @@ struct Plan {
   RunCtl *ctl = nullptr;
   void *rmax = nullptr;  // per-row maxima: RLFC_loops rows then loops rows (u64 each)
   void *ybuf = nullptr;  // RLFC sub-samples written by the column-ordered perm+filter forms
+  int y_lognc = -1;      // FftIo::in_lognc of ybuf
   void *bpart = nullptr; // row-group partial bins of the streaming perm+filter
   void *filt_bm = nullptr; // bucket-major taps of the column-ordered perm+filter forms
   int groups = 1;

@@ -198,6 +198,15 @@ void fft_plan_free(FftPlan &p) {
   p = FftPlan();
 }
 
+// fused_first_stage (radix 2^11, 2^12): its steps of 128 and 256 in r are whole
+// blocks of rows from 128 rows on, and with no more rows than the radix a block's
+// rows are all read by the one CTA.
+bool fft_reads_row_blocks(const FftPlan &p, int lognc) {
+  if (p.npass < 2 || p.precision == GSFFT_FP64 || p.tc[0]) return false;
+  const int lr = p.logR[0], lognb = p.L - lognc;
+  return (lr == 11 || lr == 12) && p.L - lr >= 2 && lognb >= 7 && lognb <= lr;
+}
+
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
              const FftIo &io, cudaStream_t st) {
   if (p.npass == 0) return GSFFT_ERR_STATE;
@@ -206,6 +215,8 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
   if (p.npass > 1 && (long long)batch * p.n * (p.npass == 3 ? 2 : 1) > p.scratch_elems)
     return GSFFT_ERR_PARAM;
   if (io.gather_x && batch > 8) return GSFFT_ERR_PARAM;
+  if (io.in_lognc >= 0 && (io.sum_rows > 1 || io.gather_x || !fft_reads_row_blocks(p, io.in_lognc)))
+    return GSFFT_ERR_UNSUPPORTED;
   if (dbl && io.sum_rows > 1) return GSFFT_ERR_UNSUPPORTED;  // FP32 passes only
   const void *src = in;
   char *scr = (char *)p.scratch;
@@ -242,6 +253,7 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
     a.gstride = io.gather_stride;
     a.samples = last ? io.samples : nullptr;
     a.row_max = last ? io.row_max : nullptr;
+    a.lognc = i == 0 ? io.in_lognc : -1;
     a.nsum = (i == 0) ? io.sum_rows : 1;
     a.sstride = io.sum_stride;
     a.write_complex = last ? (io.write_complex ? 1 : 0) : 1;

@@ -45,6 +45,7 @@ struct PassArgs {
   void *row_max;      // per batch row, with samples
   int nsum;           // first pass: add nsum partial inputs sstride apart
   long long sstride;
+  int lognc;          // first pass: FftIo::in_lognc, or -1
   int write_complex;
   // FP64 passes: fixed-point twiddles -- the radix-16 stages' tables, and the
   // two-level table of exp(-2 pi i m / Np)
@@ -447,8 +448,7 @@ template <int LOGR> __host__ __device__ constexpr int first_radix() {
 }
 
 // First stage (Ns = 1, radix E = first_radix): butterfly t of row g reads
-// r = t + e NB, e < E, from src[r S] (src = the row's sub-transform j,
-// S = 2^logS), applies the conjugation and inter-pass twiddles in registers
+// r = t + e NB, e < E, from src[j + r S] (S = 2^logS), applies the conjugation and inter-pass twiddles in registers
 // and writes its outputs to shared memory.  Butterflies go to lanes so that
 // the shared-memory stores of each half-warp hit 16 distinct bank pairs with
 // the 16/G pitch, i.e. the half-warp's four butterflies fall on four
@@ -456,8 +456,8 @@ template <int LOGR> __host__ __device__ constexpr int first_radix() {
 // t; for E = 8 (padded(8 t + e) = 8 t + t/2 + e) four t of one parity (with
 // consecutive t, t and t + 2 would share a pair).
 template <typename V, int LOGR, int G>
-__device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ src, int logS, const PreTw &pt,
-                                                  int inverse) {
+__device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ src, long long j, int logS,
+                                                  int lognc, const PreTw &pt, int inverse) {
   constexpr int R = 1 << LOGR, E = first_radix<LOGR>();
   constexpr int LOGE = E == 2 ? 1 : (E == 4 ? 2 : (E == 8 ? 3 : 4));
   constexpr int NT = nt_of(LOGR), TPF = NT / G, RP = rowpitch<float>(LOGR);
@@ -472,7 +472,14 @@ __device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ s
     t0 = tid / G;
   }
   V v[Q][E];
-  const V *p = src + ((long long)t0 << logS);
+  // row blocks (lognc >= 0): TPF and NB steps of r are whole blocks of rows, so
+  // only the first address differs
+  long long m = j + ((long long)t0 << logS);
+  if (lognc >= 0) {
+    const long long row = m >> lognc, c = m & ((1LL << lognc) - 1);
+    m = ((row & ~3LL) << lognc) + 4 * c + (row & 3);
+  }
+  const V *p = src + m;
   const long long sq = (long long)TPF << logS, se = (long long)NB << logS;
 #pragma unroll
   for (int q = 0; q < Q; q++)
@@ -602,7 +609,7 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       const long long b = u >> logS, j = u & Smask;
       PreTw ptf = pt;  // inter-pass twiddles in registers wherever Ns > 1
       ptf.on = logNs > 0;
-      fused_first_stage<V, LOGR, G>(sm, in + b * a.bstride + j, logS, ptf, a.inverse);
+      fused_first_stage<V, LOGR, G>(sm, in + b * a.bstride, j, logS, a.lognc, ptf, a.inverse);
       __syncthreads();
       fused_mid_stages<V, LOGR, G, (LOGR % 4 == 0 ? 4 : LOGR % 4)>(sm, twR, pt);
       const long long d0 = b * a.bstride + ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask);

@@ -157,17 +157,30 @@ class Arena {
 // returns false, so that a kernel whose producer never arrives records an
 // error and returns instead of hanging the GPU.
 constexpr long long kWaitLimitCycles = 1LL << 30;
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar_smem_addr, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(done)
+      : "r"(bar_smem_addr), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ bool mbar_test(unsigned bar_smem_addr, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(done)
+      : "r"(bar_smem_addr), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned bar_smem_addr, unsigned parity,
                                                   long long limit = kWaitLimitCycles) {
+  if (mbar_try_wait(bar_smem_addr, parity)) return true;  // no clock read when it is done
   const long long t0 = clock64();
   while (true) {
-    unsigned done;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(bar_smem_addr), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_try_wait(bar_smem_addr, parity)) return true;
     if (clock64() - t0 > limit) return false;
   }
 }
@@ -292,6 +305,10 @@ struct FftIo {
   // in[s * sum_stride + index], added in s order (row-group partials)
   int sum_rows = 1;
   long long sum_stride = 0;
+  // first-pass loader alternative (fft_reads_row_blocks): the input is a matrix of
+  // 2^in_lognc columns in blocks of four rows, point t = row 2^in_lognc + column at
+  // (row & ~3) 2^in_lognc + 4 column + (row & 3); -1 = in order
+  int in_lognc = -1;
   // epilogue: |X|^2 (same precision) written to samples[b * n + k]
   void *samples = nullptr;
   // optional: per-row maximum of the samples (bit pattern, u64 for double /
@@ -317,6 +334,8 @@ int fft_plan_fill(const FftPlan &p, cudaStream_t st);
 // stream that the plan is then used on (or synchronised with).
 int fft_plan_init(FftPlan &p, long long n, FftKind kind, int max_batch, cudaStream_t st);
 void fft_plan_free(FftPlan &p);
+// whether the plan's first pass reads FftIo::in_lognc input in whole sectors
+bool fft_reads_row_blocks(const FftPlan &p, int lognc);
 // in: batch entries at in + b*n; out: out + b*n.  sign -1 forward, +1 inverse.
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
              const FftIo &io, cudaStream_t st);

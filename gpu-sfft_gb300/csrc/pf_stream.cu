@@ -15,22 +15,29 @@
 // i.e. the column's hit rows are one per-loop set {j*beta_l mod nb} shifted by
 // s_l.  The host sorts that set once per run; one thread per (column, loop)
 // walks its rotated copy in ascending row order, so it touches only its own
-// ~w/B hits while the CTA streams every row of its 64 (or 32) columns exactly
+// ~w/B hits while the CTA streams every row of its columns exactly
 // once.  Sums run in ascending row (= signal position) order: fixed, no
 // atomics.
 //
-// Tiles of rt rows x 64 columns arrive by cp.async.bulk.tensor.2d, issued by a
-// producer warp, into a shared-memory ring (three stages at two CTAs per SM;
-// four at one CTA per SM in the staged-tap form) guarded by full / empty
-// mbarriers whose waits are bounded (a timeout sets an error flag instead of
-// hanging).  Taps: in the staged form (FP32, up to 9 loops) each consumer
-// thread copies its bucket's taps into its own shared-memory slot with one
-// bulk copy per work item; otherwise each hit's tap is loaded from a
-// bucket-major table in L2, one hit ahead.
+// Tiles of 256 rows x 16 columns (FP32) arrive by cp.async.bulk.tensor.2d, issued
+// by a producer warp, into a shared-memory ring guarded by full / empty mbarriers
+// whose waits are bounded (a timeout sets an error flag instead of hanging).  Each
+// consumer warp copies its walks' taps into shared memory with cp.async at the
+// start of an item; where they do not fit beside two tiles, each hit's tap is
+// loaded from a bucket-major table in L2, one hit ahead.
 //
 // RLFC loop r samples positions off_r + m*(n/W) (restLocFreqCoeffKernel,
 // innerLoop.cu:693-703); (n/W) divides B, so those are whole columns and the
-// CTA copies them from the tile to y_r[t / (n/W)].
+// CTA copies them from the tile to y_r[t / (n/W)].  A tile holds few columns of a
+// loop, so y written in order is written in parts of 32-byte sectors, which cost
+// 104 us of the n = 2^27, k = 16000 step (250 at k = 43000): where the FFT can
+// read it so, y is in blocks of four rows instead, whole sectors.
+//
+// What bounds it: 2^27 FP32 samples are 1.07 GB, 150 us with no consumer.  Whole
+// steps went 438 -> 400 us (k = 16000), 1013 -> 896 (k = 43000, 8 columns of y a
+// tile) and 539 -> 466 (24 signals of 2^18 .. 2^24) from 64 x 64 tiles; what is
+// left above the stream is the RLFC copies (about 25 us at k = 16000) and the
+// scattered stores of the bins (16).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -43,16 +50,23 @@ namespace gsfft {
 namespace {
 
 constexpr int ST = 128;      // B must be a multiple of this
-constexpr int NSTAGE = 3;    // shared-memory ring of tiles (taps read from L2)
-constexpr int NSTAGE_STG = 4; // ring of the staged-tap form (one CTA per SM)
+// Columns of a tile: 128 bytes of a row in FP32.  Of 2^27 samples in rows of 2^17,
+// 16 columns x 256 rows stream at 7.0 TB/s with no consumer (64 x 64: 7.2, 8 x 256:
+// 5.7), and a walk meets its hits in a quarter of the tiles of 64 rows: the warps'
+// instructions a tile, not the memory, were the limit there.
+constexpr int LOGCW = 4, CW = 1 << LOGCW;
+constexpr int MINNS = 2, MAXNS = 8;  // tiles of the ring
 constexpr int MAXT = 32;     // full tiles of taps per bucket (w / B) supported
 constexpr int MAXL = 16;     // loops supported
-constexpr int PFD = 1;        // filter taps loaded ahead per thread
+// Two CTAs an SM, so that one loads an item's taps while the other walks.  Whole
+// step at n = 2^27, k = 16000 / 43000, RLFC copies off: 32 KiB tiles 401 / 836 us,
+// 16 KiB 428 / 952; one CTA with 32 KiB tiles 508 / 1036.
 constexpr int CTAS_PER_SM = 2;
+constexpr int PF_TILE = 32 * 1024;  // bytes of a tile, halved where the taps leave no room for two
+constexpr int PF_SMEM = (228 / CTAS_PER_SM - 1) * 1024 - 5 * 1024;  // dynamic bytes a CTA
+constexpr int MAXRW = 4;     // RLFC warps
+constexpr int MAXTH = 32 * (CW * MAXL / 32 + 1 + MAXRW);
 constexpr unsigned NONE = 0x7fffffffu;
-
-// columns per work item: one consumer thread per (column, loop)
-inline int cols_per_item(int loops) { return 64 * loops + 64 <= 1024 ? 64 : 32; }
 
 // taps per bucket in the bucket-major table: the w/B full-tile taps plus the
 // partial one, rounded up to even so that every bucket's row is a multiple of
@@ -77,14 +91,6 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_expect(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-// The signal streams through L2 once; marking its tiles evict-first keeps the
-// (re-read) filter taps resident in L2 instead of being pushed out by it.
 __device__ __forceinline__ unsigned long long policy_evict_first() {
   unsigned long long p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -106,16 +112,6 @@ __device__ __forceinline__ void tma_load_tile(void *dst, const CUtensorMap *tm, 
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
       " [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<unsigned long long>(tm)), "r"(x0), "r"(y0), "r"(smem_u32(bar)), "l"(pol)
-      : "memory");
-}
-
-// one bucket's taps (bytes: a multiple of 16) into this thread's slot
-__device__ __forceinline__ void bulk_load_taps(void *dst, const void *src, unsigned bytes,
-                                               unsigned long long *bar, unsigned long long pol) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
       : "memory");
 }
 
@@ -142,36 +138,36 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
 
 // Persistent, warp-specialised.  A work item is (block of CW columns, row
 // group); CTA b takes items b, b + grid, ...  Warp roles:
-//  * threads [0, CW*loops): consumers.  Thread (l, col) walks loop l of
-//    column col, so each warp covers 32 columns of one loop; its taps come
-//    from its shared-memory slot (staged form) or from the bucket-major tap
-//    table one hit ahead, so the L2 reads overlap the stream.
+//  * the first NCW warps: consumers.  Thread (l, col) walks loop l of column
+//    col; its taps come from its shared-memory slot (staged form) or from the
+//    bucket-major tap table one hit ahead, so the L2 reads overlap the stream.
 //  * the next warp: producer.  One lane streams every tile of the CTA's
-//    items, in order, into an NSTAGE ring (full[s]: tile landed, tx-counted;
-//    empty[s]: every releasing warp is done with it).
-//  * the last warp (RLFC loops only): copies the RLFC sub-samples out of
-//    each tile.
+//    items, in order, into a ring of NS tiles (full[s]: tile landed,
+//    tx-counted; empty[s]: every releasing warp is done with it).
+//  * the last warps (RLFC loops only): copy the RLFC sub-samples out of each
+//    tile.
 // No block-wide barrier inside the stream.
-template <typename T, int CW, int MAXTH, int NS, bool STG>
-__global__ void __launch_bounds__(MAXTH, (MAXTH <= 640 && !STG) ? CTAS_PER_SM : 1)
+// swz: 14 where the tile is stored with TMA's 128-byte swizzle (column c of row r
+// at c ^ 2 (r mod 8)), else 0.  The RLFC warps read down a column, 16 rows in one
+// bank without it: n = 2^27 step 414 -> 402 us.
+template <typename T, bool STG>
+__global__ void __launch_bounds__(MAXTH, CTAS_PER_SM)
 pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V *__restrict__ filt,
-              int logn, int logB, int w, int rt, int tiles, int rows_per_group, int groups, int L,
-              Draws d, HitTab ht, typename Cx<T>::V *__restrict__ bins, int nrlfc, int logsig,
-              typename Cx<T>::V *__restrict__ y, int W, int *err) {
+              int logn, int logB, int w, int rt, int ord, int NS, int tiles, int rows_per_group,
+              int groups, int L, Draws d, HitTab ht, typename Cx<T>::V *__restrict__ bins, int swz, int nrlfc,
+              int logsig, int logyr, typename Cx<T>::V *__restrict__ y, int W, int *err) {
   pdl_enter();
   typedef typename Cx<T>::V V;
-  constexpr int LOGCW = CW == 64 ? 6 : 5;
-  const int NCT = CW * L;  // consumer threads
-  const int NCW = NCT / 32;
-  const int NREL = NCW + (nrlfc > 0 ? 1 : 0);  // warps releasing each stage
-  extern __shared__ __align__(128) unsigned char dsm[];
+  const int NCT = CW * L;  // walks of an item
+  const int NCW = (NCT + 31) / 32;
+  const int nrw = (int)blockDim.x / 32 - NCW - 1;  // RLFC warps
+  extern __shared__ __align__(1024) unsigned char dsm[];
   // each loop's sorted list twice in a row, so a rotated walk needs no wrap
   __shared__ unsigned S2[MAXL][2 * MAXT];
   __shared__ unsigned s_a[MAXL], s_beta[MAXL], s_xrow[MAXL];
-  __shared__ __align__(8) unsigned long long full[NS], empty[NS];
-  __shared__ __align__(8) unsigned long long tapbar[STG ? MAXTH / 32 : 1];
+  __shared__ __align__(8) unsigned long long full[MAXNS], empty[MAXNS];
   __shared__ volatile int abort_flag;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int B = 1 << logB;
   const int lognb = logn - logB;
   const int nb = 1 << lognb;
@@ -198,29 +194,42 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
     abort_flag = 0;
     for (int s = 0; s < NS; s++) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], NREL);
+      mbar_init(&empty[s], (unsigned)(NCW + nrw));
     }
-    if (STG)
-      for (int i = 0; i < NCW; i++) mbar_init(&tapbar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
 
-  const unsigned smask = (1u << logsig) - 1u;
-  if (tid >= NCT + 32) {
-    // ---------------- RLFC warp: loop r samples positions off_r + m*(n/W)
+  int st = 0;       // stage of the current tile ...
+  unsigned ph = 0;  // ... and its phase
+  auto next_tile = [&]() {
+    if (++st == NS) {
+      st = 0;
+      ph ^= 1u;
+    }
+  };
+
+  if (warp > NCW) {
+    // ---------------- RLFC warps: loop r samples positions off_r + m*(n/W)
     // (restLocFreqCoeffKernel, innerLoop.cu:693-703); n/W divides B, so those
     // are whole columns, copied from the tile to y_r[t / (n/W)]
-    if (nrlfc == 0) return;
-    const int lane = tid & 31;
-    long long k = 0;
+    const unsigned smask = (1u << logsig) - 1u;
+    const int lognc = logsig >= LOGCW ? 0 : LOGCW - logsig;  // log2 of a loop's columns in a block
+    // A loop's samples in a tile, in order: row within its block, column, block of
+    // rows.  A thread's next sample is whole blocks of rows on (32 nrw threads are a
+    // multiple of a block's samples), in the same column.
+    const int e0 = tid - 32 * (NCW + 1);
+    const int ci = (e0 >> logyr) & ((1 << lognc) - 1);
+    const int row0 = ((e0 >> (logyr + lognc)) << logyr) + (e0 & ((1 << logyr) - 1));
+    const int rstep = (32 * nrw >> (logyr + lognc)) << logyr;
+    const size_t ystep = (size_t)rstep << (logB - logsig);
+    constexpr int U = 4;  // copies in flight per thread
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
       const int cb = it % ncb, g = it / ncb;
-      const int c0 = cb * CW;
-      for (int t = 0; t < ntile; t++, k++) {
-        const int st = (int)(k % NS);
+      const unsigned c0 = (unsigned)(cb * CW);
+      for (int t = 0; t < ntile; t++, next_tile()) {
         const V *tl = tile0 + (size_t)st * rt * CW;
-        if (!mbar_wait(&full[st], (unsigned)((k / NS) & 1))) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[st], ph))) {
           abort_flag = 1;
           atomicExch(err, 1);
           return;
@@ -228,14 +237,22 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
         const unsigned r0 = (unsigned)(g * rows_per_group + t * rt);
         for (int rr = 0; rr < nrlfc; rr++) {
           const unsigned off = (unsigned)d.offs[rr];
-          const unsigned first = ((off - (unsigned)c0) & smask);  // first matching column
+          const unsigned first = (off - c0) & smask;  // first matching column
           if (first >= (unsigned)CW) continue;
-          const int lognc = logsig >= LOGCW ? 0 : LOGCW - logsig;  // log2 of the column count
-          for (int e = lane; e < (rt << lognc); e += 32) {
-            const int row = e >> lognc, ci = e & ((1 << lognc) - 1);
-            const unsigned cc = first + ((unsigned)ci << logsig);
-            const unsigned tpos = ((r0 + row) << logB) + (unsigned)c0 + cc;
-            y[(size_t)rr * W + ((tpos - off) >> logsig)] = tl[(row << LOGCW) + cc];
+          const unsigned ci0 = (c0 + first - off) >> logsig;
+          const unsigned scol = first + ((unsigned)ci << logsig);
+          V *yp = y + (size_t)rr * W + (e0 & ((1 << logyr) - 1)) +
+                  (((size_t)((r0 + row0) >> logyr) << (logB - logsig)) + ci0 + ci << logyr);
+          for (int row = row0; row < rt; row += U * rstep) {
+            V v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              const int ru = row + u * rstep;
+              if (ru < rt) v[u] = tl[(ru << LOGCW) + (scol ^ ((ru << 1) & swz))];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++, yp += ystep)
+              if (row + u * rstep < rt) *yp = v[u];
           }
         }
         __syncwarp();
@@ -244,17 +261,16 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
     }
     return;
   }
-  if (tid >= NCT) {
+  if (warp == NCW) {
     // ---------------- producer
-    if (tid == NCT) {
+    if (lane == 0) {
       const unsigned long long pol = policy_evict_first();
-      long long k = 0;
+      int k = 0;
       bool ok = true;
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
         const int cb = it % ncb, g = it / ncb;
-        for (int t = 0; t < ntile; t++, k++) {
-          const int st = (int)(k % NS);
-          if (!mbar_wait(&empty[st], (unsigned)((k / NS) & 1) ^ 1u) || abort_flag) {
+        for (int t = 0; t < ntile; t++, k++, next_tile()) {
+          if (!mbar_wait(&empty[st], ph ^ 1u) || abort_flag) {
             abort_flag = 1;
             ok = false;
             break;
@@ -265,7 +281,7 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
         }
       }
       // stay until the last load of every stage has landed (bounded)
-      for (long long j = k - NS < 0 ? 0 : k - NS; j < k; j++)
+      for (int j = k - NS < 0 ? 0 : k - NS; j < k; j++)
         if (!mbar_wait(&full[j % NS], (unsigned)((j / NS) & 1))) {
           atomicExch(err, 1);
           break;
@@ -275,40 +291,47 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
   }
 
   // ---------------- consumers
-  const int col = tid & (CW - 1), l = tid >> LOGCW, lane = tid & 31;
+  const bool act = tid < NCT;  // the last warp of an odd loop count is half full
+  const int col = tid & (CW - 1), l = act ? tid >> LOGCW : 0;
   const int residue = w & (B - 1);
   const unsigned a = s_a[l], beta = s_beta[l], xrow = s_xrow[l];
   const unsigned *S = S2[l];
   const unsigned long long keep = policy_evict_last();
-  long long k = 0;
-  // staged form: this thread's slot of TT taps after the tile ring, and its
-  // warp's copy barrier
+  // staged form: this thread's slot of TT taps after the tile ring
   V *const tslot = reinterpret_cast<V *>(dsm + (size_t)NS * stage_bytes) + (size_t)tid * TT;
-  unsigned long long *const tbar = &tapbar[STG ? (tid >> 5) : 0];
-  unsigned tap_phase = 0;
+  const int nch = (int)(TT * sizeof(V) / 16);  // 16-byte pieces of a slot
+  const int dq = 32 / nch, dr = 32 - dq * nch;
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int cb = it % ncb, g = it / ncb;
     const int c0 = cb * CW;
     const unsigned c = (unsigned)(c0 + col);
     const int rbeg = g * rows_per_group;
     // Walk state.  Rotated position k of the column's hit list is
-    // doubled-list entry m = mw + k; its row is v + s - nb when m < tiles (the
-    // entry wrapped past nb) and v + s otherwise.
+    // doubled-list entry m = mw + k; its row is (v + s) mod nb.
     const unsigned prod = c * a;
     const int bl = (int)(prod & (unsigned)(B - 1));
     const unsigned q = (prod & nmask) >> logB;
     const unsigned sl = (0u - q * beta) & nbm;
     const V *fcol = filt + (size_t)bl * TT;  // the bucket's taps, contiguous
     if constexpr (STG) {
-      // One bulk copy of the bucket's taps into this thread's slot per item,
-      // completing on the warp's barrier.  At the first __syncwarp every lane
-      // is past its last read of the previous taps and its wait on the
-      // previous phase; the proxy fence orders those reads before the copy.
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      // the warp copies its walks' taps together, 16 bytes a lane, so that a
+      // load covers whole rows; every lane is past its last read of the old ones
       __syncwarp();
-      if (lane == 0) mbar_arrive_expect(tbar, 32u * (unsigned)(TT * sizeof(V)));
-      __syncwarp();
-      bulk_load_taps(tslot, fcol, (unsigned)(TT * sizeof(V)), tbar, keep);
+      int row = (warp << 5) + lane / nch, part = lane - lane / nch * nch;
+      const int end = min(NCT, (warp + 1) << 5);
+      unsigned dst = smem_u32(tslot - (size_t)lane * TT) + (unsigned)lane * 16u;
+      while (row < end) {
+        const unsigned br = ((unsigned)(c0 + (row & (CW - 1))) * s_a[row >> LOGCW]) & (unsigned)(B - 1);
+        const char *src = reinterpret_cast<const char *>(filt + (size_t)br * TT) + part * 16;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        dst += 512u;
+        row += dq;
+        part += dr;
+        if (part >= nch) {
+          part -= nch;
+          row++;
+        }
+      }
     }
     // mw: first sorted entry with v >= nb - s (binary search)
     int lo = 0, hi = tiles;
@@ -321,93 +344,74 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
     const int mw = lo;
     // first rotated position with row >= rbeg (binary search)
     lo = 0;
-    hi = tiles;
+    hi = rbeg ? tiles : 0;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      const int m = mw + mid;
-      const unsigned row = (S[m] >> 8) + sl - (m < tiles ? (unsigned)nb : 0u);
-      if (row < (unsigned)rbeg) lo = mid + 1;
+      if ((((S[mw + mid] >> 8) + sl) & nbm) < (unsigned)rbeg) lo = mid + 1;
       else hi = mid;
     }
     int mc = mw + lo;
-    const int me = mw + tiles;
-    unsigned nm = NONE, er = NONE, ent = 0;
-    // taps of the next PFD hits, loaded ahead (the last entries of the
-    // doubled list are valid indices, so loading past me is harmless)
-    V fv[PFD];
-    if constexpr (!STG) {
-#pragma unroll
-      for (int u = 0; u < PFD; u++)
-        fv[u] = ld_tap(fcol + (S[min(mc + u, 2 * tiles - 1)] & 255u), keep);
-    }
-    V fe = mk((T)0, (T)0);
-    if (mc < me) {
-      ent = S[mc];
-      nm = (ent >> 8) + sl - (mc < tiles ? (unsigned)nb : 0u);
-    }
-    if (bl < residue) {
+    const int me = act ? mw + tiles : 0;
+    // the next hit's row, its tap and the entry after it, loaded a hit ahead, so
+    // that a hit waits for its sample alone (S has entries past the last, and
+    // the tap of one is a valid one)
+    auto tap = [&](unsigned j) {
+      if constexpr (STG) return tslot[j];
+      else return ld_tap(fcol + j, keep);
+    };
+    unsigned nm = NONE, er = NONE, ent = S[mc];
+    if (mc < me) nm = ((ent >> 8) + sl) & nbm;
+    if (act && bl < residue) {
       er = (xrow + sl) & nbm;
       if (er < (unsigned)rbeg) er = NONE;
-      else if constexpr (!STG) fe = ld_tap(fcol + tiles, keep);
     }
     if constexpr (STG) {
-      if (!mbar_wait(tbar, tap_phase)) {
-        abort_flag = 1;
-        atomicExch(err, 1);
-        return;
-      }
-      tap_phase ^= 1u;
-      if (er != NONE) fe = tslot[tiles];
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
     }
+    V fe = mk((T)0, (T)0), ftap = fe;
+    if (er != NONE) fe = tap((unsigned)tiles);
+    if (act) ftap = tap(ent & 255u);
+    ent = S[mc + 1];
     T re = 0, im = 0;
 
-    for (int t = 0; t < ntile; t++, k++) {
-      const int st = (int)(k % NS);
-      const V *tl = tile0 + (size_t)st * rt * CW;
-      if (!mbar_wait(&full[st], (unsigned)((k / NS) & 1))) {
+    for (int t = 0; t < ntile; t++, next_tile()) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[st], ph))) {
         abort_flag = 1;
         atomicExch(err, 1);
         return;
       }
       const unsigned r0 = (unsigned)(rbeg + t * rt), r1 = r0 + (unsigned)rt;
-      // full-tile taps in ascending row order, then the partial tap if it
-      // falls in this tile
-      while (nm < r1) {
-        const V xv = tl[((nm - r0) << LOGCW) + col];
-        V f;
-        if constexpr (STG) f = tslot[ent & 255u];
-        else f = fv[0];
+      const V *tl = tile0 + (size_t)st * rt * CW;
+      auto add = [&](unsigned row, V f) {
+        const V xv = tl[((row - r0) << LOGCW) + ((unsigned)col ^ ((row << 1) & (unsigned)swz))];
         re = fma(xv.x, f.x, re);
         re = fma(-xv.y, f.y, re);
         im = fma(xv.x, f.y, im);
         im = fma(xv.y, f.x, im);
-        const int m = ++mc;
-        if constexpr (STG) {
-          nm = NONE;
-          if (m < me) {
-            ent = S[m];
-            nm = (ent >> 8) + sl - (m < tiles ? (unsigned)nb : 0u);
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u + 1 < PFD; u++) fv[u] = fv[u + 1];
-          fv[PFD - 1] = ld_tap(fcol + (S[min(m + PFD - 1, 2 * tiles - 1)] & 255u), keep);
-          nm = m < me ? (S[m] >> 8) + sl - (m < tiles ? (unsigned)nb : 0u) : NONE;
+      };
+      // full-tile taps in ascending row order, the partial tap after those of
+      // its block of ord rows (the order of the sums does not depend on rt)
+      while (nm < r1) {
+        if ((er | (unsigned)(ord - 1)) < nm) {
+          add(er, fe);
+          er = NONE;
         }
+        add(nm, ftap);
+        const int m = ++mc;
+        nm = m < me ? ((ent >> 8) + sl) & nbm : NONE;
+        ftap = tap(ent & 255u);
+        ent = S[m + 1];
       }
       if (er < r1) {
-        const V xv = tl[((er - r0) << LOGCW) + col];
-        re = fma(xv.x, fe.x, re);
-        re = fma(-xv.y, fe.y, re);
-        im = fma(xv.x, fe.y, im);
-        im = fma(xv.y, fe.x, im);
+        add(er, fe);
         er = NONE;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[st]);
     }
     // partial sums of this row group: bins[group][l][b]
-    bins[((size_t)g * L + l) * B + bl] = mk(re, im);
+    if (act) bins[((size_t)g * L + l) * B + bl] = mk(re, im);
   }
 }
 
@@ -563,25 +567,46 @@ unsigned inv_odd(unsigned a) {  // a^-1 mod 2^32 for odd a (Newton)
   return x;
 }
 
-// dynamic shared memory of one CTA: the tile ring, plus the consumers' tap
-// slots in the staged form
-inline int pf_smem_bytes(int es, int cw, int rt, int loops, int tiles, int ns, bool stg) {
-  return ns * rt * cw * es + (stg ? cw * loops * taps_per_bucket(tiles) * es : 0);
+// Tile of a pass: its rows, the ring's depth, and whether the taps are staged in
+// shared memory (always but for the longest windows of the most loops).
+struct PfTile {
+  int rt, ns, swz;
+  bool staged;
+};
+inline PfTile pf_tile(int rows_per_group, int es, int loops, int tiles, int ord) {
+  PfTile t;
+  const int slots = CW * loops * taps_per_bucket(tiles) * es;
+  const int rt = std::min(rows_per_group, PF_TILE / (CW * es));
+  t.rt = rt;
+  if (PF_SMEM - slots < MINNS * rt * CW * es && rt / 2 >= ord) t.rt = rt / 2;
+  t.staged = PF_SMEM - slots >= MINNS * t.rt * CW * es;
+  if (!t.staged) t.rt = rt;
+  t.ns = std::min(MAXNS, (PF_SMEM - (t.staged ? slots : 0)) / (t.rt * CW * es));
+  // the swizzle spans 128-byte rows, in groups of eight from the tile's start
+  t.swz = CW * es == 128 && t.rt % 8 == 0 ? 14 : 0;
+  return t;
 }
-constexpr int PF_SMEM_LIMIT = 218 * 1024;  // dynamic bytes, leaving room for the static tables
 
-template <typename T, int CW, int MAXTH, int NS, bool STG>
-int launch_CW(const CUtensorMap &tm, const void *filt, int logn, int logB, int w, int rt, int tiles,
-              int groups, int loops, const Draws &d, const HitTab &ht, void *bins, int nrlfc,
-              int logsig, void *y, int W, int *err, cudaStream_t st) {
+template <typename T, bool STG>
+int launch_T(const CUtensorMap &tm, const void *filt, int logn, int logB, int w, const PfTile &pt, int ord,
+             int tiles, int groups, int loops, const Draws &d, const HitTab &ht, void *bins, int nrlfc,
+             int logsig, int logyr, void *y, int W, int *err, cudaStream_t st) {
   typedef typename Cx<T>::V V;
   const int B = 1 << logB;
-  const int smem = pf_smem_bytes((int)sizeof(V), CW, rt, loops, tiles, NS, STG);
-  const int threads = CW * loops + (nrlfc > 0 ? 64 : 32);
+  const int smem = (int)sizeof(V) * (pt.ns * pt.rt * CW + (STG ? CW * loops * taps_per_bucket(tiles) : 0));
+  // RLFC warps: a power of two, one for 256 samples of a tile (one for 512 held
+  // the ring back: 424 against 402 us), and whole blocks of rows a step
+  int rw = 0;
+  if (nrlfc) {
+    const int lognc = std::max(0, LOGCW - logsig), per_tile = std::max(pt.rt * nrlfc * CW >> logsig, 1);
+    rw = 1;
+    while (rw < MAXRW && (rw * 256 < per_tile || 32 * rw < 1 << (logyr + lognc))) rw *= 2;
+  }
+  const int threads = 32 * ((CW * loops + 31) / 32 + 1 + rw);
   static PerContext<int> attr;  // the kernel's dynamic shared memory limit, per context
   GS_CHECK(attr.ensure_at_least(smem, [](int v) {
-    if (cudaFuncSetAttribute(pf_tma_kernel<T, CW, MAXTH, NS, STG>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, v) == cudaSuccess)
+    if (cudaFuncSetAttribute(pf_tma_kernel<T, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize, v) ==
+        cudaSuccess)
       return (int)GSFFT_OK;
     set_last_error("pf_tma_kernel: %d bytes of shared memory refused: %s", v,
                    cudaGetErrorString(cudaGetLastError()));
@@ -590,53 +615,14 @@ int launch_CW(const CUtensorMap &tm, const void *filt, int logn, int logB, int w
   int dev = 0, sms = 0, per_sm = 0;
   GS_CUDA(cudaGetDevice(&dev));
   GS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf_tma_kernel<T, CW, MAXTH, NS, STG>,
-                                                        threads, smem));
+  GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pf_tma_kernel<T, STG>, threads, smem));
   const int items = (B / CW) * groups;
   const int grid = std::max(1, std::min(items, std::max(per_sm, 1) * sms));
   const int rows_per_group = (1 << (logn - logB)) / groups;
-  GS_CUDA(launch_pdl(pf_tma_kernel<T, CW, MAXTH, NS, STG>, dim3(grid), dim3(threads), smem, st, tm,
-                     (const V *)filt, logn, logB, w, rt, tiles, rows_per_group, groups, loops, d, ht,
-                     (V *)bins, nrlfc, logsig, (V *)y, W, err));
+  GS_CUDA(launch_pdl(pf_tma_kernel<T, STG>, dim3(grid), dim3(threads), smem, st, tm, (const V *)filt, logn,
+                     logB, w, pt.rt, ord, pt.ns, tiles, rows_per_group, groups, loops, d, ht, (V *)bins, pt.swz, nrlfc,
+                     logsig, logyr, (V *)y, W, err));
   return GSFFT_OK;
-}
-
-// FP32 reads the taps from a per-thread shared-memory copy (one bulk copy per
-// work item) when the slots fit beside a ring of NSTAGE_STG tiles: a warp's
-// scattered 8-byte tap loads from L2 touched 32 cache lines each and were the
-// limit of the pass.
-inline bool pf_stream_staged(int cw, int rt, int loops, int tiles) {
-  return pf_smem_bytes(8, cw, rt, loops, tiles, NSTAGE_STG, true) <= PF_SMEM_LIMIT;
-}
-// The same form for 10 to 15 loops (up to 1024 threads): the slots take more
-// room, so the ring keeps NSTAGE tiles.
-inline bool pf_stream_staged_wide(int cw, int rt, int loops, int tiles) {
-  return cw == 64 && 64 * loops + 64 <= 1024 &&
-         pf_smem_bytes(8, cw, rt, loops, tiles, NSTAGE, true) <= PF_SMEM_LIMIT;
-}
-
-template <typename T>
-int dispatch(int loops, const CUtensorMap &tm, const void *filt, int logn, int logB, int w, int rt,
-             int tiles, int groups, const Draws &d, const HitTab &ht, void *bins, int nrlfc,
-             int logsig, void *y, int W, int *err, cudaStream_t st) {
-  const int cw = cols_per_item(loops);
-  const bool small = cw * loops + (nrlfc > 0 ? 64 : 32) <= 640;
-#define GO(CWV, MT, NSV, STGV)                                                                     \
-  return launch_CW<T, CWV, MT, NSV, STGV>(tm, filt, logn, logB, w, rt, tiles, groups, loops, d, ht, \
-                                          bins, nrlfc, logsig, y, W, err, st)
-  if (cw == 64) {
-    if (small) {
-      if constexpr (sizeof(T) == 4)
-        if (pf_stream_staged(cw, rt, loops, tiles)) GO(64, 640, NSTAGE_STG, true);
-      GO(64, 640, NSTAGE, false);
-    }
-    if constexpr (sizeof(T) == 4)
-      if (pf_stream_staged_wide(cw, rt, loops, tiles)) GO(64, 1024, NSTAGE, true);
-    GO(64, 1024, NSTAGE, false);
-  }
-  if (small) GO(32, 640, NSTAGE, false);
-  GO(32, 1024, NSTAGE, false);
-#undef GO
 }
 
 }  // namespace
@@ -686,14 +672,14 @@ int stream_pf_groups(int n, int B, int w, int loops, int precision) {
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int cw = cols_per_item(loops);
-  // the staged FP32 forms run one CTA per SM (the dispatch's choice)
-  const bool stg = precision != GSFFT_FP64 && cw == 64 &&
-                   (64 * loops + 64 <= 640 ? pf_stream_staged(cw, rt, loops, w / B)
-                                           : pf_stream_staged_wide(cw, rt, loops, w / B));
-  // enough work items (column block x row group) for ~6 per persistent CTA,
-  // each item at least four tiles long
-  const long long want = 6LL * (stg ? 1 : CTAS_PER_SM) * sms;
+  // The groups' partial sums fix the FP32 rounding, so this rule does not follow
+  // the kernel's own tiles: blocks of 64 columns (32 above 15 loops) and 6 or 12
+  // items per SM, the former where a block's FP32 taps leave half the shared memory.
+  const int cw = 64 * loops + 64 <= 1024 ? 64 : 32;
+  const int slots = 8 * cw * loops * taps_per_bucket(w / B), tile = 8 * rt * cw;
+  const bool few = precision != GSFFT_FP64 && cw == 64 &&
+                   (loops <= 9 ? 4 : 3) * tile + slots <= 218 * 1024;
+  const long long want = (few ? 6LL : 12LL) * sms;
   int groups = 1;
   while ((long long)(B / cw) * groups < want && nb / (groups * 2) >= 4 * rt) groups *= 2;
   return groups;
@@ -736,7 +722,7 @@ int launch_perm_filter_cols(const void *x, int n, const void *filt, const void *
 
 int launch_perm_filter_stream(int precision, const void *x, int n, const void *filt, int w, int B,
                               int loops, const Draws &d, void *bins, int nrlfc, void *y, int W,
-                              int *err, cudaStream_t st, int groups_req) {
+                              int *err, cudaStream_t st, int groups_req, int logyr) {
   if (!stream_pf_supported(n, B, loops, W, nrlfc)) return GSFFT_ERR_UNSUPPORTED;
   const int tiles = w / B;
   if (tiles >= MAXT || tiles > 255) return GSFFT_ERR_UNSUPPORTED;
@@ -747,30 +733,34 @@ int launch_perm_filter_stream(int precision, const void *x, int n, const void *f
   // x as a 2-D tensor of 8-byte words: nb rows of B (FP32) or 2B (FP64) words
   const bool dbl = precision == GSFFT_FP64;
   const int es = dbl ? 16 : 8;
-  const int rt = stream_rows_per_tile(n, B, precision);
+  const int ord = stream_rows_per_tile(n, B, precision);
   int groups = stream_pf_groups(n, B, w, loops, precision);
   if (groups_req > 0) {
     if (!stream_pf_groups_valid(n, B, groups_req, precision)) return GSFFT_ERR_PARAM;
     groups = groups_req;
   }
-  const int cw = cols_per_item(loops);
+  const PfTile pt = pf_tile(nb / groups, es, loops, tiles, ord);
   CUtensorMap tm;
   const cuuint64_t gdim[2] = {(cuuint64_t)B * (es / 8), (cuuint64_t)nb};
   const cuuint64_t gstride[1] = {(cuuint64_t)B * es};
-  const cuuint32_t box[2] = {(cuuint32_t)(cw * (es / 8)), (cuuint32_t)rt};
+  const cuuint32_t box[2] = {(cuuint32_t)(CW * (es / 8)), (cuuint32_t)pt.rt};
   const cuuint32_t estr[2] = {1, 1};
+  // 128-byte L2 fetches: with 256 the neighbour's half was fetched twice (1.55 GB
+  // read for 1.07, the first-read data being evicted first)
   CUresult cr = encode_fn()(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void *>(x), gdim,
                             gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                            pt.swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (cr != CUDA_SUCCESS) {
     set_last_error("cuTensorMapEncodeTiled failed (%d)", (int)cr);
     return GSFFT_ERR_CUDA;
   }
-  int s = dbl ? dispatch<double>(loops, tm, filt, logn, logB, w, rt, tiles, groups, d, ht, bins,
-                                 nrlfc, logsig, y, W, err, st)
-              : dispatch<float>(loops, tm, filt, logn, logB, w, rt, tiles, groups, d, ht, bins, nrlfc,
-                                logsig, y, W, err, st);
+  auto go = [&](auto launch) {
+    return launch(tm, filt, logn, logB, w, pt, ord, tiles, groups, loops, d, ht, bins, nrlfc, logsig, logyr, y,
+                  W, err, st);
+  };
+  const int s = dbl ? (pt.staged ? go(launch_T<double, true>) : go(launch_T<double, false>))
+                    : (pt.staged ? go(launch_T<float, true>) : go(launch_T<float, false>));
   if (s != GSFFT_OK) return s;
   GS_LAUNCHED();
   return GSFFT_OK;

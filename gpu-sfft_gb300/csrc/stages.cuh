@@ -51,9 +51,11 @@ int stream_taps_count(int w, int B);
 int launch_stream_taps(int precision, const void *filt, int w, int B, void *taps_bm, cudaStream_t st);
 // filt here is the bucket-major table
 // groups: row groups (partial bin sets) of the pass; 0 = stream_pf_groups
+// logyr: y in blocks of 2^logyr rows of its (n/B) x (B W/n) matrix, the rows of a
+// block side by side (FftIo::in_lognc reads blocks of four); 0 = row by row
 int launch_perm_filter_stream(int precision, const void *x, int n, const void *filt, int w, int B,
                               int loops, const Draws &d, void *bins, int nrlfc, void *y, int W,
-                              int *err, cudaStream_t st, int groups = 0);
+                              int *err, cudaStream_t st, int groups = 0, int logyr = 0);
 // The same walk over the columns with gathers instead of a streamed signal, FP64
 // (filt: the bucket-major table; qfilt: the taps in bucket order, for the residue
 // quirk; y as above).
