@@ -207,6 +207,18 @@ bool fft_reads_row_blocks(const FftPlan &p, int lognc) {
   return (lr == 11 || lr == 12) && p.L - lr >= 2 && lognb >= 7 && lognb <= lr;
 }
 
+// FP32, two passes, the first with fused loads and stores (radix 2^11, 2^12), the second
+// one that takes four sub-transforms at a time (2^10 .. 2^12): between them the
+// array is kept tile by tile, point r of sub-transform j of the second pass at
+// (j & ~3) R + 4 r + (j & 3).  The second pass reads whole lines in order, not a
+// sector every N/R points (its loads were a third of its time: L1 lines, not DRAM),
+// and the first writes lines, not half ones.  Second pass of two rows of 2^24:
+// 221 -> 185 us.
+static bool fft_tiled(const FftPlan &p) {
+  return p.npass == 2 && p.precision != GSFFT_FP64 && !p.tc[0] && !p.tc[1] && (p.logR[0] == 11 || p.logR[0] == 12) &&
+         p.logR[1] >= 10 && p.logR[1] <= 12;
+}
+
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
              const FftIo &io, cudaStream_t st) {
   if (p.npass == 0) return GSFFT_ERR_STATE;
@@ -218,6 +230,7 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
   if (io.in_lognc >= 0 && (io.sum_rows > 1 || io.gather_x || !fft_reads_row_blocks(p, io.in_lognc)))
     return GSFFT_ERR_UNSUPPORTED;
   if (dbl && io.sum_rows > 1) return GSFFT_ERR_UNSUPPORTED;  // FP32 passes only
+  const bool tiled = fft_tiled(p) && !io.gather_x && io.sum_rows <= 1;
   const void *src = in;
   char *scr = (char *)p.scratch;
   long long Ns = 1;
@@ -254,6 +267,8 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
     a.samples = last ? io.samples : nullptr;
     a.row_max = last ? io.row_max : nullptr;
     a.lognc = i == 0 ? io.in_lognc : -1;
+    a.tile_out = tiled && i == 0;
+    a.tile_in = tiled && i == 1;
     a.nsum = (i == 0) ? io.sum_rows : 1;
     a.sstride = io.sum_stride;
     a.write_complex = last ? (io.write_complex ? 1 : 0) : 1;

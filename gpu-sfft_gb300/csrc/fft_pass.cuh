@@ -46,6 +46,7 @@ struct PassArgs {
   int nsum;           // first pass: add nsum partial inputs sstride apart
   long long sstride;
   int lognc;          // first pass: FftIo::in_lognc, or -1
+  int tile_in, tile_out;  // the array between two passes in tiles of four sub-transforms (fft_tiled)
   int write_complex;
   // FP64 passes: fixed-point twiddles -- the radix-16 stages' tables, and the
   // two-level table of exp(-2 pi i m / Np)
@@ -457,7 +458,7 @@ template <int LOGR> __host__ __device__ constexpr int first_radix() {
 // consecutive t, t and t + 2 would share a pair).
 template <typename V, int LOGR, int G>
 __device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ src, long long j, int logS,
-                                                  int lognc, const PreTw &pt, int inverse) {
+                                                  int lognc, int tile_in, const PreTw &pt, int inverse) {
   constexpr int R = 1 << LOGR, E = first_radix<LOGR>();
   constexpr int LOGE = E == 2 ? 1 : (E == 4 ? 2 : (E == 8 ? 3 : 4));
   constexpr int NT = nt_of(LOGR), TPF = NT / G, RP = rowpitch<float>(LOGR);
@@ -479,8 +480,13 @@ __device__ __forceinline__ void fused_first_stage(V *sm, const V *__restrict__ s
     const long long row = m >> lognc, c = m & ((1LL << lognc) - 1);
     m = ((row & ~3LL) << lognc) + 4 * c + (row & 3);
   }
+  int logs = logS;
+  if (tile_in) {
+    m = (j & ~3LL) * R + 4 * t0 + (j & 3);
+    logs = 2;
+  }
   const V *p = src + m;
-  const long long sq = (long long)TPF << logS, se = (long long)NB << logS;
+  const long long sq = (long long)TPF << logs, se = (long long)NB << logs;
 #pragma unroll
   for (int q = 0; q < Q; q++)
 #pragma unroll
@@ -529,6 +535,9 @@ __device__ __forceinline__ void fused_last_stage(const V *sm, const V *__restric
   V *__restrict__ out = reinterpret_cast<V *>(a.out);
   T *__restrict__ smp = reinterpret_cast<T *>(a.samples);
   T tmax = 0;
+  // tiled output (a first pass: d0 = the row's start + j): four adjacent outputs of
+  // four adjacent sub-transforms are one 128-byte line
+  const int logR2 = a.logN - LOGR;
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     const int t = t0 + q * TPF;
@@ -542,7 +551,8 @@ __device__ __forceinline__ void fused_last_stage(const V *sm, const V *__restric
     for (int e = 0; e < E; e++) {
       V x = v[bitrev<E>(e)];
       if (a.inverse) x.y = -x.y;
-      const long long d = d0 + ((long long)(t + e * NB) << logNs);
+      const long long k = t + e * NB;
+      const long long d = a.tile_out ? d0 + ((k & ~3LL) << logR2) + (k & 3) : d0 + (k << logNs);
       if (a.write_complex) out[d] = x;
       if (smp) {
         const T sv = sq_sum(x);
@@ -609,10 +619,11 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       const long long b = u >> logS, j = u & Smask;
       PreTw ptf = pt;  // inter-pass twiddles in registers wherever Ns > 1
       ptf.on = logNs > 0;
-      fused_first_stage<V, LOGR, G>(sm, in + b * a.bstride, j, logS, a.lognc, ptf, a.inverse);
+      fused_first_stage<V, LOGR, G>(sm, in + b * a.bstride, j, logS, a.lognc, a.tile_in, ptf, a.inverse);
       __syncthreads();
       fused_mid_stages<V, LOGR, G, (LOGR % 4 == 0 ? 4 : LOGR % 4)>(sm, twR, pt);
-      const long long d0 = b * a.bstride + ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask);
+      const long long d0 =
+          b * a.bstride + (a.tile_out ? 4 * j : ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask));
       fused_last_stage<T, V, LOGR, G>(sm, twR, a, b, d0, logNs);
       return;
     }
@@ -626,8 +637,8 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       for (int q = 0; q < ITER; q++) dst[q * TPF + ((q * TPF) >> 4)] = mk((T)0, (T)0);
     } else {
       const long long b = u >> logS, j = u & Smask;
-      const V *src = in + b * a.bstride + j + ((long long)r0 << logS);
-      const long long qs = (long long)TPF << logS;
+      const V *src = in + b * a.bstride + (a.tile_in ? (j & ~3LL) * R + 4 * r0 + (j & 3) : j + ((long long)r0 << logS));
+      const long long qs = (long long)TPF << (a.tile_in ? 2 : logS);
       const long long jm = j & Nsmask;
       const long long mm0 = jm * r0, dmm = jm * TPF;  // twiddle exponents, < Ns * R
       if (a.nsum <= 1) {
