@@ -39,10 +39,13 @@ __global__ void convert_taps_kernel(const double2 *__restrict__ src, void *dst, 
 // First kernel of a run (launched normally, after everything before it):
 // block 0 clears the control block and the row maxima and advances the device
 // epoch (a graph replay of the run advances it too); every block zeroes part
-// of the residue bitmaps F_l.
+// of the residue bitmaps F_l, and of the packed vote tables where this kernel
+// clears them (clear_at_start).
 __global__ void run_begin_kernel(RunCtl *ctl, unsigned long long *rmax, int nrmax, unsigned *epoch,
-                                 unsigned *bm, long long bm_words) {
+                                 unsigned *bm, long long bm_words, uint4 *votes, int vote_quads) {
   pdl_enter();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < vote_quads; i += gridDim.x * blockDim.x)
+    votes[i] = make_uint4(0u, 0u, 0u, 0u);
   if (blockIdx.x == 0) {
     int *c = reinterpret_cast<int *>(ctl);
     for (int i = threadIdx.x; i < (int)(sizeof(RunCtl) / sizeof(int)); i += blockDim.x) c[i] = 0;
@@ -195,7 +198,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
       if (t == GSFFT_ERR_UNSUPPORTED && tc_asked) t = fft_plan_shape(P->fftB, p.B, FFT_FP32_TC);
     }
     P->tc_bucket = t == GSFFT_OK;
-    if (!P->tc_bucket) s = fft_plan_shape(P->fftB, p.B, kind, tn.bucket_first_radix);
+    if (!P->tc_bucket) s = fft_plan_shape(P->fftB, p.B, kind, tn.bucket_first_radix, true);
   }
   if (s == GSFFT_OK) {
     // the RLFC transform reads the streaming pass's sub-samples; its first
@@ -205,7 +208,7 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     if (precision == GSFFT_MIXED && (flags & GSFFT_FLAG_TC_RLFC_FFT) && P->use_stream)
       t = fft_plan_shape(P->fftW, p.W_RLFC, FFT_FP32_TC);
     P->tc_rlfc = t == GSFFT_OK;
-    if (!P->tc_rlfc) s = fft_plan_shape(P->fftW, p.W_RLFC, kind, tn.rlfc_first_radix);
+    if (!P->tc_rlfc) s = fft_plan_shape(P->fftW, p.W_RLFC, kind, tn.rlfc_first_radix, true);
     // the ordered pass writes whole sectors of the sub-samples where the FFT reads them so
     const int nbW = nb < p.W_RLFC ? nb : p.W_RLFC;
     int lognc = 0;
@@ -226,8 +229,13 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   // record the shapes in use
   P->tuning.perm_filter_form = P->use_stream ? 1 : 2;
   P->tuning.row_groups = P->use_stream ? P->groups : 0;
-  P->tuning.bucket_first_radix = P->fftB.npass == 2 && !P->tc_bucket ? P->fftB.logR[0] : 0;
-  P->tuning.rlfc_first_radix = P->fftW.npass == 2 && !P->tc_rlfc ? P->fftW.logR[0] : 0;
+  // (a transform that fits one pass has no first radix to choose, also where a plan
+  // spreads it over two)
+  auto first_radix = [&](const FftPlan &f, bool tc) {
+    return f.npass == 2 && !tc && f.L > (precision == GSFFT_FP64 ? 13 : 14) ? f.logR[0] : 0;
+  };
+  P->tuning.bucket_first_radix = first_radix(P->fftB, P->tc_bucket);
+  P->tuning.rlfc_first_radix = first_radix(P->fftW, P->tc_rlfc);
   P->tuning.select_form = tn.select_form == 2 ? 2 : 1;
   if (s == GSFFT_OK &&
       (cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -324,6 +332,16 @@ int plan_epoch_advance(Plan *P, cudaStream_t st) {
   return GSFFT_OK;
 }
 
+// The packed vote tables of a small signal (two of n / 4 bytes) are cleared by the
+// run's first kernel; from 2^21 points on the next run's table is cleared on the
+// auxiliary stream beside the estimation (8 us at n = 2^27).  That costs a launch,
+// two event records and three waits: n = 2^14 runs are bound by such calls.
+static bool clear_at_start(const Plan *P) { return P->packed_vote && P->p.n <= (1 << 20); }
+// The bucket FFT of the estimation loops' rows: in one launch with the location
+// loops' where all rows are a part of the chip's threads (2^17 points), else later,
+// beside the voting.  n = 2^20, 7 rows of 2^13: it ended 8 us after the voting.
+static bool all_rows_at_once(const Plan *P) { return (long long)P->p.loops * P->p.B <= (1 << 17); }
+
 int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int *ai,
              cudaStream_t st, bool capturing, int phases) {
   if (!P->filter_set) return GSFFT_ERR_STATE;
@@ -353,9 +371,10 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   if (phases & PH_FRONT) {
     // about eight bitmap words per thread, at most 128 CTAs
     const long long bm_words = (long long)(p.W_RLFC / 32) * p.loops_loc;
-    const int grid = (int)std::min<long long>(128, std::max<long long>(1, (bm_words + 2047) / 2048));
+    const int quads = clear_at_start(P) ? p.n / 32 : 0;  // both packed tables
+    const int grid = (int)std::min<long long>(128, std::max<long long>(1, (bm_words + quads + 2047) / 2048));
     run_begin_kernel<<<grid, 256, 0, st>>>(P->ctl, (unsigned long long *)P->rmax, p.RLFC_loops + p.loops,
-                                           P->d_epoch, P->bm_sig, bm_words);
+                                           P->d_epoch, P->bm_sig, bm_words, (uint4 *)P->vote, quads);
     GS_LAUNCHED();
     if (phases != PH_ALL) {
       // a phased run (batch tail): the tail reads this run's draws from the device
@@ -428,7 +447,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
       else
         src = P->bpart;
     }
-    GS_CHECK(fft_exec(P->fftB, src, P->bins, p.loops_loc, -1, io, P->side));
+    GS_CHECK(fft_exec(P->fftB, src, P->bins, all_rows_at_once(P) ? p.loops : p.loops_loc, -1, io, P->side));
     bsrc = src;
   }
   END_ON(ST_BUCKET_FFT, P->side);
@@ -466,16 +485,16 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   // the estimation loops' bucket FFT (side stream), queued behind the RLFC
   // cutoff: that cutoff is a cooperative launch whose whole grid must be
   // resident, so the FFT's blocks would hold back its start
-  GS_CUDA(cudaEventRecord(P->ev_rsel, st));
-  GS_CUDA(cudaStreamWaitEvent(P->side, P->ev_rsel, 0));
-  if (p.loops > p.loops_loc) {
+  if (p.loops > p.loops_loc && !all_rows_at_once(P)) {
+    GS_CUDA(cudaEventRecord(P->ev_rsel, st));
+    GS_CUDA(cudaStreamWaitEvent(P->side, P->ev_rsel, 0));
     FftIo io;  // complex bins only: the estimation reads no samples
     io.err = &P->ctl->err;
     const size_t off = (size_t)(P->precision == GSFFT_FP64 ? 16 : 8) * p.loops_loc * p.B;
     GS_CHECK(fft_exec(P->fftB, (const char *)bsrc + off, (char *)P->bins + off, p.loops - p.loops_loc, -1,
                       io, P->side));
+    GS_CUDA(cudaEventRecord(P->ev_bins, P->side));
   }
-  GS_CUDA(cudaEventRecord(P->ev_bins, P->side));
   BEGIN(ST_J2);
   // F_l needs only the set of J2 ids, not the sorted list; the sorted J2
   // (num_RLFC ids) is compacted on demand by plan_debug
@@ -490,7 +509,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   // outside it); a capture needs no wait either, its replays following one
   // another on a stream.
   GS_CUDA(cudaStreamWaitEvent(st, P->ev_join, 0));
-  if (P->packed_vote && !capturing && P->vclr_eager) GS_CUDA(cudaStreamWaitEvent(st, P->ev_vclr, 0));
+  if (P->packed_vote && !clear_at_start(P) && !capturing && P->vclr_eager) GS_CUDA(cudaStreamWaitEvent(st, P->ev_vclr, 0));
   }  // front
 
   if (phases & PH_VOTE) {
@@ -506,7 +525,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   }  // voting
 
   if (phases & PH_EST) {
-  if (P->packed_vote) {
+  if (P->packed_vote && !clear_at_start(P)) {
     // the voting is done: clear the other packed table for the next run,
     // beside this run's estimation and top-k
     GS_CUDA(cudaEventRecord(P->ev_voted, st));
@@ -516,7 +535,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
     P->vclr_eager = !capturing;
   }
   // A8: estimation (after the estimation loops' bucket FFT); A9: k largest
-  GS_CUDA(cudaStreamWaitEvent(st, P->ev_bins, 0));
+  if (p.loops > p.loops_loc && !all_rows_at_once(P)) GS_CUDA(cudaStreamWaitEvent(st, P->ev_bins, 0));
   BEGIN(ST_ESTIMATE);
   // the grid covers 8k candidates at one per thread (about 4.8k at the
   // 2^27 / 16000 workload); more are taken by the grid-stride loop
@@ -536,7 +555,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
   END(ST_TOPK);
   // the clear of the next run's vote table (queued after the voting) joins the
   // run here; it has long finished beside the estimation and top-k
-  if (P->packed_vote && (phases & PH_EST)) GS_CUDA(cudaStreamWaitEvent(st, P->ev_vclr, 0));
+  if (P->packed_vote && !clear_at_start(P) && (phases & PH_EST)) GS_CUDA(cudaStreamWaitEvent(st, P->ev_vclr, 0));
   }  // top-k
 #undef BEGIN
 #undef END

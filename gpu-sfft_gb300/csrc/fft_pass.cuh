@@ -57,7 +57,7 @@ struct PassArgs {
 // Launch one pass of radix 2^logr (each covers the radices listed).
 int fft_pass_f32_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 5..10
 int fft_pass_f32_hi(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 11..14
-int fft_pass_f64_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 7..10
+int fft_pass_f64_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 6..10
 int fft_pass_f64_hi(int logr, const PassArgs &a, long long total_sub, cudaStream_t st);  // 11..13
 
 namespace {
@@ -115,7 +115,7 @@ __host__ __device__ constexpr int imax(int a, int b) { return a > b ? a : b; }
 // sub-transforms per CTA
 template <typename T> __host__ __device__ constexpr int g_of(int logr);
 template <> __host__ __device__ constexpr int g_of<double>(int logr) {
-  return logr >= 13 ? 1 : imax(2, 2048 >> logr);
+  return logr >= 13 ? 1 : imin(16, imax(2, 2048 >> logr));
 }
 template <> __host__ __device__ constexpr int g_of<float>(int logr) {
   return logr >= 14 ? 1 : (logr == 13 ? 2 : imax(4, 4096 >> logr));

@@ -5,6 +5,7 @@ namespace gsfft {
 
 int fft_pass_f64_lo(int logr, const PassArgs &a, long long total_sub, cudaStream_t st) {
   switch (logr) {
+    case 6: return launch_fx<6>(a, total_sub, st);
     case 7: return launch_fx<7>(a, total_sub, st);
     case 8: return launch_fx<8>(a, total_sub, st);
     case 9: return launch_fx<9>(a, total_sub, st);

@@ -326,8 +326,9 @@ struct FftIo {
 enum FftKind { FFT_FP64, FFT_FP32, FFT_FP32_TC, FFT_FP32_TC64 };
 // A plan in three steps, so that its tables and scratch (max_batch transforms) can
 // share an allocation: its passes (first_logr: log2 of the first pass's radix for
-// two-pass sizes of the first two kinds, 0: ceil(L/2)), its buffers, the tables.
-int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr = 0);
+// two-pass sizes of the first two kinds, 0: ceil(L/2); spread: FP64 transforms of 2^12 and
+// 2^13 in two passes on several CTAs a row, for few rows), its buffers, the tables.
+int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr = 0, bool spread = false);
 void fft_plan_request(FftPlan &p, int max_batch, Arena &mem);
 int fft_plan_fill(const FftPlan &p, cudaStream_t st);
 // The three steps with an allocation of its own; tables are built on st, the
