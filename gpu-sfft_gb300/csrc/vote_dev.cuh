@@ -65,7 +65,8 @@ struct WalkArgs {
 // with word atomics, since neighbouring locations share a word.  There are
 // two packed tables, the run with epoch e using table e & 1; after a run's
 // voting the other one is cleared for the next run (vote_clear_kernel), so
-// the clear overlaps the run's latency-bound tail.
+// the clear overlaps the run's latency-bound tail; for small n the run's first
+// kernel clears both.
 __device__ __forceinline__ unsigned *packed_table(const WalkArgs &w, unsigned *vote, unsigned epoch) {
   return vote + ((epoch & 1u) ? ((unsigned)w.n >> 4) : 0u);
 }
