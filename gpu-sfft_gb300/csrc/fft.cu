@@ -221,9 +221,11 @@ bool fft_reads_row_blocks(const FftPlan &p, int lognc) {
 // sector every N/R points (its loads were a third of its time: L1 lines, not DRAM),
 // and the first writes lines, not half ones.  Second pass of two rows of 2^24:
 // 221 -> 185 us.
+// FP64 (pairs of sub-transforms, radices 2^10 .. 2^12): the same with 2 for 4; two rows
+// of 2^22 in gsfft_fft 467 -> 446 us, the n = 2^27 step 885 -> 871.
 static bool fft_tiled(const FftPlan &p) {
-  return p.npass == 2 && p.precision != GSFFT_FP64 && !p.tc[0] && !p.tc[1] && (p.logR[0] == 11 || p.logR[0] == 12) &&
-         p.logR[1] >= 10 && p.logR[1] <= 12;
+  if (p.npass != 2 || p.tc[0] || p.tc[1]) return false;
+  return p.logR[0] >= (p.precision == GSFFT_FP64 ? 10 : 11) && p.logR[0] <= 12 && p.logR[1] >= 10 && p.logR[1] <= 12;
 }
 
 int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,

@@ -46,7 +46,7 @@ struct PassArgs {
   int nsum;           // first pass: add nsum partial inputs sstride apart
   long long sstride;
   int lognc;          // first pass: FftIo::in_lognc, or -1
-  int tile_in, tile_out;  // the array between two passes in tiles of four sub-transforms (fft_tiled)
+  int tile_in, tile_out;  // the array between two passes in tiles of four (FP64: two) sub-transforms (fft_tiled)
   int write_complex;
   // FP64 passes: fixed-point twiddles -- the radix-16 stages' tables, and the
   // two-level table of exp(-2 pi i m / Np)

@@ -123,7 +123,8 @@ __device__ __noinline__ void fx_fallback(const PassArgs &a, double2 *sm) {
   for (int q = 0; q < ITER; q++) {
     const int lt = threadIdx.x + q * NT;
     const int g = gf_in ? lt % G : lt / R, r = gf_in ? lt / G : lt % R;
-    const long long u = u0 + g, b = u >> logS, j = u & Smask, m = j + ((long long)r << logS);
+    const long long u = u0 + g, b = u >> logS, j = u & Smask,
+                    m = a.tile_in ? (j & ~1LL) * R + 2 * r + (j & 1) : j + ((long long)r << logS);
     double2 v = make_double2(0.0, 0.0);
     if (u < a.total) v = gx ? gx[a.goffs[b] + m * a.gstride] : in[b * a.bstride + m];
     if (a.inverse) v.y = -v.y;
@@ -141,7 +142,9 @@ __device__ __noinline__ void fx_fallback(const PassArgs &a, double2 *sm) {
     const int g = gf_out ? lt % G : lt / R, k = gf_out ? lt / G : lt % R;
     const long long u = u0 + g, b = u >> logS, j = u & Smask;
     if (u >= a.total) continue;
-    const long long d = b * a.bstride + ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask) + ((long long)k << logNs);
+    const long long d =
+        b * a.bstride + (a.tile_out ? ((long long)(k & ~1) << logS) + 2 * j + (k & 1)
+                                    : ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask) + ((long long)k << logNs));
     double2 v = sm[g * RP + padded(k)];
     if (a.inverse) v.y = -v.y;
     if (a.write_complex) reinterpret_cast<double2 *>(a.out)[d] = v;
@@ -238,7 +241,8 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
       src = reinterpret_cast<const double2 *>(a.gx) + (live ? a.goffs[b] + j * a.gstride : 0);
       step *= a.gstride;
     } else {
-      src = reinterpret_cast<const double2 *>(a.in) + b * a.bstride + j;
+      src = reinterpret_cast<const double2 *>(a.in) + b * a.bstride + (a.tile_in ? (j & ~1LL) * R + (j & 1) : j);
+      if (a.tile_in) step = 2;
     }
     double2 d[16];
 #pragma unroll
@@ -333,7 +337,7 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
 
   // last stage: outputs t + e R/16 straight to global memory, adjacent lanes on
   // adjacent sub-transforms when Ns >= G, else on consecutive outputs
-  const bool gf = (1LL << logNs) >= G;
+  const bool gf = a.tile_out || (1LL << logNs) >= G;
   const int g = gf ? tid % G : tid / TPF, t = gf ? tid / G : tid % TPF;
   const long long u = u0 + g, b = u >> logS, j = u & Smask;
   const bool live = u < a.total;
@@ -344,8 +348,9 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
   fx::C64 v[16];
   fx_radix16<LOGR, LOGR - 4>(v, sm + g * fx_pitch<LOGR>() + padx(t), tw, t, 1u << fx_spare(bits[NST - 1][g]),
                                a.one);
-  const long long d0 = b * a.bstride + ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask) + ((long long)t << logNs);
-  const long long ds = (long long)(R / 16) << logNs;
+  const long long d0 = b * a.bstride + (a.tile_out ? ((long long)(t & ~1) << logS) + 2 * j + (t & 1)
+                                                   : ((j >> logNs) << (logNs + LOGR)) + (j & Nsmask) + ((long long)t << logNs));
+  const long long ds = (long long)(R / 16) << (a.tile_out ? logS : logNs);
   double tmax = 0.0;
   if (live) {
     double2 *out = reinterpret_cast<double2 *>(a.out) + d0;
