@@ -145,13 +145,11 @@ template <typename T> __host__ __device__ constexpr int rowpitch(int logr) {
 template <typename T> __host__ __device__ constexpr int data_smem_of(int logr) {
   return g_of<T>(logr) * rowpitch<T>(logr) * (int)sizeof(typename Cx<T>::V);
 }
-// FP32: the twiddle table exp(-2 pi i m / R) is copied into shared memory when it fits
-__host__ __device__ constexpr bool tw_in_smem(int logr) {
-  return data_smem_of<float>(logr) + (1 << logr) * (int)sizeof(float2) <= 220 * 1024;
-}
-__host__ __device__ constexpr int smem_of(int logr) {
-  return data_smem_of<float>(logr) + (tw_in_smem(logr) ? (1 << logr) * (int)sizeof(float2) : 0);
-}
+// FP32: the first quarter of the twiddle table exp(-2 pi i m / R) in shared memory: a
+// radix-16 stage after Ns reads k R / (16 Ns) and four times that, k < Ns, and the
+// first stage (any radix) reads none
+__host__ __device__ constexpr int tw_offset(int logr) { return (data_smem_of<float>(logr) + 15) & ~15; }
+__host__ __device__ constexpr int smem_of(int logr) { return tw_offset(logr) + (1 << logr) / 4 * (int)sizeof(float2); }
 
 // Inter-pass twiddles folded into the first shared-memory stage (passes
 // after the first): the stage's inputs are conjugated (inverse) and
@@ -574,11 +572,14 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
   extern __shared__ __align__(16) unsigned char smraw[];
   V *sm = reinterpret_cast<V *>(smraw);
   const V *twR = reinterpret_cast<const V *>(a.twR);
-  if (tw_in_smem(LOGR)) {
-    V *tws = reinterpret_cast<V *>(smraw + data_smem_of<T>(LOGR));
-    for (int i = threadIdx.x; i < R; i += NT) tws[i] = twR[i];
-    twR = tws;  // made visible by the barrier before the first butterfly stage
-  }
+  // The twiddles land beside the pass's own loads, which waited for a copy through
+  // registers before (n = 2^27 steps: k = 16000 381 -> 373 us, k = 43000 856 -> 826).
+  V *tws = reinterpret_cast<V *>(smraw + tw_offset(LOGR));
+  for (int i = threadIdx.x; i < R / 8; i += NT)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(tws + 2 * i)),
+                 "l"(twR + 2 * i)
+                 : "memory");
+  twR = tws;  // made visible by the barrier before the first butterfly stage
   const V *__restrict__ in = reinterpret_cast<const V *>(a.in);
   const V *__restrict__ gx = reinterpret_cast<const V *>(a.gx);
   const V *__restrict__ thi = reinterpret_cast<const V *>(a.tw_hi);
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       PreTw ptf = pt;  // inter-pass twiddles in registers wherever Ns > 1
       ptf.on = logNs > 0;
       fused_first_stage<V, LOGR, G>(sm, in + b * a.bstride, j, logS, a.lognc, a.tile_in, ptf, a.inverse);
+      asm volatile("cp.async.wait_all;" ::: "memory");  // the twiddles
       __syncthreads();
       fused_mid_stages<V, LOGR, G, (LOGR % 4 == 0 ? 4 : LOGR % 4)>(sm, twR, pt);
       const long long d0 =
@@ -773,6 +775,7 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       }
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // the twiddles
   __syncthreads();
   if constexpr (LOGR <= 9) rt_cta_fft<V, LOGR, G, NT>(sm, twR);
   else cta_fft<V, LOGR, G>(sm, twR, pt);
