@@ -213,7 +213,9 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
     const int nbW = nb < p.W_RLFC ? nb : p.W_RLFC;
     int lognc = 0;
     while (((long long)nbW << lognc) < p.W_RLFC) lognc++;
-    P->y_lognc = P->use_stream && fft_reads_row_blocks(P->fftW, lognc) ? lognc : -1;
+    // (pairs of rows from the columns form; the FP64 stream keeps its order)
+    const bool blocks = precision == GSFFT_FP64 ? P->use_cols : P->use_stream;
+    P->y_lognc = blocks && fft_reads_row_blocks(P->fftW, lognc) ? lognc : -1;
   }
   if (s == GSFFT_OK) {
     fft_plan_request(P->fftB, p.loops, mem);
@@ -419,7 +421,7 @@ int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int 
                                        P->groups, P->y_lognc >= 0 ? 2 : 0));
   else if (P->use_cols)
     GS_CHECK(launch_perm_filter_cols(d_x, p.n, P->filt_bm, P->filt, p.w, p.B, p.loops, d, P->bins, p.RLFC_loops,
-                                     P->ybuf, p.W_RLFC, quirk, st));
+                                     P->ybuf, p.W_RLFC, quirk, st, P->y_lognc >= 0 ? 1 : 0));
   else
     GS_CHECK(launch_perm_filter(P->precision, d_x, p.n, P->filt, p.w, p.B, p.loops, d, quirk,
                                 P->bins, st));

@@ -207,10 +207,12 @@ void fft_plan_free(FftPlan &p) {
 
 // fused_first_stage (radix 2^11, 2^12): its steps of 128 and 256 in r are whole
 // blocks of rows from 128 rows on, and with no more rows than the radix a block's
-// rows are all read by the one CTA.
+// rows are all read by the one CTA.  FP64 (radix 2^10 .. 2^12, pairs of rows): steps of
+// R/16 and 256, from 32 rows on.
 bool fft_reads_row_blocks(const FftPlan &p, int lognc) {
-  if (p.npass < 2 || p.precision == GSFFT_FP64 || p.tc[0]) return false;
+  if (p.npass < 2 || p.tc[0]) return false;
   const int lr = p.logR[0], lognb = p.L - lognc;
+  if (p.precision == GSFFT_FP64) return lr >= 10 && lr <= 12 && p.L - lr >= 1 && lognb >= 5 && lognb <= lr;
   return (lr == 11 || lr == 12) && p.L - lr >= 2 && lognb >= 7 && lognb <= lr;
 }
 

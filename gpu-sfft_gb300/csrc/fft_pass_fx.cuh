@@ -107,6 +107,14 @@ __device__ __forceinline__ void fx_row_reduce(unsigned m, bool gfast, unsigned *
   }
 }
 
+// address of point m of a first pass's input: in order, or in pairs of rows of 2^lognc
+// columns (FftIo::in_lognc)
+__device__ __forceinline__ long long row_pairs(long long m, int lognc) {
+  if (lognc < 0) return m;
+  const long long row = m >> lognc, c = m & ((1LL << lognc) - 1);
+  return ((row & ~1LL) << lognc) + 2 * c + (row & 1);
+}
+
 // The pass in FP64, for sub-transforms with values outside the fixed-point
 // range: load with inter-pass twiddles, runtime-stride stages, store.
 template <int LOGR>
@@ -124,7 +132,7 @@ __device__ __noinline__ void fx_fallback(const PassArgs &a, double2 *sm) {
     const int lt = threadIdx.x + q * NT;
     const int g = gf_in ? lt % G : lt / R, r = gf_in ? lt / G : lt % R;
     const long long u = u0 + g, b = u >> logS, j = u & Smask,
-                    m = a.tile_in ? (j & ~1LL) * R + 2 * r + (j & 1) : j + ((long long)r << logS);
+                    m = a.tile_in ? (j & ~1LL) * R + 2 * r + (j & 1) : row_pairs(j + ((long long)r << logS), a.lognc);
     double2 v = make_double2(0.0, 0.0);
     if (u < a.total) v = gx ? gx[a.goffs[b] + m * a.gstride] : in[b * a.bstride + m];
     if (a.inverse) v.y = -v.y;
@@ -235,13 +243,17 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
     const int g = gf ? tid % G : tid / TPF, t0 = gf ? tid / G : tid % TPF;
     const long long u = u0 + g, b = u >> logS, j = u & Smask;
     const bool live = u < a.total;
+    // point t0 + r of the thread's sub-transform: src[r step] (row pairs: r steps over
+    // whole pairs, so only the first address differs)
     const double2 *src;
     long long step = 1LL << logS;
+    const long long m0 = j + ((long long)t0 << logS);
     if (a.gx) {
-      src = reinterpret_cast<const double2 *>(a.gx) + (live ? a.goffs[b] + j * a.gstride : 0);
+      src = reinterpret_cast<const double2 *>(a.gx) + (live ? a.goffs[b] + m0 * a.gstride : 0);
       step *= a.gstride;
     } else {
-      src = reinterpret_cast<const double2 *>(a.in) + b * a.bstride + (a.tile_in ? (j & ~1LL) * R + (j & 1) : j);
+      src = reinterpret_cast<const double2 *>(a.in) + b * a.bstride +
+            (a.tile_in ? (j & ~1LL) * R + 2 * t0 + (j & 1) : row_pairs(m0, a.lognc));
       if (a.tile_in) step = 2;
     }
     double2 d[16];
@@ -249,7 +261,7 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
     for (int q = 0; q < Q0; q++)
 #pragma unroll
       for (int e = 0; e < E0; e++)
-        d[q * E0 + e] = live ? src[(t0 + q * TPF + e * NB0) * step] : make_double2(0.0, 0.0);
+        d[q * E0 + e] = live ? src[(q * TPF + e * NB0) * step] : make_double2(0.0, 0.0);
     unsigned mx = 0;
 #pragma unroll
     for (int i = 0; i < 16; i++) {

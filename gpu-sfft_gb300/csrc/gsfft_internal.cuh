@@ -307,7 +307,8 @@ struct FftIo {
   long long sum_stride = 0;
   // first-pass loader alternative (fft_reads_row_blocks): the input is a matrix of
   // 2^in_lognc columns in blocks of four rows, point t = row 2^in_lognc + column at
-  // (row & ~3) 2^in_lognc + 4 column + (row & 3); -1 = in order
+  // (row & ~3) 2^in_lognc + 4 column + (row & 3); FP64 the same with pairs of rows;
+  // -1 = in order
   int in_lognc = -1;
   // epilogue: |X|^2 (same precision) written to samples[b * n + k]
   void *samples = nullptr;

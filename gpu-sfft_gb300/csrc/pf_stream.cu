@@ -425,8 +425,10 @@ pf_tma_kernel(const __grid_constant__ CUtensorMap tmap, const typename Cx<T>::V 
 // owns 32 columns (four lines a row); its warps walk the loops of those columns in
 // ascending row order side by side (a barrier every PC_U hits keeps them together:
 // 482 -> 448 us), and its threads copy the RLFC columns at the same pace, so
-// samples that share a line are read close together.  At n = 2^27 the kernel takes
-// 440 us with the RLFC rows in it and the W-point FFT falls from 392 to 297 us; at
+// samples that share a line are read close together, and stored by pairs of rows
+// where the W-point FFT reads them so (whole sectors: step 860 -> 843 us).  At n =
+// 2^27 the kernel took 440 us with the RLFC rows in order, and the W-point FFT fell
+// from 392 to 297 us; at
 // n = 2^14 .. 2^26 it is faster by itself (27 -> 11, 33 -> 17 at 2^20, 175 -> 107
 // at 2^25, 289 -> 224 us at 2^26), so every FP64 plan whose sizes allow it takes it.
 // Streaming the whole signal through shared memory (pf_tma_kernel) took 489 us at
@@ -439,7 +441,7 @@ constexpr int PC_U = 3;  // hits in flight per thread
 __global__ void __launch_bounds__(512, 2)
 pf_cols_kernel(const double2 *__restrict__ x, const double2 *__restrict__ filt,
                const double2 *__restrict__ qfilt, int logn, int logB, int w, int tiles, int L, Draws d,
-               HitTab ht, double2 *__restrict__ bins, int nrlfc, int logsig,
+               HitTab ht, double2 *__restrict__ bins, int nrlfc, int logsig, int logyr,
                double2 *__restrict__ y, int W, int quirk) {
   pdl_enter();
   __shared__ unsigned S2[MAXL][2 * MAXT];
@@ -469,7 +471,7 @@ pf_cols_kernel(const double2 *__restrict__ x, const double2 *__restrict__ filt,
   const int logcpr = logsig >= 5 ? 0 : 5 - logsig;  // log2 of a loop's columns in the block
   const int steps = max((tiles + PC_U - 1) / PC_U, 1);
   const int total = (nb * nrlfc) << logcpr;
-  const int per = (total + steps - 1) / steps;
+  const int per = ((total + steps - 1) / steps + 1) & ~1;
   const int nthr = 32 * L;
   double re = 0.0, im = 0.0;
   auto accumulate = [&](double2 xv, double2 f) {
@@ -494,13 +496,15 @@ pf_cols_kernel(const double2 *__restrict__ x, const double2 *__restrict__ filt,
     }
     const int e1 = min((st + 1) * per, total);
     for (int e = st * per + tid; e < e1; e += nthr) {
-      const int ci = e & ((1 << logcpr) - 1), q = e >> logcpr;
-      const int rr = q % nrlfc, row = q / nrlfc;
+      // logyr = 1: two rows of a column side by side, whole 32-byte sectors of y
+      const int ci = (e >> logyr) & ((1 << logcpr) - 1), q = e >> (logcpr + logyr);
+      const int rr = q % nrlfc, row = (q / nrlfc << logyr) + (e & logyr);
       const unsigned off = (unsigned)d.offs[rr];
       const unsigned cc = ((off - blockIdx.x * 32u) & ((1u << logsig) - 1u)) + ((unsigned)ci << logsig);
       if (cc < 32u) {
         const unsigned t = ((unsigned)row << logB) + blockIdx.x * 32u + cc;
-        y[(size_t)rr * W + ((t - off) >> logsig)] = __ldg(x + t);
+        const unsigned col = (blockIdx.x * 32u + cc - off) >> logsig;
+        y[(size_t)rr * W + (((((unsigned)row >> logyr) << (logB - logsig)) + col) << logyr) + (e & logyr)] = __ldg(x + t);
       }
     }
 #pragma unroll
@@ -709,13 +713,13 @@ static void hit_table(int n, int B, int tiles, int loops, const Draws &d, HitTab
 }
 
 int launch_perm_filter_cols(const void *x, int n, const void *filt, const void *qfilt, int w, int B, int loops,
-                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st) {
+                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st, int logyr) {
   if (!stream_pf_supported(n, B, loops, W, nrlfc) || w / B >= MAXT) return GSFFT_ERR_UNSUPPORTED;
   HitTab ht;
   hit_table(n, B, w / B, loops, d, ht);
   GS_CUDA(launch_pdl(pf_cols_kernel, dim3(B / 32), dim3(32 * loops), 0, st, (const double2 *)x,
                      (const double2 *)filt, (const double2 *)qfilt, ilog2(n), ilog2(B), w, w / B, loops, d, ht,
-                     (double2 *)bins, nrlfc, ilog2(n / W), (double2 *)y, W, quirk ? 1 : 0));
+                     (double2 *)bins, nrlfc, ilog2(n / W), logyr, (double2 *)y, W, quirk ? 1 : 0));
   GS_LAUNCHED();
   return GSFFT_OK;
 }

@@ -60,7 +60,7 @@ int launch_perm_filter_stream(int precision, const void *x, int n, const void *f
 // (filt: the bucket-major table; qfilt: the taps in bucket order, for the residue
 // quirk; y as above).
 int launch_perm_filter_cols(const void *x, int n, const void *filt, const void *qfilt, int w, int B, int loops,
-                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st);
+                            const Draws &d, void *bins, int nrlfc, void *y, int W, bool quirk, cudaStream_t st, int logyr = 0);
 // whether `groups` row groups suit the streaming pass at this shape (one, or
 // a power of two leaving at least four tiles of rows per group)
 bool stream_pf_groups_valid(int n, int B, int groups, int precision);

@@ -19,6 +19,11 @@ CFGS = [  # (q, k, Bcst, loops_loc, loops_thresh, loops_est, RLFC_cst, RLFC_loop
     ((18, 100, 1.0, 2, 2, 5, 32, 2), 0.6),    # w < B: no full tile
     ((18, 100, 1.9, 2, 2, 5, 32, 2), 0.4),    # one full tile
     ((22, 777, 0.93, 2, 2, 7, 512, 2), 1e-8),
+    # RLFC rows in pairs (first radix 2^10, 2^11, 2^12)
+    ((20, 500, 1.0, 2, 2, 5, 2048, 2), 1e-8),
+    ((22, 777, 0.93, 2, 2, 7, 4096, 2), 1e-8),
+    ((23, 2000, 0.93, 2, 2, 7, 4096, 3), 1e-8),
+    ((24, 1000, 2.5, 2, 2, 5, 16384, 2), 1e-8),
 ]
 
 
