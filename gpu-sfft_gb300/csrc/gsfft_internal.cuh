@@ -166,15 +166,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar_smem_addr, unsigned p
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool mbar_test(unsigned bar_smem_addr, unsigned parity) {
-  unsigned done;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(done)
-      : "r"(bar_smem_addr), "r"(parity)
-      : "memory");
-  return done != 0;
-}
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned bar_smem_addr, unsigned parity,
                                                   long long limit = kWaitLimitCycles) {
   if (mbar_try_wait(bar_smem_addr, parity)) return true;  // no clock read when it is done
