@@ -74,7 +74,8 @@ int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr, bool s
   if (n < 256 || (n & (n - 1)) != 0) return GSFFT_ERR_UNSUPPORTED;
   int L = 0;
   while ((1LL << L) < n) L++;
-  const int one_pass_max = kind == FFT_FP64 ? 13 : 14;
+  const bool dbl = kind == FFT_FP64 || kind == FFT_FP64_DIRECT;
+  const int one_pass_max = dbl ? 13 : 14;
   int r[3] = {0, 0, 0}, npass = 0;
   if (kind == FFT_FP32_TC) {
     // the second pass is a CUDA-core pass of radix 2^(L-12)
@@ -119,12 +120,13 @@ int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr, bool s
   } else {
     return GSFFT_ERR_UNSUPPORTED;
   }
-  if (kind == FFT_FP64 || kind == FFT_FP32)
+  if (dbl || kind == FFT_FP32)
     for (int i = 0; i < npass; i++)
       if (r[i] < (spread ? 6 : 7) || r[i] > one_pass_max) return GSFFT_ERR_UNSUPPORTED;
   p.n = n;
   p.L = L;
-  p.precision = kind == FFT_FP64 ? GSFFT_FP64 : GSFFT_MIXED;
+  p.precision = dbl ? GSFFT_FP64 : GSFFT_MIXED;
+  p.direct = kind == FFT_FP64_DIRECT;
   p.npass = npass;
   int lg = 0;
   for (int i = 0; i < npass; i++) {
@@ -145,7 +147,7 @@ void fft_plan_request(FftPlan &p, int max_batch, Arena &mem) {
     mem.add(&p.tw_lo[i], es * nlo);
     mem.add(&p.tw_hi[i], es * nhi);
     mem.add(&p.tw_R[i], es << p.logR[i]);
-    if (dbl) {
+    if (dbl && !p.direct) {
       mem.add(&p.fx_tw[i], sizeof(fx::Tw) * fx_stage_entries(p.logR[i]));
       mem.add(&p.fx_hi[i], sizeof(longlong2) * nhi);
       mem.add(&p.fx_lo[i], sizeof(fx::Tw) * nlo);
@@ -174,7 +176,7 @@ int fft_plan_fill(const FftPlan &p, cudaStream_t st) {
     add(p.tw_lo[i], kind, nlo, lg, 0, 0);
     add(p.tw_hi[i], kind, nhi, lg, h, 0);
     add(p.tw_R[i], kind, 1 << p.logR[i], p.logR[i], 0, 0);
-    if (dbl) {
+    if (dbl && !p.direct) {
       add(p.fx_tw[i], TAB_FX_STAGES, fx_stage_entries(p.logR[i]), 0, 0, p.logR[i]);
       add(p.fx_hi[i], TAB_FX_HI, nhi, lg, h, 0);
       add(p.fx_lo[i], TAB_FX_LO, nlo, lg, 0, 0);
@@ -272,6 +274,7 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
     a.fx_hi = p.fx_hi[i];
     a.fx_lo = p.fx_lo[i];
     a.one = 1;
+    a.direct = p.direct ? 1 : 0;
     a.gx = (i == 0) ? io.gather_x : nullptr;
     for (int q = 0; q < 8; q++) a.goffs[q] = io.gather_offsets[q];
     a.gstride = io.gather_stride;

@@ -52,6 +52,7 @@ struct PassArgs {
   // two-level table of exp(-2 pi i m / Np)
   const void *fx_tw, *fx_hi, *fx_lo;
   int one;  // 1, as a value that the compiler does not see (fix64.cuh)
+  int direct;  // FP64 arithmetic for every sub-transform (no fixed-point twiddles)
 };
 
 // Launch one pass of radix 2^logr (each covers the radices listed).

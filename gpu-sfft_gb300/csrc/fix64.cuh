@@ -80,12 +80,6 @@ FX_FN C64 cmul(C64 x, Tw w, int one) {
   return C64{madw(nyh, w.z, madw(xh, w.x, top64(tr, one))), madw(yh, w.x, madw(xh, w.z, top64(ti, one)))};
 }
 
-// v m 2^-64, rounded, m = mh 2^32 + ml real, |m| <= 2^62
-FX_FN long long mul_limbs(long long v, int mh, int ml, int one) {
-  const int h = limb_hi(v), l = limb_lo(v);
-  return madw(h, mh, top64(madw(l, mh, mulw(h, ml)), one));
-}
-
 FX_FN Tw limbs(C64 w) { return Tw{limb_hi(w.x), limb_lo(w.x), limb_hi(w.y), limb_lo(w.y)}; }
 
 // product of two twiddle factors scaled by 2^62, again scaled by 2^62

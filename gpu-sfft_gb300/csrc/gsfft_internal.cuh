@@ -246,7 +246,8 @@ struct FftPlan {
   void *tw_lo[3] = {nullptr, nullptr, nullptr};
   int tw_h[3] = {0, 0, 0};
   void *tw_R[3] = {nullptr, nullptr, nullptr};  // exp(-2 pi i m / R) for the pass radix
-  // FP64: fixed-point twiddles of the pass (fft_pass_fx.cuh)
+  bool direct = false;     // FFT_FP64_DIRECT
+  // FP64, not direct: fixed-point twiddles of the pass (fft_pass_fx.cuh)
   void *fx_tw[3] = {nullptr, nullptr, nullptr};
   void *fx_hi[3] = {nullptr, nullptr, nullptr};
   void *fx_lo[3] = {nullptr, nullptr, nullptr};
@@ -311,14 +312,15 @@ struct FftIo {
   int *err = nullptr;
 };
 
-// Kinds of plan: FP64 or FP32 on the integer / CUDA cores; FP32 with a radix-4096
+// Kinds of plan: FP64 on the integer pipes or (_DIRECT) in FP64 arithmetic throughout;
+// FP32 on the CUDA cores; FP32 with a radix-4096
 // tensor-core pass, then a CUDA-core pass of radix n / 4096 (n = 2^(17..26)); FP32
 // with a CUDA-core radix-2^(L-6) first pass, then a tensor-core radix-64 last pass
 // (13 <= L <= 20).  GSFFT_ERR_UNSUPPORTED for other sizes.
-enum FftKind { FFT_FP64, FFT_FP32, FFT_FP32_TC, FFT_FP32_TC64 };
+enum FftKind { FFT_FP64, FFT_FP64_DIRECT, FFT_FP32, FFT_FP32_TC, FFT_FP32_TC64 };
 // A plan in three steps, so that its tables and scratch (max_batch transforms) can
 // share an allocation: its passes (first_logr: log2 of the first pass's radix for
-// two-pass sizes of the first two kinds, 0: ceil(L/2); spread: FP64 transforms of 2^12 and
+// two-pass sizes of the kinds without tensor cores, 0: ceil(L/2); spread: FP64 transforms of 2^12 and
 // 2^13 in two passes on several CTAs a row, for few rows), its buffers, the tables.
 int fft_plan_shape(FftPlan &p, long long n, FftKind kind, int first_logr = 0, bool spread = false);
 void fft_plan_request(FftPlan &p, int max_batch, Arena &mem);
