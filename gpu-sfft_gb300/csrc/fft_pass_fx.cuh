@@ -21,6 +21,19 @@
 // per pass (relative L2: noise, impulses, tones; 2e-16 where the samples spread
 // over e^+-40), the FP64 pass 1e-16 to 3e-16.
 //
+// Small samples beside large ones: a double keeps its 53 bits wherever it lies, a
+// fixed-point value those above 2^-58 .. 2^-62 of the row's largest.  Where samples share
+// one scale that is no loss (FP64 additions round at 2^-53 of the larger value), but
+// where large samples cancel exactly it is, ones and 1e-20-sized samples in turn for
+// instance.  So each thread adds up how many binades beyond FX_NEAR its 16 samples lie below
+// the row's largest; above FX_FAR in any thread the CTA takes fx_fallback.  A
+// single sample may lie 2^-36 below, four 2^-21, sixteen 2^-17 on average (41 bits and
+// more are kept).  The chance halves with every unit: on normally distributed samples
+// (real or complex) it is below 1e-10 a thread; two tones that beat slowly in a row
+// hold many small samples in a thread (FX_NEAR 8, FX_FAR 28 sent 2 or 3 CTAs of a
+// noiseless n = 2^24, k = 4000 run to the other form, 350 -> 390 us).  The check costs 2.5 % of the
+// passes (the two of two 2^22-point rows 285 -> 293 us).
+//
 // Sub-transforms whose largest sample lies outside 2^-800 .. 2^970 (2^+-250 in a
 // pass that writes |X|^2; infinities, NaN and subnormals among them) are
 // transformed in FP64 by fx_fallback, as every pass was; the filter design asks for
@@ -55,6 +68,7 @@ constexpr int FX_MAXST = 3;  // radix-16 stages after the first, at most
 
 // exponent fields of the largest sample that the fixed-point form takes: every
 // non-zero output (at least 2^-960) and every |X|^2 is then a normal double
+constexpr int FX_NEAR = 16, FX_FAR = 20;  // binades
 constexpr int FX_EXP_MIN = 223, FX_EXP_MAX = 1993, FX_EXP_MIN_SQ = 1023 - 250, FX_EXP_MAX_SQ = 1023 + 250;
 
 __device__ __forceinline__ long long fx_lift(long long v, unsigned m) {
@@ -259,6 +273,7 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
   if (tid < G) emax[tid] = 0u;
   if (tid < 16 * FX_MAXST) bits[tid / 16][tid % 16] = 0u;
 
+  unsigned far = 0;  // binades that this thread's samples lie far below their row's largest
   int s_in;  // the exponent of the fixed-point values after the first stage, per row
   {
     // adjacent lanes take adjacent sub-transforms (whole 32-byte sectors) when
@@ -317,11 +332,15 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
     const int em = emax[g] >> 20 ? (int)(emax[g] >> 20) : 1023;
     const bool pre = logNs > 0;
     const int c = em + 62 - (pre ? PIN : P);
+    const unsigned near = (unsigned)(em - FX_NEAR - 1);
     fx::C64 v[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-      v[i].x = fx::from_double(d[i].x, c);
-      v[i].y = fx::from_double(d[i].y, c);
+      const int ex = fx::exponent(d[i].x), ey = fx::exponent(d[i].y);
+      // binades below `near`; a zero's exponent field wraps and counts none
+      far += near - min((unsigned)max(ex, ey) - 1u, near);
+      v[i].x = fx::from_double(d[i].x, ex, c);
+      v[i].y = fx::from_double(d[i].y, ey, c);
       if (a.inverse) v[i].y = -v[i].y;
     }
     if (pre) {
@@ -367,7 +386,10 @@ fft_fx_kernel(const __grid_constant__ PassArgs a) {
     fx_row_reduce<G, TPF, false>(m, gf, bits[0], g);
     s_in = -1022 - (pre ? PIN - 2 : P) + 4 * NST;
   }
-  __syncthreads();
+  if (__syncthreads_or(far > (unsigned)FX_FAR)) {
+    fx_fallback<LOGR>(a, reinterpret_cast<double2 *>(smraw));
+    return;
+  }
   const fx::Tw *tw = reinterpret_cast<const fx::Tw *>(a.fx_tw);
   fx_mid_stages<LOGR, LOGE0, 1>(sm, tw, bits, a.one);
 

@@ -181,20 +181,34 @@ template <int E> FX_FN void dft(C64 *v, int one) {
 }
 
 // double -> fixed: d 2^(P - (emax - 1022)) truncated, where emax is the largest
-// exponent field of the block (so the result is below 2^P), c = emax + 62 - P.
+// exponent field of the block (so the result is below 2^P), c = emax + 62 - P; e is
+// d's own exponent field.
 // The 53-bit mantissa at bits 9..61 is shifted right by c - exponent; a zero, a
 // subnormal or a value far below the block's largest shifts out.  On the integer
 // pipes: conversion instructions run at 2.06 a clock and SM, and the pass waited
 // for them (126 -> 142 us).
-FX_FN long long from_double(double d, int c) {
+FX_FN unsigned double_hi(double d) {
 #ifdef __CUDA_ARCH__
-  const unsigned lo = (unsigned)__double2loint(d), hi = (unsigned)__double2hiint(d);
+  return (unsigned)__double2hiint(d);
 #else
   unsigned long long b;
   __builtin_memcpy(&b, &d, 8);
-  const unsigned lo = (unsigned)b, hi = (unsigned)(b >> 32);
+  return (unsigned)(b >> 32);
 #endif
-  const int s = c - (int)((hi >> 20) & 0x7ffu);
+}
+FX_FN unsigned double_lo(double d) {
+#ifdef __CUDA_ARCH__
+  return (unsigned)__double2loint(d);
+#else
+  unsigned long long b;
+  __builtin_memcpy(&b, &d, 8);
+  return (unsigned)b;
+#endif
+}
+FX_FN int exponent(double d) { return (int)((double_hi(d) >> 20) & 0x7ffu); }  // its field
+FX_FN long long from_double(double d, int e, int c) {
+  const unsigned lo = double_lo(d), hi = double_hi(d);
+  const int s = c - e;
   const unsigned long long m = (((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo) << 9;
 #ifdef __CUDA_ARCH__
   unsigned long long v;

@@ -1,11 +1,39 @@
-"""FP64 plans of very small or very large signals (the passes' FP64 form with its gathers,
-row pairs, |X|^2 and row maxima)."""
+"""FP64 transforms of samples on very different scales, and plans of very small or very
+large signals (the passes' FP64 form with its gathers, row pairs, |X|^2 and row maxima)."""
 import numpy as np
 import pytest
 
 from gsfft import synth
 
 pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+
+
+@pytest.mark.parametrize("log2n,batch", [(8, 1), (8, 17), (9, 3), (10, 2), (11, 3), (12, 1), (13, 1), (14, 2), (17, 1), (20, 1)])
+@pytest.mark.parametrize("small", [1e-20, 1e-90, 2.0 ** -24])
+def test_small_samples_beside_large_ones(G, torch_cuda, log2n, batch, small):
+    """Ones at the even positions cancel exactly in all but two outputs; the others are
+    the transform of the small samples at the odd positions, each output within
+    log2(n) roundings of 2^-53 of them (relative L2, both sides)."""
+    torch, n = torch_cuda, 1 << log2n
+    rng = np.random.default_rng(log2n)
+    odd = np.zeros((batch, n), np.complex128)
+    odd[:, 1::2] = rng.standard_normal((batch, n // 2)) + 1j * rng.standard_normal((batch, n // 2))
+    x = odd * small
+    x[:, ::2] = 1.0
+    d = torch.from_numpy(x).cuda()
+    y = torch.empty_like(d)
+    G.fft(d.data_ptr(), y.data_ptr(), n, batch, -1, G.FP64)
+    y = y.cpu().numpy()
+    want = np.fft.fft(odd.astype(np.clongdouble), axis=1)
+    rest = np.ones(n, bool)
+    rest[[0, n // 2]] = False
+    assert np.allclose(y[:, 0], n / 2, rtol=1e-6) and np.allclose(y[:, n // 2], n / 2, rtol=1e-6)
+    e = y[:, rest].astype(np.clongdouble) / np.longdouble(small) - want[:, rest]
+    rel = np.sqrt((np.abs(e) ** 2).sum(1) / (np.abs(want[:, rest]) ** 2).sum(1))
+    assert float(rel.max()) <= 2 * log2n * U
+
 
 CFGS = [  # (configuration, flags by name)
     ((14, 10, 2.5, 2, 2, 5, 16, 2), ()),                      # B = 256: sixteen rows a CTA
