@@ -354,15 +354,23 @@ int select_impl(const void *keys, long long size, const int *size_dev, int num, 
 //   1. a sample of about 2^18 samples a row (whole groups of 128 or 64, spread over the
 //      chunk; short rows are taken whole) is counted by leading digits, and the
 //      lower edge L of the digit that holds about 1.1 num samples above it is
-//      chosen -- or the smallest non-zero sample when that few are non-zero;
+//      chosen -- or the smallest non-zero sample when that few are non-zero; a digit
+//      with more samples than the lists hold is counted again in 2048 parts;
 //   2. every warp lists its samples >= L, in order, in shared memory, and their
 //      next digits are counted;
 //   3. either every non-zero sample is listed and they are at most num: all are
 //      taken, and the first zeros fill the rest; or the digit with the num-th largest
-//      is known, its few samples are exchanged, and each CTA finds the num-th by
-//      rank (key, then index) and writes its own.
-// A guess that proves wrong (a list too small, fewer than num above L, many samples
-// in the last digit) costs time only: sel_passes then does the selection.
+//      is known.  With at most 256 samples in it these are exchanged, and each CTA
+//      finds the num-th by rank (key, then index) and writes its own; with more
+//      the listed samples are counted in finer parts of it, down to one value, whose first
+//      ones by index are taken.  (Ranking up to 768, every pair in every CTA, took more than
+//      20 us, and sel_passes from 769 on 25: the k largest of a noiseless n = 2^26 run, all
+//      of one magnitude, 49 -> 23 us; two uniform rows of 2^22 floats 99 -> 42, of doubles
+//      148 -> 46.)
+// A guess that proves wrong (a list too small, fewer than num above L) costs time
+// only: sel_passes then does the selection.  That is left where one value, or values
+// within a 2^-14 of each other, fill a long row: 0.72 to 0.86 times the speed of
+// sel_passes alone.
 //
 // sel_passes: each radix pass builds the CTA's chunk histogram in shared memory and
 // adds it to the row's global histogram once; after a grid-wide sync every CTA
@@ -538,8 +546,9 @@ template <typename K> __device__ __forceinline__ K row_floor(const CoopArgs &a, 
 }
 
 constexpr int WARPS = CT / 32;
-constexpr int AMB_MAX = 768;   // samples of the deciding digit, at most
-constexpr int LIST_SLOTS = 5;  // row slots of HIST_BINS words that sel_lists uses and clears
+constexpr unsigned AMB_MAX = 256;  // samples of the deciding digit that are ranked, at most
+constexpr int LIST_SLOTS = 5;      // row slots of HIST_BINS words that sel_lists uses and clears
+constexpr int FINER_SLOT = 5;      // one more where it counts finer digits
 // dynamic shared memory: per-warp lists (16-bit offset in the warp's segment, key),
 // a histogram, the exchanged samples
 template <typename K> constexpr int list_cap() { return sizeof(K) == 4 ? 512 : 288; }
@@ -611,7 +620,9 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
   extern __shared__ unsigned wh[];
   ListSmem<K> &sm = *reinterpret_cast<ListSmem<K> *>(wh);
   __shared__ unsigned ws[WARPS], wcnt[WARPS];
-  __shared__ unsigned s_digit, s_need, s_amb;
+  __shared__ unsigned s_digit, s_above, s_bin, s_at;
+  __shared__ unsigned r_need[MAXB], r_amb[MAXB];  // a row's deciding digit: need-th of amb samples
+  __shared__ unsigned weq[WARPS];
   __shared__ K s_key;
   __shared__ int s_idx;
   __shared__ int s_last;
@@ -630,21 +641,42 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
   const int ngroups = (int)((hi - lo + GK - 1) / GK), gpw = (ngroups + WARPS - 1) / WARPS;
   const int g0 = min(wid * gpw, ngroups), g1 = min(g0 + gpw, ngroups);
 
+  auto clear_slots = [&](int r, int part, int parts, int n) {
+    for (int i = part * CT + tid; i < n * HIST_BINS; i += parts * CT) slot(i / HIST_BINS, r)[i % HIST_BINS] = 0;
+  };
+  // leaves the selection to sel_passes, the first n slots zero (all CTAs behind the barrier)
+  auto give_up = [&](int n) {
+    if (solo) {
+      __syncthreads();
+    } else {
+      sync_all<CLU>();  // every CTA has read the row's figures
+      for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++)
+        clear_slots(r, CLU ? ci : blockIdx.x, CLU ? a.cpr : gridDim.x, n);
+      sync_all<CLU>();
+    }
+    return false;
+  };
+
   // 1. the sample
   const int step = sz >> 18 > 1 ? (int)(sz >> 18) : 1;
-  for (int i = tid; i < HIST_BINS; i += CT) sm.hist[i] = 0;
-  __syncthreads();
-  for (int j = wid; j * step < ngroups; j += WARPS) {
-    const int g = j * step + (step > 1 ? (int)((((unsigned)j * 0x9E3779B1u) >> 16) % (unsigned)step) : 0);
-    if (g < ngroups) {
-      K ks[EPQ];
-      load_group<K, VEC>(row, lo + (long long)g * GK + lane * EPQ, hi, ks);
+  auto count_sample = [&](auto &&bin) {  // sm.hist[bin(key)] of the sampled keys; none where bin < 0
+    for (int i = tid; i < HIST_BINS; i += CT) sm.hist[i] = 0;
+    __syncthreads();
+    for (int j = wid; j * step < ngroups; j += WARPS) {
+      const int g = j * step + (step > 1 ? (int)((((unsigned)j * 0x9E3779B1u) >> 16) % (unsigned)step) : 0);
+      if (g < ngroups) {
+        K ks[EPQ];
+        load_group<K, VEC>(row, lo + (long long)g * GK + lane * EPQ, hi, ks);
 #pragma unroll
-      for (int e = 0; e < EPQ; e++)
-        if (ks[e] >= lowest) atomicAdd(&sm.hist[dig.of(ks[e])], 1u);
+        for (int e = 0; e < EPQ; e++) {
+          const int d = ks[e] >= lowest ? bin(ks[e]) : -1;
+          if (d >= 0) atomicAdd(&sm.hist[d], 1u);
+        }
+      }
     }
-  }
-  __syncthreads();
+    __syncthreads();
+  };
+  count_sample([&](K k) { return (int)dig.of(k); });
   auto publish = [&](int p) {  // the histogram to its row's slot
     if (solo) return;
     unsigned *gh = slot(p, b);
@@ -658,27 +690,73 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
   };
   publish(0);
   // the lower edge: the highest digit with at least `want` sampled samples from it up
+  // (`had` of them above the counted range)
   K L = lowest;
   {
     const float mean = (float)a.num / (float)step;
     const unsigned want = step > 1 ? (unsigned)(mean + 5.f * sqrtf(mean) + 8.f) : (unsigned)a.num;
-    const uint4 h = four_bins(0, b);
-    const unsigned hs[4] = {h.x, h.y, h.z, h.w};
-    unsigned tot;
-    unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);  // samples below the bin
-    if (tid == 0) s_digit = 0u;
-    __syncthreads();
-    if (tot >= want) {
+    auto pick = [&](int p, int r, unsigned had) {
+      const uint4 h = four_bins(p, r);
+      const unsigned hs[4] = {h.x, h.y, h.z, h.w};
+      unsigned tot;
+      unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);  // samples below the bin
+      if (tid == 0) s_digit = s_above = s_bin = 0u;
+      __syncthreads();
+      tot += had;
+      if (tot >= want) {
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        // samples from this bin up: tot - from
-        if (tot - from >= want && tot - from - hs[q] < want) s_digit = (unsigned)(4 * tid + q);
-        from += hs[q];
+        for (int q = 0; q < 4; q++) {
+          // samples from this bin up: tot - from
+          if (tot - from >= want && tot - from - hs[q] < want) {
+            s_digit = (unsigned)(4 * tid + q);
+            s_above = tot - from - hs[q];
+            s_bin = hs[q];
+          }
+          from += hs[q];
+        }
       }
+      __syncthreads();
+    };
+    // whether the lists would run over (three quarters of their room: a warp's share varies)
+    auto crowded = [&]() {
+      return (long long)(s_above + s_bin) * step * 4 > (long long)a.cpr * WARPS * CAP * 3;
+    };
+    // Samples that lie together fill a digit -- an octave wide for doubles without a
+    // row maximum: half of a uniform row -- so a crowded one is counted again in 2048
+    // parts.  Decided by all CTAs behind the barrier alike: their one row's figures, or
+    // (octaves) every row's.
+    const bool octaves = sizeof(K) == 8 && !a.row_max;
+    bool finer = false;
+    if (!CLU && octaves)
+      for (int r = 0; r < a.batch; r++) {
+        if (r == b) continue;
+        pick(0, r, 0u);
+        finer |= s_digit > 0 && crowded();
+        __syncthreads();
+      }
+    pick(0, b, 0u);
+    const K edge = dig.edge(s_digit);
+    const unsigned digit0 = s_digit, above = s_above;
+    const bool mine = digit0 > 0 && crowded();
+    if (edge > L) L = edge;
+    finer |= mine && (CLU || octaves || a.batch == 1);
+    if (__builtin_expect(finer, 0)) {
+      const int s1 = dig.shift - 11;
+      __syncthreads();  // the histogram has been read
+      count_sample([&](K k) {
+        if (!mine || dig.of(k) != digit0) return -1;
+        const K t = (k - edge) >> s1;
+        return t < (K)(HIST_BINS - 1) ? (int)t : HIST_BINS - 1;
+      });
+      publish(3);
+      if (mine) {
+        pick(3, b, above);
+        const K e = edge + ((K)s_digit << s1);
+        if (e > L) L = e;
+      }
+      // many samples of one value (known to all only where there is one row)
+      if ((CLU || a.batch == 1) && crowded()) return give_up(LIST_SLOTS);
     }
-    __syncthreads();
-    const K e = dig.edge(s_digit);
-    if (e > L) L = e;
   }
   const bool all_listed = L == lowest;
 
@@ -742,6 +820,7 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
     }
   }
   if (lane == 0) wcnt[wid] = wc;
+  if (tid < MAXB) r_amb[tid] = 0u;
   __syncthreads();  // lists and the cleared histogram
   const int nl = (int)min(wc, (unsigned)CAP);
   for (int j = lane; j < nl; j += 32) atomicAdd(&sm.hist[next_digit<K>(sm.key[wid][j], L, shift2)], 1u);
@@ -768,8 +847,31 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
 
   // 3. what is known of every row behind the barrier (own row last, so its figures stay)
   bool bad = false, any_rank = false, my_rank = false;
-  const int nrows = CLU ? 1 : a.batch;
-  unsigned digit = 0, need = 0, amb = 0;
+  const int nrows = CLU ? 1 : a.batch, own = CLU ? 0 : b;
+  // the digit of histogram p in which row r's want-th largest lies
+  auto settle = [&](int p, int r, unsigned want) -> unsigned {
+    const uint4 h = four_bins(p, r);
+    const unsigned hs[4] = {h.x, h.y, h.z, h.w};
+    unsigned tot;
+    unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const unsigned up = tot - from;  // samples from this bin up
+      if (up >= want && up - hs[e] < want) {
+        s_digit = (unsigned)(4 * tid + e);
+        r_need[CLU ? 0 : r] = want - (up - hs[e]);
+        r_amb[CLU ? 0 : r] = hs[e];
+      }
+      from += hs[e];
+    }
+    __syncthreads();
+    const unsigned d = s_digit;
+    __syncthreads();
+    return d;
+  };
+  K base = L;          // the row's deciding digit: keys of [base, base + 2^my_sh),
+  int my_sh = shift2;
+  bool open = false;   // or all from base up
   for (int q = 1; q <= nrows; q++) {
     const int r = CLU ? b : (b + q) % nrows;
     const unsigned *ctl = slot(2, r);
@@ -780,73 +882,125 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
       bad = true;
     } else if (listed > (unsigned)a.num || !all) {
       my_rank = any_rank = true;
-      const uint4 h = four_bins(1, r);
-      const unsigned hs[4] = {h.x, h.y, h.z, h.w};
-      unsigned tot;
-      unsigned from = ct_excl_scan(h.x + h.y + h.z + h.w, ws, &tot);
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const unsigned up = tot - from;  // listed samples from this bin up
-        if (up >= (unsigned)a.num && up - hs[e] < (unsigned)a.num) {
-          s_digit = (unsigned)(4 * tid + e);
-          s_need = (unsigned)a.num - (up - hs[e]);
-          s_amb = hs[e];
-        }
-        from += hs[e];
-      }
-      __syncthreads();
-      digit = s_digit;
-      need = s_need;
-      amb = s_amb;
-      __syncthreads();
-      if (amb > (unsigned)AMB_MAX) bad = true;
+      const unsigned d = settle(1, r, (unsigned)a.num);
+      open = d == (unsigned)HIST_BINS - 1u;
+      if (open && r_amb[CLU ? 0 : r] > AMB_MAX) bad = true;
+      base = L + ((K)d << shift2);
     }
   }
-  auto clear_slots = [&](int r, int part, int parts) {
-    for (int i = part * CT + tid; i < LIST_SLOTS * HIST_BINS; i += parts * CT) slot(i / HIST_BINS, r)[i % HIST_BINS] = 0;
+  if (__builtin_expect(bad, 0)) return give_up(LIST_SLOTS);
+  // A digit with too many samples to rank is counted again in 2048 parts, down to single
+  // values.  Three histograms take turns: one is read, one filled, one cleared.
+  auto any_left = [&]() {
+    bool c = false;
+    for (int r = 0; r < nrows; r++) c |= r_amb[r] > AMB_MAX;
+    return c;
   };
-  if (bad) {
-    if (solo) {
-      __syncthreads();
-      return false;
+  int levels = 0;
+  for (int sh = shift2; __builtin_expect(sh > 0 && any_left(), 0); levels++) {
+    const int s1 = sh > 11 ? sh - 11 : 0;
+    const int p = levels % 3 == 0 ? FINER_SLOT : levels % 3 == 1 ? 0 : 1;
+    const int z = levels % 3 == 0 ? 0 : levels % 3 == 1 ? 1 : FINER_SLOT;
+    const bool mine = r_amb[own] > AMB_MAX;
+    __syncthreads();
+    for (int i = tid; i < HIST_BINS; i += CT) sm.hist[i] = 0;
+    if (!solo)
+      for (int i = ci * CT + tid; i < HIST_BINS; i += a.cpr * CT) slot(z, b)[i] = 0;
+    __syncthreads();
+    if (mine)
+      for (int j = lane; j < nl; j += 32) {
+        const K k = sm.key[wid][j];
+        if (k >= base && (k - base) >> sh == 0) atomicAdd(&sm.hist[(k - base) >> s1], 1u);
+      }
+    __syncthreads();
+    publish(p);
+    for (int q = 1; q <= nrows; q++) {
+      const int r = CLU ? b : (b + q) % nrows;
+      if (r_amb[CLU ? 0 : r] > AMB_MAX) {
+        const unsigned d = settle(p, r, r_need[CLU ? 0 : r]);
+        if (r == b) base += (K)d << s1;
+      }
     }
-    sync_all<CLU>();  // every CTA has read the row's figures
-    for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++) clear_slots(r, CLU ? ci : blockIdx.x, CLU ? a.cpr : gridDim.x);
-    sync_all<CLU>();
-    return false;
+    if (mine) my_sh = s1;
+    sh = s1;
   }
+  const unsigned need = r_need[own], amb = r_amb[own];
+  const bool ties = my_rank && amb > AMB_MAX;  // of the one value base
+  auto deciding = [&](K k) { return k >= base && (open || (k - base) >> my_sh == 0); };
 
   int *o = a.out + (size_t)b * a.out_stride;
   const unsigned *tb = a.tiles + (size_t)b * a.max_tiles * 2;
   const long long seg = lo + (long long)g0 * GK;  // this warp's first sample
   if (my_rank) {
-    // exchange the deciding digit's samples
+    // exchange the deciding digit's samples, or their counts
     unsigned na = 0, nd = 0;
     for (int j = lane; j < nl; j += 32) {
-      const unsigned d = next_digit<K>(sm.key[wid][j], L, shift2);
-      nd += d > digit;
-      na += d == digit;
+      const K k = sm.key[wid][j];
+      const bool in = deciding(k);
+      nd += k >= base && !in;
+      na += in;
     }
     const unsigned packed = na | (nd << 16);  // at most 16 x 512 listed samples a CTA
     unsigned tot;
     const unsigned pre = ct_excl_scan(packed, ws, &tot);
     if (tid == 0) {
-      a.tiles[((size_t)b * a.max_tiles + ci) * 2 + 1] = tot >> 16;
-      s_need = !solo && (tot & 0xffffu) ? atomicAdd(&slot(2, b)[3], tot & 0xffffu) : 0u;
+      unsigned *t = a.tiles + ((size_t)b * a.max_tiles + ci) * 2;
+      t[1] = tot >> 16;
+      if (ties) t[0] = tot & 0xffffu;
+      else s_at = !solo && (tot & 0xffffu) ? atomicAdd(&slot(2, b)[3], tot & 0xffffu) : 0u;
     }
     __syncthreads();
-    unsigned at = s_need + (pre & 0xffffu);
+    unsigned at = s_at + (pre & 0xffffu);
     K *ek = solo ? sm.amb.key : reinterpret_cast<K *>(slot(3, b));
     int *ei = solo ? sm.amb.idx : reinterpret_cast<int *>(slot(4, b));
-    for (int j = lane; j < nl; j += 32)
-      if (next_digit<K>(sm.key[wid][j], L, shift2) == digit) {
+    for (int j = lane; !ties && j < nl; j += 32)
+      if (deciding(sm.key[wid][j])) {
         ek[at] = sm.key[wid][j];
         ei[at] = (int)(seg + sm.off[wid][j]);
         at++;
       }
   }
   if (any_rank && !solo) sync_all<CLU>();
-  if (my_rank) {
+  if (__builtin_expect(ties, 0)) {
+    // every sample above base, and the first `need` that equal it
+    unsigned bg = 0, be = 0;
+    for (int c = tid; c < ci; c += CT) {
+      be += __ldcg(&tb[c * 2]);
+      bg += __ldcg(&tb[c * 2 + 1]);
+    }
+    unsigned gt0, eq0;
+    ct_excl_scan(bg, ws, &gt0);
+    ct_excl_scan(be, ws, &eq0);
+    unsigned mg = 0, me = 0;
+    for (int j = lane; j < nl; j += 32) {
+      mg += sm.key[wid][j] > base;
+      me += sm.key[wid][j] == base;
+    }
+    mg = __reduce_add_sync(0xffffffffu, mg);
+    me = __reduce_add_sync(0xffffffffu, me);
+    __syncthreads();
+    if (lane == 0) {
+      wcnt[wid] = mg;
+      weq[wid] = me;
+    }
+    __syncthreads();
+    for (int i = 0; i < wid; i++) {
+      gt0 += wcnt[i];
+      eq0 += weq[i];
+    }
+    unsigned pos = gt0 + min(eq0, need);
+    for (int j0 = 0; j0 < nl; j0 += 32) {
+      const int j = j0 + lane;
+      const K k = j < nl ? sm.key[wid][j] : (K)0;
+      const bool eq = j < nl && k == base;
+      const unsigned be = __ballot_sync(0xffffffffu, eq), under = (1u << lane) - 1u;
+      const bool take = j < nl && (k > base || (eq && eq0 + __popc(be & under) < need));
+      const unsigned bl = __ballot_sync(0xffffffffu, take);
+      if (take) o[pos + __popc(bl & under)] = (int)(seg + sm.off[wid][j]);
+      pos += __popc(bl);
+      eq0 += __popc(be);
+    }
+  } else if (my_rank) {
     // the num-th largest: rank `need` of the exchanged samples by key, then index
     for (int e = tid; !solo && e < (int)amb; e += CT) {
       sm.amb.key[e] = __ldcg(reinterpret_cast<const K *>(slot(3, b)) + e);
@@ -943,7 +1097,7 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
   __syncthreads();
   if (s_last) {
     __threadfence();
-    for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++) clear_slots(r, 0, 1);
+    for (int r = CLU ? b : 0; r < (CLU ? b + 1 : a.batch); r++) clear_slots(r, 0, 1, levels ? FINER_SLOT + 1 : LIST_SLOTS);
   }
   return true;
 }
