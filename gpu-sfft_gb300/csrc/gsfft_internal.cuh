@@ -70,6 +70,18 @@ class PerContext {
     }
     return rc;
   }
+  // Calls f the first time in this context (not at all when the table is full).
+  template <typename F>
+  void once(F &&f) {
+    CtxKey k;
+    if (current_ctx_key(&k) != 0) return;
+    std::lock_guard<std::mutex> lock(mu_);
+    for (int i = 0; i < n_; i++)
+      if (keys_[i] == k) return;
+    if (n_ == kSlots) return;
+    keys_[n_++] = k;
+    f();
+  }
 
  private:
   static constexpr int kSlots = 64;
@@ -117,6 +129,13 @@ extern thread_local int g_launch_counter;
 // makes a plan per call, spent 0.8 of its 1.25 ms on them at n = 2^20.  add()
 // notes a buffer, commit() allocates the block and sets the pointers; the buffers
 // added with zero = true lie together and are cleared with one memset on st.
+//
+// The first commit in a context also takes 512 bytes that stay: allocations below 2 MB
+// share 2 MB blocks, and one that finds no block in use maps a new one (31 us, and 27 us
+// to unmap it when it is freed) where it takes 2 us from a block that is there.  A plan's many
+// small buffers kept such blocks in use; with one large one per plan, the calls
+// that allocate their own scratch beside a living plan had gone from 45 to 120 us
+// (gsfft_fft of 2^8 floats), 42 to 120 (gsfft_cutoff of 1000), 33 to 163 (gsfft_stage_estimate).
 class Arena {
  public:
   template <typename T>
@@ -129,6 +148,11 @@ class Arena {
     all = plain;
     for (const auto &w : zeroed_) all += round_up(w.second);
     *block = nullptr;
+    static PerContext<int> small_block;
+    small_block.once([] {
+      void *stays = nullptr;
+      if (cudaMalloc(&stays, 512) != cudaSuccess) cudaGetLastError();  // only slower without
+    });
     const cudaError_t e = cudaMalloc(block, all ? all : 16);
     if (e != cudaSuccess) {
       set_last_error("cudaMalloc(%zu): %s", all, cudaGetErrorString(e));
