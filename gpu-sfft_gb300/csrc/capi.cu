@@ -616,14 +616,15 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
   unsigned *bm = nullptr, *d_ep = nullptr;
   int *cnt = nullptr, *csum = nullptr, *stash = nullptr;
   RunCtl *ctl = nullptr;
-  int s = GSFFT_OK;
-  if (cudaMalloc(&bm, sizeof(unsigned) * words) != cudaSuccess ||
-      cudaMalloc(&cnt, sizeof(int) * B_thresh) != cudaSuccess ||
-      cudaMalloc(&csum, sizeof(int) * vote_csum_ints(B_thresh, n / B)) != cudaSuccess ||
-      cudaMalloc(&stash, sizeof(int) * vote_stash_ints(B_thresh)) != cudaSuccess ||
-      cudaMalloc(&ctl, sizeof(RunCtl)) != cudaSuccess ||
-      cudaMalloc(&d_ep, sizeof(unsigned)) != cudaSuccess)
-    s = GSFFT_ERR_ALLOC;
+  Arena mem;
+  void *block = nullptr;
+  mem.add(&bm, sizeof(unsigned) * words);
+  mem.add(&cnt, sizeof(int) * (size_t)B_thresh);
+  mem.add(&csum, sizeof(int) * (size_t)vote_csum_ints(B_thresh, n / B));
+  mem.add(&stash, sizeof(int) * (size_t)vote_stash_ints(B_thresh));
+  mem.add(&ctl, sizeof(RunCtl));
+  mem.add(&d_ep, sizeof(unsigned));
+  int s = mem.commit(&block, st);
   Draws d;
   memset(&d, 0, sizeof(d));
   d.a[0] = a;
@@ -647,12 +648,7 @@ int gsfft_stage_reverse_hash(const int *d_J, int B_thresh, const int *d_J2, int 
     *h_count = c.cand_count;
     if (c.overflow) s = GSFFT_ERR_CAPACITY;
   }
-  cudaFree(bm);
-  cudaFree(cnt);
-  cudaFree(csum);
-  cudaFree(stash);
-  cudaFree(ctl);
-  cudaFree(d_ep);
+  if (block) cudaFree(block);
   return s;
 }
 

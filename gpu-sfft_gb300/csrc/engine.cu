@@ -319,9 +319,12 @@ int launch_convert_taps(const double2 *d_ft, void *dst, int w, bool to_float, cu
 int plan_set_filter(Plan *P, const void *d_ft, const void *d_ff, cudaStream_t st) {
   const gsfft_params &p = P->p;
   if (!d_ft || !d_ff) return GSFFT_ERR_PARAM;
-  GS_CHECK(launch_convert_taps((const double2 *)d_ft, P->filt, p.w, P->precision == GSFFT_MIXED, st));
-  if (P->use_stream || P->use_cols)
-    GS_CHECK(launch_stream_taps(P->precision, P->filt, p.w, p.B, P->filt_bm, st));
+  // the column-ordered forms read the bucket-major table (its taps the caller's own in
+  // FP64) and, with the residue quirk, the taps in order too
+  const bool mixed = P->precision == GSFFT_MIXED, table = P->use_stream || P->use_cols;
+  if (mixed || !table || (P->flags & GSFFT_FLAG_QUIRK_RESIDUE))
+    GS_CHECK(launch_convert_taps((const double2 *)d_ft, P->filt, p.w, mixed, st));
+  if (table) GS_CHECK(launch_stream_taps(P->precision, mixed ? P->filt : d_ft, p.w, p.B, P->filt_bm, st));
   GS_CHECK(launch_hinv((const double2 *)d_ff, p.n, p.n / p.B, P->hinv, st));
   GS_CUDA(cudaStreamSynchronize(st));
   P->filter_set = true;
