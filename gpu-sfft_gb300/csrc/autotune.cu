@@ -12,6 +12,12 @@
 // each candidate plan timed with CUDA events over a few runs on the caller's
 // signal, filter and draws.  Results are kept in a plain text file, one line
 // per (device, precision, flags, sizes) key.
+//
+// In FP64 form 2 means gathers in column order, or with GSFFT_FLAG_FORCE_GATHER
+// in bucket order: the flag belongs to the measured plans and to the key.  FP64
+// keys also name the column order, so that a line stored when bucket order was
+// the only other form (it made the ordered pass win at n = 2^27, where columns
+// take 436 us and the pass 489) is not an answer.
 #include "engine.cuh"
 
 #include <stdio.h>
@@ -28,7 +34,7 @@ std::mutex g_cache_mu;
 
 // the flags that change a plan's pipeline, and so belong to the cache key
 constexpr unsigned kTuneFlags = GSFFT_FLAG_QUIRK_RESIDUE | GSFFT_FLAG_RAW_SELECTION |
-                                GSFFT_FLAG_TC_BUCKET_FFT | GSFFT_FLAG_TC_RLFC_FFT |
+                                GSFFT_FLAG_FORCE_GATHER | GSFFT_FLAG_TC_BUCKET_FFT | GSFFT_FLAG_TC_RLFC_FFT |
                                 GSFFT_FLAG_CC_BUCKET_FFT;
 
 int cache_key(const gsfft_params &p, int precision, unsigned flags, std::string *key) {
@@ -40,9 +46,10 @@ int cache_key(const gsfft_params &p, int precision, unsigned flags, std::string 
   for (char &c : name)
     if (c == ' ' || c == '\t') c = '_';
   char buf[512];
-  snprintf(buf, sizeof(buf), "%s|sms=%d|prec=%d|flags=%u|n=%d|B=%d|W=%d|w=%d|Bt=%d|loops=%d|ll=%d|R=%d",
+  snprintf(buf, sizeof(buf), "%s|sms=%d|prec=%d|flags=%u|n=%d|B=%d|W=%d|w=%d|Bt=%d|loops=%d|ll=%d|R=%d%s",
            name.c_str(), prop.multiProcessorCount, precision, flags & kTuneFlags, p.n, p.B,
-           p.W_RLFC, p.w, p.B_thresh, p.loops, p.loops_loc, p.RLFC_loops);
+           p.W_RLFC, p.w, p.B_thresh, p.loops, p.loops_loc, p.RLFC_loops,
+           precision == GSFFT_FP64 ? "|gather=cols" : "");
   *key = buf;
   return GSFFT_OK;
 }
@@ -167,7 +174,7 @@ int gsfft_autotune_plan(const gsfft_params *p, int precision, unsigned flags, co
   Bench b;
   b.p = p;
   b.precision = precision;
-  b.flags = flags & ~(GSFFT_FLAG_FORCE_GATHER | GSFFT_FLAG_FORCE_STREAM);
+  b.flags = flags & ~GSFFT_FLAG_FORCE_STREAM;
   b.d_x = d_x;
   b.ft = d_filter_time;
   b.ff = d_filter_freq;

@@ -121,7 +121,9 @@ int gsfft_plan_create(const gsfft_params *p, int precision, unsigned flags,
  * rules; zero in a field keeps the rule.  gsfft_autotune_plan chooses them by
  * timing. */
 typedef struct {
-  int perm_filter_form;    /* 1: one ordered pass over the signal, 2: gathers */
+  int perm_filter_form;    /* 1: one ordered pass over the signal, 2: gathers (FP64: in
+                              column order where the sizes allow it, without
+                              GSFFT_FLAG_FORCE_GATHER) */
   int row_groups;          /* ordered pass: row groups of the signal matrix, each
                               with its own partial bins (power of two) */
   int bucket_first_radix;  /* log2 of the bucket FFT's first-pass radix (two-pass sizes) */
