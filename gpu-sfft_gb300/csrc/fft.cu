@@ -240,9 +240,10 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
   if (p.npass > 1 && (long long)batch * p.n * (p.npass == 3 ? 2 : 1) > p.scratch_elems)
     return GSFFT_ERR_PARAM;
   if (io.gather_x && batch > 8) return GSFFT_ERR_PARAM;
-  if (io.in_lognc >= 0 && (io.gather_x || !fft_reads_row_blocks(p, io.in_lognc)))
+  if (io.in_lognc >= 0 && (io.sum_rows > 1 || io.gather_x || !fft_reads_row_blocks(p, io.in_lognc)))
     return GSFFT_ERR_UNSUPPORTED;
-  const bool tiled = fft_tiled(p) && !io.gather_x;
+  if (dbl && io.sum_rows > 1) return GSFFT_ERR_UNSUPPORTED;  // FP32 passes only
+  const bool tiled = fft_tiled(p) && !io.gather_x && io.sum_rows <= 1;
   const void *src = in;
   char *scr = (char *)p.scratch;
   long long Ns = 1;
@@ -282,6 +283,8 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
     a.lognc = i == 0 ? io.in_lognc : -1;
     a.tile_out = tiled && i == 0;
     a.tile_in = tiled && i == 1;
+    a.nsum = (i == 0) ? io.sum_rows : 1;
+    a.sstride = io.sum_stride;
     a.write_complex = last ? (io.write_complex ? 1 : 0) : 1;
     const long long total_sub = (p.n >> p.logR[i]) * batch;
     a.total = total_sub;
@@ -305,6 +308,8 @@ int fft_exec(const FftPlan &p, const void *in, void *out, int batch, int sign,
       t.row_max = a.row_max;
       t.write_complex = a.write_complex;
       t.err = io.err;
+      t.nsum = a.nsum;
+      t.sstride = a.sstride;
       s = p.logR[i] == 6 ? launch_tc64_last_pass(t, st) : launch_tc4096_pass(t, st);
     } else {
       s = dispatch_pass(dbl, p.logR[i], a, total_sub, st);

@@ -43,6 +43,8 @@ struct PassArgs {
   long long gstride;
   void *samples;      // last pass only, or null
   void *row_max;      // per batch row, with samples
+  int nsum;           // first pass: add nsum partial inputs sstride apart
+  long long sstride;
   int lognc;          // first pass: FftIo::in_lognc, or -1
   int tile_in, tile_out;  // the array between two passes in tiles of four (FP64: two) sub-transforms (fft_tiled)
   int write_complex;
@@ -341,16 +343,16 @@ __device__ __forceinline__ void rt_smem_stage(V *sm, const V *__restrict__ twR, 
   __syncthreads();
 }
 
+// radix 16 where a thread holds 16 points, radix 8 where it holds 8
 template <typename V, int LOGR, int G, int NT>
 __device__ __forceinline__ void rt_cta_fft(V *sm, const V *__restrict__ twR) {
-  static_assert((1 << LOGR) * G / NT >= 16, "radix-16 stages: at least 16 points a thread");
-  constexpr int LEFT = LOGR % 4;
+  constexpr int LOGE = (1 << LOGR) * G / NT >= 16 ? 4 : 3, LEFT = LOGR % LOGE;
   int Ns = 1;
   if (LEFT == 1) { rt_smem_stage<V, LOGR, G, 2, NT>(sm, twR, Ns); Ns <<= 1; }
   if (LEFT == 2) { rt_smem_stage<V, LOGR, G, 4, NT>(sm, twR, Ns); Ns <<= 2; }
   if (LEFT == 3) { rt_smem_stage<V, LOGR, G, 8, NT>(sm, twR, Ns); Ns <<= 3; }
 #pragma unroll 1
-  for (int s = 0; s < LOGR / 4; s++) { rt_smem_stage<V, LOGR, G, 16, NT>(sm, twR, Ns); Ns <<= 4; }
+  for (int s = 0; s < LOGR / LOGE; s++) { rt_smem_stage<V, LOGR, G, 1 << LOGE, NT>(sm, twR, Ns); Ns <<= LOGE; }
 }
 
 template <typename V, int LOGR, int G, int LOGNS>
@@ -609,11 +611,12 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
   // passes after the first fold the conjugation and the inter-pass
   // twiddles into their first stage (fast load path; radix 2^11 to 2^13, where
   // the first stage keeps its inputs in registers without spilling)
-  pt.on = LOGR >= 11 && LOGR <= 13 && g_fast_in && !gx && logNs > 0;
+  pt.on = LOGR >= 11 && LOGR <= 13 && g_fast_in && !gx && a.nsum <= 1 &&
+          logNs > 0;
   if constexpr (fused_io(LOGR)) {
     // S >= G with both powers of two: the grid covers the batch exactly and
     // all G sub-transforms of a CTA lie in one batch row
-    if (g_fast_in && !gx) {
+    if (g_fast_in && !gx && a.nsum <= 1) {
       const long long u = u0 + tid % G;
       const long long b = u >> logS, j = u & Smask;
       PreTw ptf = pt;  // inter-pass twiddles in registers wherever Ns > 1
@@ -640,68 +643,136 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
       const V *src = in + b * a.bstride + (a.tile_in ? (j & ~3LL) * R + 4 * r0 + (j & 3) : j + ((long long)r0 << logS));
       const long long qs = (long long)TPF << (a.tile_in ? 2 : logS);
       const long long jm = j & Nsmask;
+      const long long mm0 = jm * r0, dmm = jm * TPF;  // twiddle exponents, < Ns * R
+      if (a.nsum <= 1) {
 #pragma unroll
-      for (int q = 0; q < ITER; q++)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
-                         (unsigned)__cvta_generic_to_shared(dst + q * TPF + ((q * TPF) >> 4))),
-                     "l"(src + q * qs), "n"(sizeof(V))
-                     : "memory");
-      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-      if ((a.inverse || logNs > 0) && !pt.on) {
-        // each thread rewrites only the elements it loaded: no barrier needed here
-        TwRun tr;
-        if (logNs > 0)
-          tr.init(reinterpret_cast<const float2 *>(thi), reinterpret_cast<const float2 *>(tlo),
-                  a.tw_h, hmask, jm, r0, TPF);
+        for (int q = 0; q < ITER; q++)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(dst + q * TPF + ((q * TPF) >> 4))),
+                       "l"(src + q * qs), "n"(sizeof(V))
+                       : "memory");
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        if ((a.inverse || logNs > 0) && !pt.on) {
+          // each thread rewrites only the elements it loaded: no barrier needed here
+          TwRun tr;
+          if (logNs > 0)
+            tr.init(reinterpret_cast<const float2 *>(thi), reinterpret_cast<const float2 *>(tlo),
+                    a.tw_h, hmask, jm, r0, TPF);
 #pragma unroll
-        for (int q = 0; q < ITER; q++) {
-          V *p = dst + q * TPF + ((q * TPF) >> 4);
-          V v = *p;
-          if (a.inverse) v.y = -v.y;
-          if (logNs > 0) v = cmul(v, tr.next(q));
-          *p = v;
+          for (int q = 0; q < ITER; q++) {
+            V *p = dst + q * TPF + ((q * TPF) >> 4);
+            V v = *p;
+            if (a.inverse) v.y = -v.y;
+            if (logNs > 0) v = cmul(v, tr.next(q));
+            *p = v;
+          }
+        }
+      } else {
+        // row-group partials added on load (first pass after the streaming perm+filter)
+        // (a first pass: logNs = 0 in practice, so per-element look-ups stay)
+        constexpr int LB = ITER < 4 ? ITER : 4;
+#pragma unroll
+        for (int q0 = 0; q0 < ITER; q0 += LB) {
+          V vbuf[LB];
+#pragma unroll
+          for (int q = 0; q < LB; q++) {
+            const V *p = src + (q0 + q) * qs;
+            V v = p[0];
+            for (int s2 = 1; s2 < a.nsum; s2++) v = cadd(v, p[s2 * a.sstride]);
+            vbuf[q] = v;
+          }
+#pragma unroll
+          for (int q = 0; q < LB; q++) {
+            V v = vbuf[q];
+            if (a.inverse) v.y = -v.y;
+            if (logNs > 0) {
+              const long long mm = mm0 + (q0 + q) * dmm;
+              v = cmul(v, cmul(thi[mm >> a.tw_h], tlo[mm & hmask]));
+            }
+            dst[(q0 + q) * TPF + (((q0 + q) * TPF) >> 4)] = v;
+          }
         }
       }
     }
   } else {
-    // every element straight into shared memory with cp.async: all ITER loads
-    // of a thread in flight, no registers held
-#pragma unroll
-    for (int q = 0; q < ITER; q++) {
-      const int lt = threadIdx.x + q * NT;
-      int g, r;
-      if (g_fast_in) { g = lt % G; r = lt / G; } else { r = lt % R; g = lt / R; }
-      const long long u = u0 + g;
-      const long long b = u >> logS, j = u & Smask;
-      const long long m = j + ((long long)r << logS);
-      V *dst = &sm[g * RP + padded(r)];
-      if (u >= a.total) {
-        *dst = mk((T)0, (T)0);
-      } else {
-        const V *src = gx ? &gx[a.goffs[b] + m * a.gstride] : &in[b * a.bstride + m];
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                     "l"(src), "n"(sizeof(V))
-                     : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-    if (a.inverse || logNs > 0) {
-      // each thread rewrites only the elements it loaded: no barrier needed here
+    if (a.nsum <= 1) {
+      // every element straight into shared memory with cp.async: all ITER loads
+      // of a thread in flight, no registers held
 #pragma unroll
       for (int q = 0; q < ITER; q++) {
         const int lt = threadIdx.x + q * NT;
         int g, r;
         if (g_fast_in) { g = lt % G; r = lt / G; } else { r = lt % R; g = lt / R; }
-        V *p = &sm[g * RP + padded(r)];
-        V v = *p;
-        if (a.inverse) v.y = -v.y;
-        if (logNs > 0) {
-          const long long j = (u0 + g) & Smask;
-          const long long mm = (j & Nsmask) * r;  // < Ns * R
-          V w = cmul(thi[mm >> a.tw_h], tlo[mm & hmask]);
-          v = cmul(v, w);
+        const long long u = u0 + g;
+        const long long b = u >> logS, j = u & Smask;
+        const long long m = j + ((long long)r << logS);
+        V *dst = &sm[g * RP + padded(r)];
+        if (u >= a.total) {
+          *dst = mk((T)0, (T)0);
+        } else {
+          const V *src = gx ? &gx[a.goffs[b] + m * a.gstride] : &in[b * a.bstride + m];
+          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                       "l"(src), "n"(sizeof(V))
+                       : "memory");
         }
-        *p = v;
+      }
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+      if (a.inverse || logNs > 0) {
+        // each thread rewrites only the elements it loaded: no barrier needed here
+#pragma unroll
+        for (int q = 0; q < ITER; q++) {
+          const int lt = threadIdx.x + q * NT;
+          int g, r;
+          if (g_fast_in) { g = lt % G; r = lt / G; } else { r = lt % R; g = lt / R; }
+          V *p = &sm[g * RP + padded(r)];
+          V v = *p;
+          if (a.inverse) v.y = -v.y;
+          if (logNs > 0) {
+            const long long j = (u0 + g) & Smask;
+            const long long mm = (j & Nsmask) * r;  // < Ns * R
+            V w = cmul(thi[mm >> a.tw_h], tlo[mm & hmask]);
+            v = cmul(v, w);
+          }
+          *p = v;
+        }
+      }
+    } else {
+      // row-group partials added on load (first pass after the streaming perm+filter)
+      constexpr int LB = ITER < 4 ? ITER : 4;
+#pragma unroll
+      for (int q0 = 0; q0 < ITER; q0 += LB) {
+        V vbuf[LB];
+#pragma unroll
+        for (int q = 0; q < LB; q++) {
+          const int lt = threadIdx.x + (q0 + q) * NT;
+          int g, r;
+          if (g_fast_in) { g = lt % G; r = lt / G; } else { r = lt % R; g = lt / R; }
+          const long long u = u0 + g;
+          const long long b = u >> logS, j = u & Smask;
+          const long long m = j + ((long long)r << logS);
+          V v = mk((T)0, (T)0);
+          if (u < a.total) {
+            const long long idx = b * a.bstride + m;
+            v = in[idx];
+            for (int s2 = 1; s2 < a.nsum; s2++) v = cadd(v, in[idx + s2 * a.sstride]);
+          }
+          vbuf[q] = v;
+        }
+#pragma unroll
+        for (int q = 0; q < LB; q++) {
+          const int lt = threadIdx.x + (q0 + q) * NT;
+          int g, r;
+          if (g_fast_in) { g = lt % G; r = lt / G; } else { r = lt % R; g = lt / R; }
+          V v = vbuf[q];
+          if (a.inverse) v.y = -v.y;
+          if (logNs > 0) {
+            const long long j = (u0 + g) & Smask;
+            const long long mm = (j & Nsmask) * r;
+            V w = cmul(thi[mm >> a.tw_h], tlo[mm & hmask]);
+            v = cmul(v, w);
+          }
+          sm[g * RP + padded(r)] = v;
+        }
       }
     }
   }

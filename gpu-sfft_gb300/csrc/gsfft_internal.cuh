@@ -299,6 +299,8 @@ struct TcPassArgs {
   void *row_max;        // u32 bit pattern per row, with samples
   int write_complex;
   int *err;             // set when a completion wait timed out (may be null)
+  int nsum = 1;         // radix-4096 form: add nsum partial inputs sstride apart
+  long long sstride = 0;
 };
 size_t tc_F_bytes();
 int tc_build_F(void *F, cudaStream_t st);
@@ -315,6 +317,10 @@ struct FftIo {
   const void *gather_x = nullptr;
   long long gather_offsets[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // one per batch entry (batch <= 8)
   long long gather_stride = 0;
+  // first-pass loader alternative: element = sum over s < sum_rows of
+  // in[s * sum_stride + index], added in s order (row-group partials)
+  int sum_rows = 1;
+  long long sum_stride = 0;
   // first-pass loader alternative (fft_reads_row_blocks): the input is a matrix of
   // 2^in_lognc columns in blocks of four rows, point t = row 2^in_lognc + column at
   // (row & ~3) 2^in_lognc + 4 column + (row & 3); FP64 the same with pairs of rows;

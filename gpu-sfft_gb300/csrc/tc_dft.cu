@@ -346,8 +346,8 @@ __device__ __forceinline__ void store_parts8_row(unsigned char *xb, int row, int
 // memory) per tile.  With r = r1 + 64 r2 and k = k2 + 64 k1:
 //   Y[r1][k2] = sum_r2 v[r1 + 64 r2] W64^(r2 k2)                   (product 1)
 //   V[k2 + 64 k1] = sum_r1 W64^(r1 k1) W4096^(r1 k2) Y[r1][k2]       (product 2)
-// where v[r] = in[j + r S] (S = N / 4096 sub-transforms per row) and
-// out[j 4096 + k] = V[k].
+// where v[r] = in[j + r S] (S = N / 4096 sub-transforms per row, the sum of
+// nsum partial inputs sstride apart) and out[j 4096 + k] = V[k].
 // Product 1's X operand: row n = (jj, r1) = 64 jj + r1, column K = r2 (Re) and
 // 64 + r2 (Im).  Its result D (TMEM lane 2 k2 + c, column n) is read back
 // lane by lane: lanes 2 k2 and 2 k2 + 1 (adjacent threads of one warp) hold
@@ -445,6 +445,19 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) tc4096_pass_kernel(TcPassArgs a
         for (int q = 0; q < 8; q++)
           xv[h][q] = __ldg(reinterpret_cast<const float4 *>(
               src + ((long long)(r1 + 64 * (8 * (g0 + 4 * h) + q)) << logS)));
+      for (int s2 = 1; s2 < a.nsum; s2++) {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(
+                src + s2 * a.sstride + ((long long)(r1 + 64 * (8 * (g0 + 4 * h) + q)) << logS)));
+            xv[h][q].x += v.x;
+            xv[h][q].y += v.y;
+            xv[h][q].z += v.z;
+            xv[h][q].w += v.w;
+          }
+      }
       unsigned char *xb = X + b * TQ_XBUF;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -896,7 +909,7 @@ int tc_build_F_smem(void *F, cudaStream_t st) {
 int launch_tc64_last_pass(const TcPassArgs &a, cudaStream_t st) {
   // the last pass (Ns = N / 64), at least 128 sub-transforms per row, the
   // inter-pass twiddle tables of the pass, 16-byte aligned rows
-  if (a.logN < 13 || a.logNs != a.logN - 6 || !a.tw_hi || !a.tw_lo || !a.F)
+  if (a.logN < 13 || a.logNs != a.logN - 6 || !a.tw_hi || !a.tw_lo || !a.F || a.nsum > 1)
     return GSFFT_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) ||
       (reinterpret_cast<uintptr_t>(a.samples) & 7) || (a.bstride & 1) || (a.row_max && !a.samples))
@@ -928,7 +941,7 @@ int launch_tc4096_pass(const TcPassArgs &a, cudaStream_t st) {
   if (a.logNs != 0 || a.logN < 13 || !a.tw_R || !a.F || a.samples || a.row_max || !a.write_complex)
     return GSFFT_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) ||
-      (a.bstride & 1) || (a.total & 1))
+      (a.bstride & 1) || (a.nsum > 1 && (a.sstride & 1)) || a.nsum < 1 || (a.total & 1))
     return GSFFT_ERR_UNSUPPORTED;
   static PerContext<int> attr;  // the kernel's dynamic shared memory limit, per context
   GS_CHECK(attr.ensure_at_least(TQ_SMEM, [](int v) {
