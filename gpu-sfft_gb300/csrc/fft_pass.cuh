@@ -343,16 +343,16 @@ __device__ __forceinline__ void rt_smem_stage(V *sm, const V *__restrict__ twR, 
   __syncthreads();
 }
 
-// radix 16 where a thread holds 16 points, radix 8 where it holds 8
 template <typename V, int LOGR, int G, int NT>
 __device__ __forceinline__ void rt_cta_fft(V *sm, const V *__restrict__ twR) {
-  constexpr int LOGE = (1 << LOGR) * G / NT >= 16 ? 4 : 3, LEFT = LOGR % LOGE;
+  static_assert((1 << LOGR) * G / NT >= 16, "radix-16 stages: at least 16 points a thread");
+  constexpr int LEFT = LOGR % 4;
   int Ns = 1;
   if (LEFT == 1) { rt_smem_stage<V, LOGR, G, 2, NT>(sm, twR, Ns); Ns <<= 1; }
   if (LEFT == 2) { rt_smem_stage<V, LOGR, G, 4, NT>(sm, twR, Ns); Ns <<= 2; }
   if (LEFT == 3) { rt_smem_stage<V, LOGR, G, 8, NT>(sm, twR, Ns); Ns <<= 3; }
 #pragma unroll 1
-  for (int s = 0; s < LOGR / LOGE; s++) { rt_smem_stage<V, LOGR, G, 1 << LOGE, NT>(sm, twR, Ns); Ns <<= LOGE; }
+  for (int s = 0; s < LOGR / 4; s++) { rt_smem_stage<V, LOGR, G, 16, NT>(sm, twR, Ns); Ns <<= 4; }
 }
 
 template <typename V, int LOGR, int G, int LOGNS>

@@ -1,4 +1,4 @@
-// Instantiations of the FP64 FFT pass: radix 2^7 .. 2^10.
+// Instantiations of the FP64 FFT pass: radix 2^6 .. 2^10.
 #include "fft_pass_fx.cuh"
 
 namespace gsfft {

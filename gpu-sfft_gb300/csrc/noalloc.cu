@@ -116,8 +116,6 @@ extern "C" int gsfft_cutoff_noalloc(const void *d_samples, int size, int num, in
   // what the selection expects to find zeroed; the rest is written before it is read
   GS_CUDA(cudaMemsetAsync(ss.state, 0, L.b.state, st));
   GS_CUDA(cudaMemsetAsync(ss.coop_hist, 0, L.b.coop_hist, st));
-  // The SelectScratch does not own the array: it is never passed to
-  // select_scratch_free.
   return select_top(d_samples, precision == GSFFT_FP64 ? 8 : 4, size, nullptr, num, batch, size,
                     d_out, num, nullptr, ss, st);
 }

@@ -666,8 +666,9 @@ bool stream_pf_supported(int n, int B, int loops, int W, int RLFC_loops) {
   return encode_fn() != nullptr;
 }
 
+// Blocks of rows after which a column's partial tap is added, whatever the tiles are.
 static int stream_rows_per_tile(int n, int B, int precision) {
-  return std::min(n / B, precision == GSFFT_FP64 ? 32 : 64);  // 32 KiB tiles of 64 columns
+  return std::min(n / B, precision == GSFFT_FP64 ? 32 : 64);
 }
 
 int stream_pf_groups(int n, int B, int w, int loops, int precision) {
@@ -676,9 +677,11 @@ int stream_pf_groups(int n, int B, int w, int loops, int precision) {
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // The groups' partial sums fix the FP32 rounding, so this rule does not follow
-  // the kernel's own tiles: blocks of 64 columns (32 above 15 loops) and 6 or 12
-  // items per SM, the former where a block's FP32 taps leave half the shared memory.
+  // The number of groups fixes the order of a bin's sums and so its last FP32 bit:
+  // it is part of what a plan returns, and not derived from the kernel's tiles (16
+  // columns, two CTAs an SM).  It doubles until there are 6 or 12 items of 64 columns (32
+  // above 15 loops) per SM: 6 where an item's FP32 taps and four tiles of 32 KiB (three
+  // above 9 loops) fit 218 KiB, as a kernel of one CTA an SM had them.
   const int cw = 64 * loops + 64 <= 1024 ? 64 : 32;
   const int slots = 8 * cw * loops * taps_per_bucket(w / B), tile = 8 * rt * cw;
   const bool few = precision != GSFFT_FP64 && cw == 64 &&
