@@ -241,11 +241,13 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   P->tuning.select_form = tn.select_form == 2 ? 2 : 1;
   // The side stream's few blocks go before the RLFC chain's: they waited for whole
   // passes of it, and the voting for them (n = 2^27, k = 16000: 409 -> 396 us,
-  // k = 43000: 882 -> 876, FP64: the same).
+  // k = 43000: 882 -> 876, FP64: the same).  One step above the lowest priority, which
+  // ordinary streams have, does that; a program's own streams of higher priority stay
+  // ahead of it.
   int low = 0, high = 0;
   if (s == GSFFT_OK &&
       (cudaDeviceGetStreamPriorityRange(&low, &high) != cudaSuccess ||
-       cudaStreamCreateWithPriority(&P->side, cudaStreamNonBlocking, high) != cudaSuccess ||
+       cudaStreamCreateWithPriority(&P->side, cudaStreamNonBlocking, std::max(low - 1, high)) != cudaSuccess ||
        cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
        cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming) != cudaSuccess ||
        cudaEventCreateWithFlags(&P->ev_bins, cudaEventDisableTiming) != cudaSuccess ||
