@@ -240,8 +240,8 @@ int plan_create(const gsfft_params &pp, int precision, unsigned flags, int max_c
   P->tuning.rlfc_first_radix = first_radix(P->fftW, P->tc_rlfc);
   P->tuning.select_form = tn.select_form == 2 ? 2 : 1;
   // The side stream's few blocks go before the RLFC chain's: they waited for whole
-  // passes of it, and the voting for them (n = 2^27, k = 16000: 409 -> 396 us,
-  // k = 43000: 882 -> 876, FP64: the same).  One step above the lowest priority, which
+  // passes of it, and the voting for them (n = 2^27, k = 16000: 392 -> 381 us,
+  // k = 43000: 837 -> 822, FP64: 901 -> 893; n = 2^20: the same).  One step above the lowest priority, which
   // ordinary streams have, does that; a program's own streams of higher priority stay
   // ahead of it.
   int low = 0, high = 0;
@@ -347,11 +347,16 @@ int plan_epoch_advance(Plan *P, cudaStream_t st) {
 // The packed vote tables of a small signal (two of n / 4 bytes) are cleared by the
 // run's first kernel; from 2^21 points on the next run's table is cleared on the
 // auxiliary stream beside the estimation (8 us at n = 2^27).  That costs a launch,
-// two event records and three waits: n = 2^14 runs are bound by such calls.
+// two event records and three waits: n = 2^14 runs are bound by such calls.  Mixed runs
+// at the start / on the stream: n = 2^14 56.2 / 57.4 us, 2^18 71.6 / 72.0, 2^20 91.0 /
+// 92.6, 2^22 89.0 / 89.9, 2^25 173.7 / 172.5 (FP64 238.3 / 236.3).
 static bool clear_at_start(const Plan *P) { return P->packed_vote && P->p.n <= (1 << 20); }
 // The bucket FFT of the estimation loops' rows: in one launch with the location
 // loops' where all rows are a part of the chip's threads (2^17 points), else later,
-// beside the voting.  n = 2^20, 7 rows of 2^13: it ended 8 us after the voting.
+// beside the voting.  n = 2^20, 7 rows of 2^13: it ended 8 us after the voting.  FP64
+// runs with one launch / two: n = 2^17 (7 x 2^9) 83.6 / 89.7 us, 2^20 (7 x 2^13) 96.9 /
+// 111.8, 2^22 (7 x 2^14) 111 / 116.5, 2^24 (7 x 2^15) 226 / 186; mixed 72 / 76, 91 / 100,
+// 90 / 92.4, 154 / 149.5.
 static bool all_rows_at_once(const Plan *P) { return (long long)P->p.loops * P->p.B <= (1 << 17); }
 
 int plan_run(Plan *P, const void *d_x, const int *offs, const int *a, const int *ai,

@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(nt_of(LOGR), minb_of(LOGR)) fft_pass_kernel(Pa
   V *sm = reinterpret_cast<V *>(smraw);
   const V *twR = reinterpret_cast<const V *>(a.twR);
   // The twiddles land beside the pass's own loads, which waited for a copy through
-  // registers before (n = 2^27 steps: k = 16000 381 -> 373 us, k = 43000 856 -> 826).
+  // registers before (n = 2^27 steps: k = 16000 387 -> 377 us, k = 43000 847 -> 807).
   V *tws = reinterpret_cast<V *>(smraw + tw_offset(LOGR));
   for (int i = threadIdx.x; i < R / 8; i += NT)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(tws + 2 * i)),

@@ -17,9 +17,9 @@
 // gives the number of spare leading bits ("lift"), so an impulse or a tone keeps
 // as many bits as noise does; the stage's twiddle factors carry 1/16, its worst
 // growth, which keeps |value| below 2^62.5 throughout.  Outputs are rounded to
-// double once.  Against an extended-precision transform the result is 5e-17 off
-// per pass (relative L2: noise, impulses, tones; 2e-16 where the samples spread
-// over e^+-40), the FP64 pass 1e-16 to 3e-16.
+// double once.  Against an extended-precision transform (relative L2, noise) one pass is
+// 5e-17 off and two passes of 2^16, 2^20 and 2^22 points 6.8e-17, in FP64 arithmetic
+// 2.8e-16, 3.1e-16 and 3.4e-16.
 //
 // Small samples beside large ones: a double keeps its 53 bits wherever it lies, a
 // fixed-point value those above 2^-58 .. 2^-62 of the row's largest.  Where samples share

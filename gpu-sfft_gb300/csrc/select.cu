@@ -366,7 +366,7 @@ int select_impl(const void *keys, long long size, const int *size_dev, int num, 
 //      ones by index are taken.  (Ranking up to 768, every pair in every CTA, took more than
 //      20 us, and sel_passes from 769 on 25: the k largest of a noiseless n = 2^26 run, all
 //      of one magnitude, 49 -> 23 us; two uniform rows of 2^22 floats 99 -> 42, of doubles
-//      148 -> 46.)
+//      150 -> 46.)
 // A guess that proves wrong (a list too small, fewer than num above L) costs time
 // only: sel_passes then does the selection.  That is left where one value, or values
 // within a 2^-14 of each other, fill a long row: 0.72 to 0.86 times the speed of
@@ -386,8 +386,9 @@ int select_impl(const void *keys, long long size, const int *size_dev, int num, 
 // What bounds them: instructions and block barriers, not the reads.  sel_passes ran
 // 80 instructions a sample on a noiseless row (two reads, 38 us for two rows of 2^22
 // floats) and read a noisy row five times (72 us; two rows of 2^24: 194 us);
-// sel_lists takes 26, 33 and 54 us.  Short rows (a cluster, or one CTA) are a chain of
-// barriers in both: 23 -> 21 us for rows of 2^17, 12 -> 9 for one CTA.
+// sel_lists takes 28, 34 and 55 us (1 to 2 of them for the code of the finer digits).
+// Short rows (a cluster, or one CTA) are a chain of barriers in both: 23 -> 22 us for
+// rows of 2^17, 12 -> 9 for one CTA.
 //
 // Rows that start on 16-byte boundaries (with a capacity of whole 16-byte words) are
 // read with 16-byte loads.  Histograms are left zeroed for the next call.

@@ -291,7 +291,10 @@ int gsfft_evaluate(gsfft_plan plan, const complex_t *d_x_f, const int *d_true_lo
 
 /* Batched unnormalised complex FFT of power-of-two size n_fft >= 256,
  * out-of-place or in place; sign -1 forward, +1 inverse; precision selects
- * complex_t or {float, float} elements. */
+ * complex_t or {float, float} elements.  FP64 passes compute in 64-bit fixed
+ * point relative to the largest sample of a sub-transform (error below that of
+ * FP64 arithmetic), and in FP64 arithmetic where many samples lie far below the
+ * largest, or it lies outside 2^-800 .. 2^970. */
 int gsfft_fft(const void *d_in, void *d_out, long long n_fft, int batch, int sign,
               int precision, void *stream);
 
