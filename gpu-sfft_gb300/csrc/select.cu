@@ -369,7 +369,7 @@ int select_impl(const void *keys, long long size, const int *size_dev, int num, 
 //      150 -> 46.)
 // A guess that proves wrong (a list too small, fewer than num above L) costs time
 // only: sel_passes then does the selection.  That is left where one value, or values
-// within a 2^-14 of each other, fill a long row: 0.72 to 0.86 times the speed of
+// within a 2^-14 of each other, fill a row: 0.71 to 0.93 times the speed of
 // sel_passes alone.
 //
 // sel_passes: each radix pass builds the CTA's chunk histogram in shared memory and
@@ -767,7 +767,8 @@ __device__ __forceinline__ bool sel_lists(const CoopArgs &a, int b, int ci, long
   constexpr int GU = 4;  // groups in flight
   const int gfull = (int)((hi - lo) / GK);  // groups without a bound check
   const uint4 *vrow = reinterpret_cast<const uint4 *>(row) + lo / EPQ + lane;
-  for (int g = g0; g < g1; g += GU) {
+  // (a warp whose list has run over stops: the row is left to sel_passes)
+  for (int g = g0; g < g1 && wc <= (unsigned)CAP; g += GU) {
     K ks[GU][EPQ];
     if (VEC && g + GU <= min(g1, gfull)) {
       uint4 v[GU];
